@@ -1,0 +1,174 @@
+// face.cuh -- the flux of one limited face in 64-bit fixed point.
+//
+// A face carries phi = C * FBND, FBND = FUP + a * LIMITER(R) * X
+// (src/ModRamDrift.f90:169-183).  In terms of the upwind cell u, the cell
+// downwind of it d and the one upwind of it uu (u, d, uu = F(f), F(f+1),
+// F(f-1) for C >= 0 and F(f+1), F(f), F(f+2) for C < 0) both directions read
+//   phi = C * (u + 1/2 (1 - U) * sgn(d-u) * lim),   U the Courant number,
+//   lim = min(beta*lo, hi), lo/hi the smaller/larger of |d-u|, |u-uu|
+// where u-uu and d-u have the same sign and |d-u| > 1e-27, else phi = C*u.
+// (max(min(beta|D|,|X|), min(|D|,beta|X|)) is that lim for beta >= 1.)
+//
+// The FP64 unit issues one warp instruction per 64 cycles per scheduler
+// while the integer pipes are mostly free, so the whole face runs on them:
+// the three cells are aligned to u's exponent in 64-bit fixed point with
+// u in [2^59, 2^60).  d and uu keep every bit down to 2^-59 of u (seven
+// below u's own last place); cells of 8u and more saturate at 4u or above,
+// where lim no longer depends on them (lo <= u when both differences have
+// one sign).  1 - U, lim and their product stay in fixed point, so nothing
+// is normalised or rounded until phi itself, which is rounded once: its
+// error is below that of the FP64 sequence (a rounded X, a, FBND and phi).
+// Negative, infinite, NaN and zero upwind cells, Courant numbers of 1 and
+// more, a zero C and the extremes of the exponent range report `special`;
+// the caller takes the FP64 form there.
+//
+// Bound and figures (GB300, four species on 20x25x35x72, one launch): the
+// FP64 sequence held the FP64 pipe, five operations a face (coefficient, X,
+// the limited correction, two for the update; phi, a and beta|X| were
+// integer products already).  Here three remain (coefficient, update) and
+// the integer ALU is the busiest pipe (63 % against FP64's 57 % in DRIFTP,
+// about 190 instructions a face in all): DRIFTR 64.5 -> 54.3 us, DRIFTP
+// 61.8 -> 48.3 us, on 40x49x70x144 DRIFTP 783 -> 598 us.  Normalising the
+// factor and the differences, as the FP64 form's integer products did, took
+// more instructions than aligning the cells once.
+//
+// Compiles for the host too (the arithmetic is tested on the CPU).
+#pragma once
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define RG_HD __host__ __device__ __forceinline__
+#else
+#define RG_HD static inline
+#endif
+
+namespace ramgpu {
+
+// v >> s with 0 for s >= 64 (also for s < 0 read as unsigned)
+RG_HD uint64_t shr_clamp(uint64_t v, int s) {
+#ifdef __CUDA_ARCH__
+  uint64_t r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+  return r;
+#else
+  return (unsigned)s > 63u ? 0ULL : v >> s;
+#endif
+}
+// position of the top set bit (-1 for 0)
+RG_HD int top_bit(uint32_t v) {
+#ifdef __CUDA_ARCH__
+  int r;
+  asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+#else
+  return v ? 31 - __builtin_clz(v) : -1;
+#endif
+}
+RG_HD uint32_t max3u(uint32_t a, uint32_t b, uint32_t c) {
+#ifdef __CUDA_ARCH__
+  return __vimax3_u32(a, b, c);
+#else
+  return a > b ? (a > c ? a : c) : (b > c ? b : c);
+#endif
+}
+// floor(x*y / 2^64) up to one unit low (the low halves' product is left
+// out), for x*y < 2^126 with x or y below 2^63 and the cross products' sum
+// below 2^64
+RG_HD uint64_t mulhi_cross(uint64_t x, uint64_t y) {
+  const uint32_t xh = (uint32_t)(x >> 32), xl = (uint32_t)x, yh = (uint32_t)(y >> 32), yl = (uint32_t)y;
+  const uint64_t t = (uint64_t)xh * yl + (uint64_t)xl * yh;
+  return (uint64_t)xh * yh + (uint32_t)(t >> 32);
+}
+// significand of a normal double with its top bit at 2^63 (sign and
+// exponent shift out), or at 2^62
+RG_HD uint64_t sig_top(uint64_t x) { return (x << 11) | 0x8000000000000000ULL; }
+RG_HD uint64_t sig_62(uint64_t x) { return ((x << 10) & 0x7FFFFFFFFFFFFFFFULL) | 0x4000000000000000ULL; }
+RG_HD int hi32(uint64_t x) { return (int)(x >> 32); }
+
+// (beta - 1) * 2^64 of the limiter's beta (1 <= beta <= 2; 2 gives 2^64 - 1)
+RG_HD uint64_t beta_fix(uint64_t beta_bits) {
+  return (beta_bits >> 52) >= 1024 ? ~0ULL : (beta_bits << 12);
+}
+// beta * v for v < 2^63
+RG_HD uint64_t beta_times(uint64_t v, uint64_t betaf) {
+  const uint32_t vh = (uint32_t)(v >> 32), vl = (uint32_t)v, bh = (uint32_t)(betaf >> 32), bl = (uint32_t)betaf;
+  uint64_t f = (uint64_t)vh * bh + (uint32_t)(((uint64_t)vl * bh) >> 32);
+  if (bl) f += ((uint64_t)vh * bl) >> 32;  // 0 for beta a multiple of 2^-32, e.g. 1.5
+  return v + f;
+}
+
+// The face coefficient C prepared for face_flux: its significand, exponent,
+// sign bit and (1 - U) * 2^63; `bad` is negative where the fixed point does
+// not hold (U >= 1, C infinite or NaN).
+struct FaceCoef {
+  uint64_t m;      // sig_62 of C
+  uint64_t a63;    // (1 - U) * 2^63
+  int e;           // biased exponent of C
+  uint32_t sign;   // sign bit of C
+  int bad;
+};
+// U = |C| (the R and P sweeps)
+RG_HD FaceCoef face_coef(uint64_t c) {
+  FaceCoef q;
+  const uint32_t h = (uint32_t)(c >> 32);
+  q.sign = h & 0x80000000u;
+  q.e = (int)((h >> 20) & 0x7FFu);
+  q.m = sig_62(c);
+  q.bad = 1022 - q.e;
+  q.a63 = 0x7FFFFFFFFFFFFFFFULL - shr_clamp(q.m, q.bad);
+  return q;
+}
+
+// Cells of 2^180 and more, and products phi below about 2^-820, take the FP64
+// form too: with those limits one sign test of the exponent of phi covers
+// every zero and subnormal operand.
+constexpr uint32_t kFaceTop = (1023u + 180u) << 20;
+constexpr int kFaceLow = 200;
+
+// phi as bits, from the bits of the cells.  kCase: cs is the limiter's
+// branch (0 upwind only, 1 beta*D, 2 X, 3 D, 4 beta*X).
+template <bool kCase>
+RG_HD uint64_t face_flux(uint64_t uu, uint64_t u, uint64_t d, const FaceCoef& q, uint64_t betaf, bool& special,
+                         int& cs) {
+  const uint32_t hu = (uint32_t)(u >> 32), hd = (uint32_t)(d >> 32), huu = (uint32_t)(uu >> 32);
+  const int eu = (int)(hu >> 20);
+  const uint64_t mu = ((u << 7) & 0x07FFFFFFFFFFFFFFULL) | 0x0800000000000000ULL;
+  const int sd = eu + 4 - (int)(hd >> 20), suu = eu + 4 - (int)(huu >> 20);
+  const uint64_t ad = shr_clamp(sig_top(d), sd > 1 ? sd : 1);
+  const uint64_t auu = shr_clamp(sig_top(uu), suu > 1 ? suu : 1);
+  const uint64_t X = ad - mu, D = mu - auu;
+  const int32_t s = hi32(X) >> 31;  // 0 or -1
+  const uint64_t sm = ((uint64_t)(uint32_t)s << 32) | (uint32_t)s;
+  // |X|, |D| where both have the sign s, one unit low when it is negative
+  const uint64_t ax = X ^ sm, adx = D ^ sm;
+  bool act = hi32(adx) >= 0;
+  bool undecided = false;
+  if (eu < 993) {
+    // |X| > 1e-27.  From eu = 993 (u >= 2^-30) on, a difference below the
+    // threshold is at most one unit here, whose correction is zero.  Below
+    // eu = 932 (u < 4.1e-28) only an increase to d > 1e-27 can be active.
+    const uint64_t thr = shr_clamp(0x9E74D1B791E08000ULL, eu > 930 ? eu - 929 : 1);  // sig_top of 1e-27
+    undecided = eu < 932 && hd >= 0x3A53CE9Au && act && s == 0;
+    act = act && eu >= 932 && ax > thr;
+  }
+  const bool dlo = adx <= ax;
+  const uint64_t lo = dlo ? adx : ax, hi = dlo ? ax : adx;
+  const uint64_t bl = beta_times(lo, betaf);
+  const uint64_t lim = bl < hi ? bl : hi;
+  if (kCase) {
+    const int c = dlo ? (bl <= hi ? 1 : 2) : (hi <= bl ? 3 : (betaf ? 4 : 2));
+    cs = (act && X != 0 && D != 0) ? c : 0;
+  }
+  const uint64_t corr = act ? mulhi_cross(lim, q.a63) : 0ULL;
+  const uint64_t fb = mu + (corr ^ sm) + (uint32_t)(-s);
+  const uint64_t p = mulhi_cross(fb, q.m);  // < 2^59
+  const int tb = top_bit((uint32_t)(p >> 32));
+  const int E = eu + q.e + tb - (1049 + kFaceLow);  // exponent field less one, less kFaceLow
+  const uint64_t t = p >> ((tb - 21) & 63);
+  const uint32_t top = max3u(hu, hd, huu);
+  special = top >= kFaceTop || undecided || (q.bad | E | hi32(fb) | (tb - 21)) < 0;
+  const uint32_t field = ((uint32_t)E << 20) + (q.sign + ((uint32_t)kFaceLow << 20));
+  return ((uint64_t)field << 32) + (t >> 1) + (t & 1ULL);
+}
+
+}  // namespace ramgpu

@@ -10,13 +10,15 @@
 //   DRIFTE  src/ModRamDrift.f90:285-376
 //   DRIFTMU src/ModRamDrift.f90:382-473
 // with the face coefficients taken from separable tables built in tables.cu
-// (C = A(I,J) + G(I,J,L)*k(K) etc.).  The FP64 unit is the limit: sign,
-// abs and limiter tests run on bit patterns, and the products that are only
-// compared (beta*|X|, the CFL quotients) and the flux C*FBND (mul_rn_int,
-// rounded exactly like the FP64 multiply) run on the integer pipe, leaving
-// 6 FP64 add/mul/fma per face.  More integer work than that made the
-// forward DRIFTE and DRIFTMU issue-bound (measured).
+// (C = A(I,J) + G(I,J,L)*k(K) etc.).  The FP64 unit was the limit: sign, abs
+// and limiter tests run on bit patterns; in DRIFTR and DRIFTP the whole face
+// flux is formed in 64-bit fixed point (face.cuh), which leaves three FP64
+// operations a face (the coefficient and the two of the update); in DRIFTE
+// and DRIFTMU the products that are only compared (beta*|X|, the CFL
+// quotients) and the flux C*FBND (mul_rn_int, rounded exactly like the FP64
+// multiply) run on the integer pipe, leaving 6 to 7.
 #include "ramgpu_internal.cuh"
+#include "face.cuh"
 #include "kernels.cuh"
 
 namespace ramgpu {
@@ -29,6 +31,48 @@ namespace ramgpu {
 __device__ __forceinline__ unsigned rget(const unsigned char* p, int rsh) { return (unsigned)*p >> rsh; }
 __device__ __forceinline__ void rput(unsigned char* p, int rsh, unsigned v) {
   *p = (unsigned char)(rsh ? (v << 4) : (*p | v));
+}
+
+// phi of a face by the FP64 unit, for what face_flux leaves out.  Out of
+// line, so that its FP64 instructions are not issued predicated off.
+// x, dd: the reference's X and D; kRec 2: with the branch rcs.
+struct PhiCase {
+  double phi;
+  int cs;
+};
+template <int kRec>
+static __device__ __noinline__ PhiCase face_phi_fp64(double x, double dd, double u, double c, double mh, double beta,
+                                                     int rcs) {
+  const BetaBits b(beta);
+  const bool neg = is_neg(c);
+  const double a = fma(c, mh, neg ? -0.5 : 0.5);
+  PhiCase r;
+  r.cs = rcs;
+  const double fb = kRec == 2 ? face_value_frozen(x, dd, u, a, b, rcs)
+                              : face_value_case(x, babs_bits(b, x), dd, babs_bits(b, dd), u, a, r.cs);
+  r.phi = __dmul_rn(c, fb);
+  return r;
+}
+
+// Flux of a limited face (face.cuh) with the prepared coefficient q of C.
+// mh: -1/2 (R, P) or -1/2 over the bin width.  kRec 1: cs is the branch
+// taken; 2: the recorded branch cs is applied (the same bits as the
+// recording sweep's where that is the branch the values select).
+template <int kRec>
+__device__ __forceinline__ double face_phi(double uu, double u, double d, double c, const FaceCoef& q, double mh,
+                                           double beta, uint64_t betaf, int& cs) {
+  bool special;
+  int taken = 0;
+  double phi = bitsd(face_flux<kRec == 1 || kRec == 2>(dbits(uu), dbits(u), dbits(d), q, betaf, special, taken));
+  if (kRec == 2) special = special || taken != cs;
+  if (kRec == 1) cs = taken;
+  if (special) {
+    const bool neg = hi32(dbits(c)) < 0;
+    const PhiCase r = face_phi_fp64<kRec>(neg ? u - d : d - u, neg ? uu - u : u - uu, u, c, mh, beta, cs);
+    phi = r.phi;
+    if (kRec == 1) cs = r.cs;
+  }
+  return phi;
 }
 
 // ----------------------------------------------------------------- DRIFTR
@@ -65,15 +109,15 @@ __global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned cha
       double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + (long long)line * nr;
       // branch record of the frozen-limiter adjoint: one byte per face/cell
       unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + (u / bpi) * d.ncell + (long long)line * nr : nullptr;
-      // face coefficients C and CORR factor a: stored by the forward sweep,
-      // read back by the reverse one (same DTs, same potential)
+      // face coefficients C: stored by the forward sweep, read back by the
+      // reverse one (same DTs, same potential)
       double* __restrict__ cst = kCo ? coef_ptr(d, 0, 0, u / bpi) + (long long)line * nr : nullptr;
-      double* __restrict__ ast = kCo ? coef_ptr(d, 0, 1, u / bpi) + (long long)line * nr : nullptr;
       const double* __restrict__ grt = d.grt + ((long long)l * nt + j) * nr;
       const double* __restrict__ cr = d.cr + ((long long)m * nt + j) * nr;
       const int* __restrict__ outside = d.outside + (long long)j * nr;
       const double p4 = d.p4[s * ne + (line / nt) % ne];
-      const BetaBits beta(d.betalim);
+      const double beta = d.betalim;
+      const uint64_t betaf = beta_fix(dbits(beta));
       const bool closed = d.flags & 1u;
 
       const int k = (line / nt) % ne;
@@ -98,43 +142,30 @@ __global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned cha
       if (kCfl && outside[0] == 0) q = umax64(q, cfl_bits(c, kBits1em10));
       // face 1: FBND(1) = 0 (outflow) or F(2) (inflow)
       double phi_prev = c * ((inflow && !closed) ? g0 : 0.0);
-      double xm = g0 - gm; bits64 bxm = babs_bits(beta, xm);
-      double x = gp - g0; bits64 bx = babs_bits(beta, x);
       for (int f = 2; f <= nr - 1; ++f) {  // 1-based face f, updates cell f
         const double gpp = (f + 2 <= nr) ? fl[f + 1] : g1;
-        const double xp = gpp - gp; const bits64 bxp = babs_bits(beta, xp);
         c = (kCo == 2) ? cst[f - 1] : ((f == nr - 1) ? cNm : fma(grt[f - 1], p4, cr[f - 1]));
+        if (kCo == 1) cst[f - 1] = c;
         if (kCfl && outside[f - 1] == 0) q = umax64(q, cfl_bits(c, kBits1em10));
-        const bool neg = is_neg(c);
-        const double a = (kCo == 2) ? ast[f - 1] : corr_a_int(dbits(c) & kAbsMask, neg, c, -0.5);
-        if (kCo == 1) { cst[f - 1] = c; ast[f - 1] = a; }
-        int cs;
-        const double fb = (kRec == 2)
-            ? face_value_frozen(x, neg ? xp : xm, neg ? gp : g0, a, beta, cs = rget(rl + (f - 1), rsh) & 7)
-            : face_value_case(x, bx, neg ? xp : xm, neg ? bxp : bxm, neg ? gp : g0, a, cs);
-        const double phi = mul_rn_int(c, fb);
+        const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
+        int cs = kRec == 2 ? (int)(rget(rl + (f - 1), rsh) & 7) : 0;
+        const double phi = face_phi<kRec>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), -0.5,
+                                          beta, betaf, cs);
         const double raw = (g0 - phi) + phi_prev;
         fl[f - 1] = (kRec == 2) ? clip_frozen(raw, rget(rl + (f - 1), rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
         if (kRec == 1) rput(rl + (f - 1), rsh, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
         gm = g0; g0 = gp; gp = gpp;
-        xm = x; bxm = bx; x = xp; bx = bxp;
       }
-      // face NR (g0 = F(NR), gp = F(NR+1), x = X(NR))
+      // face NR (g0 = F(NR), gp = F(NR+1)): limited on inflow lines, F(NR)
+      // on outflow lines
       if (kCfl && outside[nr - 1] == 0) q = umax64(q, cfl_bits(cN, kBits1em10));
-      double fbn;
-      int csn = 0;
-      if (!inflow) {
-        fbn = g0;
-      } else {
-        const double xp = g2 - g1; const bits64 bxp = babs_bits(beta, xp);
-        const double an = corr_a_int(dbits(cN) & kAbsMask, true, cN, -0.5);
-        fbn = (kRec == 2) ? face_value_frozen(x, xp, g1, an, beta, csn = rget(rl + (nr - 1), rsh) & 7)
-                          : face_value_case(x, bx, xp, bxp, g1, an, csn);
-      }
-      if (closed) fbn = 0.0;
-      const double phin = cN * fbn;
+      int csn = kRec == 2 ? (int)(rget(rl + (nr - 1), rsh) & 7) : 0;
+      double phin = 0.0;
+      if (!closed)
+        phin = inflow ? face_phi<kRec>(g2, g1, g0, cN, face_coef(dbits(cN)), -0.5, beta, betaf, csn)
+                      : mul_rn_int(cN, g0);
       const double rawn = (g0 - phin) + phi_prev;
       fl[nr - 1] = (kRec == 2) ? clip_frozen(rawn, rget(rl + (nr - 1), rsh)) : clip(rawn);
       if (kRec == kRecCount) nclip += is_neg(rawn);
@@ -182,74 +213,57 @@ __global__ void __launch_bounds__(256) k_sweep_p(Dev d, double dts, unsigned cha
       unsigned char* __restrict__ rl =
           (kRec == 1 || kRec == 2) ? rec + (u / bpi) * d.ncell + ((long long)kl * nt) * nr + i : nullptr;
       double* __restrict__ cst = kCo ? coef_ptr(d, 1, 0, u / bpi) + ((long long)kl * nt) * nr + i : nullptr;
-      double* __restrict__ ast = kCo ? coef_ptr(d, 1, 1, u / bpi) + ((long long)kl * nt) * nr + i : nullptr;
       const double* __restrict__ gpt = d.gpt + ((long long)l * nt) * nr + i;
       const double* __restrict__ ca = d.ca + ((long long)m * nt) * nr + i;
       const int* __restrict__ outside = d.outside + i;
       const double p2 = d.p2[((long long)s * ne + k) * nr + i];
-      const BetaBits beta(d.betalim);
+      const double beta = d.betalim;
+      const uint64_t betaf = beta_fix(dbits(beta));
   #define GJ(J) fl[(long long)((J)-1) * st]
   #define CJ(J) fma(gpt[(long long)((J)-1) * nr], p2, ca[(long long)((J)-1) * nr])
       const double G1 = GJ(1), G2 = GJ(2), G3 = GJ(3), GNm = GJ(nt - 1), GN = GJ(nt);
-      const double X1 = G2 - G1; const bits64 bX1 = babs_bits(beta, X1);
-      const double X2 = G3 - G2; const bits64 bX2 = babs_bits(beta, X2);
-      const double XNm = GN - GNm; const bits64 bXNm = babs_bits(beta, XNm);
-      const double XN = G2 - GN; const bits64 bXN = babs_bits(beta, XN);
       // face NT first: its flux enters cell 2 through FBND(1)=FBND(NT)
       const double cN = (kCo == 2) ? cst[(long long)(nt - 1) * st] : CJ(nt);
+      if (kCo == 1) cst[(long long)(nt - 1) * st] = cN;
       if (kCfl && outside[(long long)(nt - 1) * nr] == 0) q = umax64(q, cfl_bits(cN, kBits1em10));
-      double phiN;
-      int csN;
-      {
-        const bool neg = is_neg(cN);
-        const double a = (kCo == 2) ? ast[(long long)(nt - 1) * st] : corr_a_int(dbits(cN) & kAbsMask, neg, cN, -0.5);
-        if (kCo == 1) { cst[(long long)(nt - 1) * st] = cN; ast[(long long)(nt - 1) * st] = a; }
-        phiN = cN * ((kRec == 2)
-            ? face_value_frozen(XN, neg ? X2 : XNm, neg ? G2 : GN, a, beta, csN = rget(rl + (long long)(nt - 1) * st, rsh) & 7)
-            : face_value_case(XN, bXN, neg ? X2 : XNm, neg ? bX2 : bXNm, neg ? G2 : GN, a, csN));
-      }
+      int csN = kRec == 2 ? (int)(rget(rl + (long long)(nt - 1) * st, rsh) & 7) : 0;
+      const bool negN = is_neg(cN);
+      const double phiN = face_phi<kRec>(negN ? G3 : GNm, negN ? G2 : GN, negN ? GN : G2, cN, face_coef(dbits(cN)),
+                                         -0.5, beta, betaf, csN);
       double phi_prev = phiN;
-      double g0 = G2, gp = G3, xm = X1, x = X2;
-      bits64 bxm = bX1, bx = bX2;
+      double gm = G1, g0 = G2, gp = G3;
+      // The reference's D of face NT-1 against the flow is F(2)-F(1), with
+      // F(1) in the place of F(NT); the two differ only in states that are
+      // not periodic.
+      const bool oddwrap = dbits(G1) != dbits(GN);
       // the cell two faces ahead is loaded one iteration early, before this
       // face's store: the compiler cannot move a load past a store to the
       // line at a run-time stride (DRIFTR's contiguous lines come from L1)
       double nxt = GJ(4);
       for (int J = 2; J <= nt - 1; ++J) {
-        double gpp = 0.0, xp;
-        bits64 bxp;
         const double nn = GJ(min(J + 3, nt));
-        if (J <= nt - 3) {
-          gpp = nxt;
-          xp = gpp - gp;
-          bxp = babs_bits(beta, xp);
-        } else if (J == nt - 2) {
-          gpp = GN;
-          xp = XNm;
-          bxp = bXNm;
-        } else {  // J = NT-1: N = NT+1 wraps to 2, D = F(2)-F(1)
-          xp = X1;
-          bxp = bX1;
-        }
+        const double gpp = J == nt - 1 ? G2 : nxt;
         const double c = (kCo == 2) ? cst[(long long)(J - 1) * st] : CJ(J);
+        if (kCo == 1) cst[(long long)(J - 1) * st] = c;
         if (kCfl && outside[(long long)(J - 1) * nr] == 0) q = umax64(q, cfl_bits(c, kBits1em10));
-        const bool neg = is_neg(c);
-        const double a = (kCo == 2) ? ast[(long long)(J - 1) * st] : corr_a_int(dbits(c) & kAbsMask, neg, c, -0.5);
-        if (kCo == 1) { cst[(long long)(J - 1) * st] = c; ast[(long long)(J - 1) * st] = a; }
-        int cs;
+        const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
         const unsigned char* rj = (kRec == 1 || kRec == 2) ? rl + (long long)(J - 1) * st : nullptr;
-        const double fb = (kRec == 2)
-            ? face_value_frozen(x, neg ? xp : xm, neg ? gp : g0, a, beta, cs = rget(rj, rsh) & 7)
-            : face_value_case(x, bx, neg ? xp : xm, neg ? bxp : bxm, neg ? gp : g0, a, cs);
-        const double phi = mul_rn_int(c, fb);
+        int cs = kRec == 2 ? (int)(rget(rj, rsh) & 7) : 0;
+        double phi = face_phi<kRec>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), -0.5, beta,
+                                    betaf, cs);
+        if (J == nt - 1 && neg && oddwrap) {
+          const PhiCase r = face_phi_fp64<kRec>(gp - g0, G2 - G1, gp, c, -0.5, beta,
+                                                kRec == 2 ? (int)(rget(rj, rsh) & 7) : 0);
+          phi = r.phi;
+          cs = r.cs;
+        }
         const double raw = (g0 - phi) + phi_prev;
         GJ(J) = (kRec == 2) ? clip_frozen(raw, rget(rj, rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
         if (kRec == 1) rput(rl + ((long long)(J - 1) * st), rsh, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
-        g0 = gp; gp = gpp;
+        gm = g0; g0 = gp; gp = gpp;
         nxt = nn;
-        xm = x; bxm = bx; x = xp; bx = bxp;
       }
       const double rawN = (GN - phiN) + phi_prev;
       const double vN = (kRec == 2) ? clip_frozen(rawN, rget(rl + (long long)(nt - 1) * st, rsh)) : clip(rawN);
