@@ -362,13 +362,13 @@ int ramgpu_sum_pressure(ramgpu_ctx *ctx, int member, double *pallsum, double *pp
 
 /* ---- execution tuning (no reference counterpart) ------------------------ */
 
-/* Sweeps whose face coefficient C and CORR factor the forward half of a
- * ram_run call keeps for its reverse half, which then reads them instead of
- * recomputing them: bit 0 R, 1 P, 2 E, 3 MU.  Each set bit costs 16 bytes
- * per cell and (member, species) of device memory, taken only while it fits
- * in a quarter of the free memory.  Default 4 (DRIFTE only, whose C costs
- * two FP64 operations; for the other sweeps the stores cost more time than
- * the FP64 work they save).  Results are identical for every mask. */
+/* Whether the adjoint's first DRIFTE transpose of a call keeps its face
+ * coefficients for the second: bit 2 of mask (8 bytes per cell and (member,
+ * species) of device memory, taken by ramgpu_adj_backward only while it fits
+ * in a quarter of the free memory; default 4).  Bits 0, 1 and 3 are accepted
+ * and change nothing: the sweeps form their coefficients, one fma a face,
+ * faster than they would read stored ones.  Results are identical for every
+ * mask. */
 int ramgpu_set_coef_store(ramgpu_ctx *ctx, int mask);
 
 /* Replay ram_run / ram_run_async from a CUDA graph captured on first use and

@@ -63,10 +63,9 @@ struct ramgpu_ctx {
   bool have_grid = false, have_fields = false;
   bool field_dirty = true, static_dirty = true;
   double tables_dts = -1.0;
-  // sweeps (bit w: R, P, E, MU) whose face coefficients the forward half
-  // stores for the reverse half; measured on GB300, only DRIFTE (two FP64
-  // operations for C) gains, the others lose more to the stores than they
-  // save in FP64 work
+  // bit 2: a call's first DRIFTE transpose keeps its face coefficients for
+  // the second (the sweeps form theirs anew: one fma a face is cheaper than
+  // the stored value's traffic, DRIFTE 42 us loading against 33 forming it)
   unsigned coef_mask = 4u;
   // implicit pitch-angle diffusion: species with a coefficient, tables state
   std::vector<int> pd_on_h;
@@ -120,10 +119,8 @@ struct ramgpu_ctx {
   bool adj_overlap = true;
   cudaStream_t adj_stream = nullptr;
   void* adj_shadow = nullptr;
-  double* adj_shadow_coef = nullptr;  // the second stream's DRIFTE coefficient store
   void* adj_ring = nullptr;           // the transposes' per-call table sets
   std::vector<cudaEvent_t> adj_ring_events;
-  size_t adj_shadow_coef_bytes = 0;
   std::vector<cudaEvent_t> adj_events;
   // ramgpu_ram_run_host: item groups, their streams and events, and the
   // graph of the whole pipeline for one set of host buffers
@@ -291,7 +288,7 @@ static int rebuild_items(ramgpu_ctx* ctx) {
     CK(cudaMemcpyAsync(ctx->items_d, ctx->items_h.data(), sizeof(int2) * ctx->items_h.size(),
                        cudaMemcpyHostToDevice, ctx->stream));
   ctx->d.items = ctx->items_d;
-  ctx->d.nitems = (int)ctx->items_h.size();
+  ctx->d.nitems = ctx->d.nlist = (int)ctx->items_h.size();
   ctx->items_dirty = false;
   ctx->items_version += 1;
   return RAMGPU_OK;
@@ -352,26 +349,26 @@ static int prepare(ramgpu_ctx* ctx, double dts) {
     int rc = rebuild_items(ctx);
     if (rc) return rc;
   }
-  // face-coefficient store for the reverse half: 64 bytes per cell and item,
-  // kept only while it takes at most a quarter of the free device memory
-  if (ctx->coef_mask && ctx->d.coef_items < ctx->d.nitems) {
-    cudaFree(ctx->d.coef);
-    ctx->d.coef = nullptr;
-    ctx->d.coef_items = 0;
-    int nw = 0;
-    for (int w = 0; w < 4; ++w) ctx->d.coef_slot[w] = ((ctx->coef_mask >> w) & 1u) ? nw++ : -1;
-    const size_t need = (size_t)2 * nw * ctx->d.nitems * ctx->d.ncell * sizeof(double);
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && need <= fr / 4 &&
-        cudaMalloc(&ctx->d.coef, need) == cudaSuccess) {
-      ctx->d.coef_items = ctx->d.nitems;
-    } else {
-      ctx->d.coef = nullptr;
-      cudaGetLastError();
-    }
-    ctx->shape_version += 1;  // launch sequence changed: recapture the graph
-  }
   return RAMGPU_OK;
+}
+
+// The DRIFTE coefficient store of the adjoint's transposes: 8 bytes per cell
+// and item, kept only while it takes at most a quarter of the free device
+// memory.
+static void ensure_coef(ramgpu_ctx* ctx) {
+  Dev& d = ctx->d;
+  if (!(ctx->coef_mask & 4u) || d.coef_items >= d.nitems) return;
+  cudaFree(d.coef);
+  d.coef = nullptr;
+  d.coef_items = 0;
+  const size_t need = (size_t)d.nitems * d.ncell * sizeof(double);
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && need <= fr / 4 && cudaMalloc(&d.coef, need) == cudaSuccess) {
+    d.coef_items = d.nitems;
+  } else {
+    d.coef = nullptr;
+    cudaGetLastError();
+  }
 }
 
 // SUMRC of every item into stage buffer `stage`, then fold into the device
@@ -408,11 +405,10 @@ static int enqueue_forward(ramgpu_ctx* ctx, double dts, bool loss_fused, const d
   if (clear_cfl)
     CK(cudaMemsetAsync(ctx->d.cflq, 0, sizeof(unsigned long long) * 5 * ctx->d.nm * ctx->d.ns, ctx->stream));
   const Dev& d = ctx->d;
-  auto co = [&](int w) { return (d.coef && d.coef_slot[w] >= 0) ? 1 : 0; };
-  { Timed t(ctx, 2); launch_sweep_r(d, dts, true, ctx->stream, nullptr, false, co(0)); }
-  { Timed t(ctx, 3); launch_sweep_p(d, dts, true, ctx->stream, nullptr, false, co(1)); }
-  { Timed t(ctx, 4); launch_sweep_e(d, dts, true, ctx->stream, nullptr, false, co(2)); }
-  { Timed t(ctx, 5); launch_sweep_mu(d, dts, true, loss_fused ? 1 : 0, loss_table, ctx->stream, nullptr, false, co(3)); }
+  { Timed t(ctx, 2); launch_sweep_r(d, dts, true, ctx->stream); }
+  { Timed t(ctx, 3); launch_sweep_p(d, dts, true, ctx->stream); }
+  { Timed t(ctx, 4); launch_sweep_e(d, dts, true, ctx->stream); }
+  { Timed t(ctx, 5); launch_sweep_mu(d, dts, true, loss_fused ? 1 : 0, loss_table, ctx->stream); }
   ctx->launches += 4;
   CKL("forward sweeps");
   return RAMGPU_OK;
@@ -423,11 +419,10 @@ static int enqueue_forward(ramgpu_ctx* ctx, double dts, bool loss_fused, const d
 static int enqueue_reverse(ramgpu_ctx* ctx, double dts, bool loss_fused, const double* loss_table,
                            bool after_forward) {
   const Dev& d = ctx->d;
-  auto co = [&](int w) { return (after_forward && d.coef && d.coef_slot[w] >= 0) ? 2 : 0; };
-  { Timed t(ctx, 5); launch_sweep_mu(d, dts, false, loss_fused ? 2 : 0, loss_table, ctx->stream, nullptr, false, co(3)); }
-  { Timed t(ctx, 4); launch_sweep_e(d, dts, false, ctx->stream, nullptr, false, co(2)); }
-  { Timed t(ctx, 3); launch_sweep_p(d, dts, false, ctx->stream, nullptr, false, co(1)); }
-  { Timed t(ctx, 2); launch_sweep_r(d, dts, false, ctx->stream, nullptr, false, co(0)); }
+  { Timed t(ctx, 5); launch_sweep_mu(d, dts, false, loss_fused ? 2 : 0, loss_table, ctx->stream); }
+  { Timed t(ctx, 4); launch_sweep_e(d, dts, false, ctx->stream); }
+  { Timed t(ctx, 3); launch_sweep_p(d, dts, false, ctx->stream); }
+  { Timed t(ctx, 2); launch_sweep_r(d, dts, false, ctx->stream); }
   ctx->launches += 4;
   CKL("reverse sweeps");
   return RAMGPU_OK;
@@ -588,21 +583,18 @@ static int enqueue_call_rec(ramgpu_ctx* ctx, double dts, unsigned char* rec, boo
   ctx->launches += 3;
   const int G = clamp_groups(ctx, ctx->step_groups);
   if (int rc = ensure_group_streams(ctx, G)) return rc;
-  // DRIFTE keeps its face coefficients for the reverse half as in the plain
-  // step (same DTs and VT within a call)
-  const int co_e = (ctx->d.coef && ctx->d.coef_slot[2] >= 0) ? 1 : 0;
   return over_groups(ctx, G, [&](int i0) {
     const Dev& d = ctx->d;
     const cudaStream_t st = ctx->stream;
     unsigned char* r = rec + (size_t)i0 * d.ncell;
-    launch_sweep_r(d, dts, false, st, r + 0 * isz, false, 0, 4);
-    launch_sweep_p(d, dts, false, st, r + 1 * isz, false, 0, 4);
-    launch_sweep_e(d, dts, false, st, r + 2 * isz, false, co_e, 4);
-    launch_sweep_mu(d, dts, false, 1, d.loss2, st, r + 3 * isz, false, 0, 4);
-    launch_sweep_mu(d, dts, false, 0, nullptr, st, r + 3 * isz, false, 0, 0);
-    launch_sweep_e(d, dts, false, st, r + 2 * isz, false, 2 * co_e, 0);
-    launch_sweep_p(d, dts, false, st, r + 1 * isz, false, 0, 0);
-    launch_sweep_r(d, dts, false, st, r + 0 * isz, false, 0, 0);
+    launch_sweep_r(d, dts, false, st, r + 0 * isz, false, 4);
+    launch_sweep_p(d, dts, false, st, r + 1 * isz, false, 4);
+    launch_sweep_e(d, dts, false, st, r + 2 * isz, false, 4);
+    launch_sweep_mu(d, dts, false, 1, d.loss2, st, r + 3 * isz, false, 4);
+    launch_sweep_mu(d, dts, false, 0, nullptr, st, r + 3 * isz, false, 0);
+    launch_sweep_e(d, dts, false, st, r + 2 * isz, false, 0);
+    launch_sweep_p(d, dts, false, st, r + 1 * isz, false, 0);
+    launch_sweep_r(d, dts, false, st, r + 0 * isz, false, 0);
     launch_finish(d, st);
     if (moments) launch_moments(d, st);
     else launch_anisch_state(d, st);
@@ -625,14 +617,14 @@ static int enqueue_call_replay(ramgpu_ctx* ctx, double dts, unsigned char* rec) 
     const Dev& d = ctx->d;
     const cudaStream_t st = ctx->stream;
     unsigned char* r = rec + (size_t)i0 * d.ncell;
-    launch_sweep_r(d, dts, false, st, r + 0 * isz, true, 0, 4);
-    launch_sweep_p(d, dts, false, st, r + 1 * isz, true, 0, 4);
-    launch_sweep_e(d, dts, false, st, r + 2 * isz, true, 0, 4);
-    launch_sweep_mu(d, dts, false, 1, d.loss2, st, r + 3 * isz, true, 0, 4);
-    launch_sweep_mu(d, dts, false, 0, nullptr, st, r + 3 * isz, true, 0, 0);
-    launch_sweep_e(d, dts, false, st, r + 2 * isz, true, 0, 0);
-    launch_sweep_p(d, dts, false, st, r + 1 * isz, true, 0, 0);
-    launch_sweep_r(d, dts, false, st, r + 0 * isz, true, 0, 0);
+    launch_sweep_r(d, dts, false, st, r + 0 * isz, true, 4);
+    launch_sweep_p(d, dts, false, st, r + 1 * isz, true, 4);
+    launch_sweep_e(d, dts, false, st, r + 2 * isz, true, 4);
+    launch_sweep_mu(d, dts, false, 1, d.loss2, st, r + 3 * isz, true, 4);
+    launch_sweep_mu(d, dts, false, 0, nullptr, st, r + 3 * isz, true, 0);
+    launch_sweep_e(d, dts, false, st, r + 2 * isz, true, 0);
+    launch_sweep_p(d, dts, false, st, r + 1 * isz, true, 0);
+    launch_sweep_r(d, dts, false, st, r + 0 * isz, true, 0);
     launch_finish(d, st);
     launch_anisch_state(d, st);
     ctx->launches += 10;
@@ -835,7 +827,6 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
   auto lo = [&](int c) { return (int)((long long)npa * c / C); };
   cudaEvent_t* ev = ctx->chunk_events.data();
   cudaEvent_t ev_start = ev[3 * C], ev_tab = ev[3 * C + 1], ev_mu = ev[3 * C + 2];
-  auto co = [&](int w, int k) { return (full.coef && full.coef_slot[w] >= 0) ? k : 0; };
   int rc = RAMGPU_OK;
   CK(cudaEventRecord(ev_start, main));
   if ((rc = enqueue_tables(ctx, dts))) return rc;
@@ -850,9 +841,9 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
     Dev dc = full;
     dc.lw0 = lo(c);
     dc.lw1 = lo(c + 1);
-    { NvtxRange r("DRIFTR"); launch_sweep_r(dc, dts, true, st, nullptr, false, co(0, 1)); }
-    { NvtxRange r("DRIFTP"); launch_sweep_p(dc, dts, true, st, nullptr, false, co(1, 1)); }
-    { NvtxRange r("DRIFTE"); launch_sweep_e(dc, dts, true, st, nullptr, false, co(2, 1)); }
+    { NvtxRange r("DRIFTR"); launch_sweep_r(dc, dts, true, st); }
+    { NvtxRange r("DRIFTP"); launch_sweep_p(dc, dts, true, st); }
+    { NvtxRange r("DRIFTE"); launch_sweep_e(dc, dts, true, st); }
     ctx->launches += 3;
     CKL("chunk forward sweeps");
     CK(cudaEventRecord(ev[3 * c + 1], st));
@@ -860,8 +851,8 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
   }
   {
     NvtxRange r("DRIFTMU");
-    launch_sweep_mu(full, dts, true, 1, full.loss2, main, nullptr, false, co(3, 1));
-    launch_sweep_mu(full, dts, false, 0, nullptr, main, nullptr, false, co(3, 2));
+    launch_sweep_mu(full, dts, true, 1, full.loss2, main);
+    launch_sweep_mu(full, dts, false, 0, nullptr, main);
     ctx->launches += 2;
     CKL("pitch-angle sweeps");
   }
@@ -872,9 +863,9 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
     Dev dc = full;
     dc.lw0 = lo(c);
     dc.lw1 = lo(c + 1);
-    { NvtxRange r("DRIFTE"); launch_sweep_e(dc, dts, false, st, nullptr, false, co(2, 2)); }
-    { NvtxRange r("DRIFTP"); launch_sweep_p(dc, dts, false, st, nullptr, false, co(1, 2)); }
-    { NvtxRange r("DRIFTR"); launch_sweep_r(dc, dts, false, st, nullptr, false, co(0, 2)); }
+    { NvtxRange r("DRIFTE"); launch_sweep_e(dc, dts, false, st); }
+    { NvtxRange r("DRIFTP"); launch_sweep_p(dc, dts, false, st); }
+    { NvtxRange r("DRIFTR"); launch_sweep_r(dc, dts, false, st); }
     launch_finish(dc, st);
     ctx->launches += 4;
     CKL("chunk reverse sweeps");
@@ -1021,6 +1012,12 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   const size_t nr = d.nr, nt = d.nt, ne = d.ne, npa = d.npa, ns = d.ns, nm = d.nm, nf = d.nf;
   const size_t nijl = nr * nt * npa, nfield = nf * nt * npa, nslot = nm * ns;
   bool ok = true;
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      ok = false;
+  }
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) ok = false;
   ctx->own_stream = ok;
   d.lz = dalloc<double>(ctx, nf, &ok); d.rlz = dalloc<double>(ctx, nf, &ok);
@@ -1032,7 +1029,7 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   d.wmu = dalloc<double>(ctx, npa, &ok);
   d.upa_atm = dalloc<int>(ctx, nr, &ok); d.upa_mom = dalloc<int>(ctx, nr, &ok);
   d.mhde = dalloc<double>(ctx, ne, &ok); d.iwe = dalloc<double>(ctx, ne, &ok);
-  d.ide = dalloc<double>(ctx, ne, &ok);
+  d.ide = dalloc<double>(ctx, ne + 1, &ok);
   d.mhdmu = dalloc<double>(ctx, npa, &ok); d.iwmu = dalloc<double>(ctx, npa, &ok);
   d.idmu = dalloc<double>(ctx, npa, &ok);
   d.bmhde = dalloc<double>(ctx, ne, &ok); d.bmhdmu = dalloc<double>(ctx, npa, &ok);
@@ -1065,6 +1062,8 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   d.p2 = dalloc<double>(ctx, ns * ne * nr, &ok); d.edot = dalloc<double>(ctx, ns * ne * nr, &ok);
   d.eb = dalloc<double>(ctx, ns * ne, &ok); d.ek = dalloc<double>(ctx, ns * ne, &ok);
   d.kap = dalloc<double>(ctx, ns * 2, &ok);
+  d.ebin = dalloc<FaceBin>(ctx, ns * ne, &ok);
+  d.er = dalloc<double>(ctx, nr, &ok); d.erq = dalloc<double>(ctx, ns * nr, &ok);
   d.loss1 = dalloc<double>(ctx, ns * ncell, &ok); d.loss2 = dalloc<double>(ctx, ns * ncell, &ok);
   d.charge = dalloc<double>(ctx, ns * ncell, &ok); d.atm = dalloc<double>(ctx, ns * ncell, &ok);
   d.kp = dalloc<double>(ctx, nm, &ok); d.vt_mode = dalloc<int>(ctx, nm, &ok);
@@ -1149,7 +1148,6 @@ int ramgpu_destroy(ramgpu_ctx* ctx) {
   for (cudaEvent_t e : ctx->adj_events) cudaEventDestroy(e);
   if (ctx->adj_stream) cudaStreamDestroy(ctx->adj_stream);
   cudaFree(ctx->adj_shadow);
-  cudaFree(ctx->adj_shadow_coef);
   cudaFree(ctx->adj_ring);
   for (cudaEvent_t e : ctx->adj_ring_events) cudaEventDestroy(e);
   if (ctx->status_h) cudaFreeHost(ctx->status_h);
@@ -1221,10 +1219,11 @@ int ramgpu_set_grid(ramgpu_ctx* ctx, const ramgpu_grid* g) {
   }
   CK(cudaMemcpy((void*)d.upa_atm, ua.data(), sizeof(int) * nr, cudaMemcpyHostToDevice));
   CK(cudaMemcpy((void*)d.upa_mom, um.data(), sizeof(int) * nr, cudaMemcpyHostToDevice));
-  std::vector<double> r1(ne), r2(ne), r3(ne), q1(npa), q2(npa), q3(npa);
+  std::vector<double> r1(ne), r2(ne), r3(ne + 1), q1(npa), q2(npa), q3(npa);
   for (int k = 0; k < ne; ++k) { r1[k] = -0.5 / G.de[k]; r2[k] = 1.0 / G.we[k]; r3[k] = 1.0 / G.de[k]; }
+  r3[ne] = *std::max_element(r3.begin(), r3.begin() + ne);
   for (int l = 0; l < npa; ++l) { q1[l] = -0.5 / G.dmu[l]; q2[l] = 1.0 / G.wmu[l]; q3[l] = 1.0 / G.dmu[l]; }
-  CK(up(d.mhde, r1.data(), ne)); CK(up(d.iwe, r2.data(), ne)); CK(up(d.ide, r3.data(), ne));
+  CK(up(d.mhde, r1.data(), ne)); CK(up(d.iwe, r2.data(), ne)); CK(up(d.ide, r3.data(), ne + 1));
   CK(up(d.mhdmu, q1.data(), npa)); CK(up(d.iwmu, q2.data(), npa)); CK(up(d.idmu, q3.data(), npa));
   for (int k = 0; k < ne; ++k) r1[k] *= d.betalim;
   for (int l = 0; l < npa; ++l) q1[l] *= d.betalim;
@@ -3143,20 +3142,7 @@ static int adj_shadow_prepare(ramgpu_ctx* ctx, Dev& q) {
   }
   q = d;
   table_set_assign(ctx->adj_shadow, q);
-  q.coef = nullptr;
-  if (d.coef) {
-    int nw = 0;
-    for (int w = 0; w < 4; ++w) nw += d.coef_slot[w] >= 0 ? 1 : 0;
-    const size_t need = (size_t)2 * nw * d.coef_items * d.ncell * sizeof(double);
-    if (ctx->adj_shadow_coef_bytes != need) {
-      cudaFree(ctx->adj_shadow_coef);
-      ctx->adj_shadow_coef = nullptr;
-      ctx->adj_shadow_coef_bytes = 0;
-      if (cudaMalloc(&ctx->adj_shadow_coef, need) == cudaSuccess) ctx->adj_shadow_coef_bytes = need;
-      else { ctx->adj_shadow_coef = nullptr; cudaGetLastError(); }
-    }
-    q.coef = ctx->adj_shadow_coef;
-  }
+  q.coef = nullptr;  // the transposes' alone
   q.count_clips = 0;
   return RAMGPU_OK;
 }
@@ -3192,17 +3178,16 @@ static int adj_recompute_call(ramgpu_ctx* ctx, const Dev& q, cudaStream_t st, in
   Dev qc = q;  // Kp of the call read from the window's array
   qc.kp = ctx->adj.kp_d + (size_t)call * ctx->cfg.n_members;
   const size_t isz = (size_t)q.nitems * q.ncell;
-  const int co_e = (q.coef && q.coef_slot[2] >= 0) ? 1 : 0;
   launch_member_coef(qc, dts, st);
   launch_ghost(q, st);
-  launch_sweep_r(q, dts, false, st, rec + 0 * isz, false, 0, 4);
-  launch_sweep_p(q, dts, false, st, rec + 1 * isz, false, 0, 4);
-  launch_sweep_e(q, dts, false, st, rec + 2 * isz, false, co_e, 4);
-  launch_sweep_mu(q, dts, false, 1, q.loss2, st, rec + 3 * isz, false, 0, 4);
-  launch_sweep_mu(q, dts, false, 0, nullptr, st, rec + 3 * isz, false, 0, 0);
-  launch_sweep_e(q, dts, false, st, rec + 2 * isz, false, 2 * co_e, 0);
-  launch_sweep_p(q, dts, false, st, rec + 1 * isz, false, 0, 0);
-  launch_sweep_r(q, dts, false, st, rec + 0 * isz, false, 0, 0);
+  launch_sweep_r(q, dts, false, st, rec + 0 * isz, false, 4);
+  launch_sweep_p(q, dts, false, st, rec + 1 * isz, false, 4);
+  launch_sweep_e(q, dts, false, st, rec + 2 * isz, false, 4);
+  launch_sweep_mu(q, dts, false, 1, q.loss2, st, rec + 3 * isz, false, 4);
+  launch_sweep_mu(q, dts, false, 0, nullptr, st, rec + 3 * isz, false, 0);
+  launch_sweep_e(q, dts, false, st, rec + 2 * isz, false, 0);
+  launch_sweep_p(q, dts, false, st, rec + 1 * isz, false, 0);
+  launch_sweep_r(q, dts, false, st, rec + 0 * isz, false, 0);
   launch_finish(q, st);
   launch_anisch_state(q, st);
   ctx->launches += 13;
@@ -3226,7 +3211,8 @@ int ramgpu_adj_backward(ramgpu_ctx* ctx, double* grad_f2, double* grad_fgeos) {
   if ((rc = ensure_group_streams(ctx, G))) return rc;
   // the first DRIFTE transpose of each call keeps its face coefficients in
   // the DRIFTE coefficient store for the second
-  const int co_e = (d.coef && d.coef_slot[2] >= 0) ? 1 : 0;
+  ensure_coef(ctx);
+  const int co_e = d.coef ? 1 : 0;
   CK(cudaMemsetAsync(d.lam, 0, sizeof(double) * nslot * d.ncell, ctx->stream));
   CK(cudaMemsetAsync(d.gfg, 0, sizeof(double) * nslot * nfg, ctx->stream));
   // The records of the last nkeep segments are still the forward pass's

@@ -454,8 +454,7 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
       continue;
     double* __restrict__ lam = d.lam + (long long)slot * d.ncell + base;
     const unsigned char* __restrict__ rl = rec + (u / bpi) * d.ncell + base;
-    double* __restrict__ cst = kCo ? coef_ptr(d, 2, 0, u / bpi) + base : nullptr;
-    double* __restrict__ csa = kCo ? coef_ptr(d, 2, 1, u / bpi) + base : nullptr;
+    double* __restrict__ cst = kCo ? coef_ptr(d, u / bpi) + base : nullptr;
     const long long fij = ((long long)l * nt + j) * nr + i;
     const double wet = d.wet[fij];
     const double ue = d.ue[(long long)m * nr * nt * d.npa + fij];
@@ -477,16 +476,8 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
       if (kCo == 1) cst[(long long)(K - 1) * st] = C;
       const bool neg = is_neg(C);
       const int cs = (rl[(long long)(K - 1) * st] >> rsh) & 7;
-      if (kAdjIntMask & 4u) {
-        // the CORR factor a too goes to the store (case-free: each transpose
-        // applies its own record's k)
-        const bits64 a = (kCo == 2) ? dbits(csa[(long long)(K - 1) * st]) : corr_a_fix(courant_u(C, d.ide[K - 1]), neg);
-        if (kCo == 1) csa[(long long)(K - 1) * st] = bitsd(a);
-        face_acc_a(C * (wl1 - wl0), neg, cs, a, beta, cm1, c0, c1, c2);
-      } else {
-        face_acc(adj_mul(kCo == 2 ? 0u : 4u, C, wl1 - wl0), neg, cs,
-                 face_ak<true>(C, neg, cs, d.mhde[K - 1], d.bmhde[K - 1], hb), cm1, c0, c1, c2);
-      }
+      face_acc(adj_mul(kCo == 2 ? 0u : 4u, C, wl1 - wl0), neg, cs,
+               face_ak<true>(C, neg, cs, d.mhde[K - 1], d.bmhde[K - 1], hb), cm1, c0, c1, c2);
     };
     auto shift = [&](double lec, double wl) {
       cm1 = c0; c0 = c1; c1 = c2; c2 = lec;

@@ -22,15 +22,18 @@
 // more, a zero C and the extremes of the exponent range report `special`;
 // the caller takes the FP64 form there.
 //
-// Bound and figures (GB300, four species on 20x25x35x72, one launch): the
-// FP64 sequence held the FP64 pipe, five operations a face (coefficient, X,
-// the limited correction, two for the update; phi, a and beta|X| were
-// integer products already).  Here three remain (coefficient, update) and
-// the integer ALU is the busiest pipe (63 % against FP64's 57 % in DRIFTP,
-// about 190 instructions a face in all): DRIFTR 64.5 -> 54.3 us, DRIFTP
-// 61.8 -> 48.3 us, on 40x49x70x144 DRIFTP 783 -> 598 us.  Normalising the
-// factor and the differences, as the FP64 form's integer products did, took
-// more instructions than aligning the cells once.
+// Bound and figures (GB300, one launch over four species on 20x25x35x72): the
+// FP64 sequence held the FP64 pipe, five operations a face in DRIFTR and
+// DRIFTP and up to seven in DRIFTE (phi, beta|X| and the Courant products
+// were integer products already).  Here three remain (the coefficient's fma
+// and the update); instruction issue (55-64 %, 170-210 instructions a face),
+// the integer ALU (60 %) and the FP64 pipe (58 %) are about even.  DRIFTR
+// 64.5 -> 52.1 us, DRIFTP 61.8 -> 46.9, DRIFTE 66.8 -> 54.4; on 40x49x70x144
+// DRIFTP 783 -> 543, DRIFTE 875 -> 580.  Normalising the factor and the
+// differences, as the FP64 form's integer products did, took more
+// instructions than aligning the cells once.  The rare forms must stay rare:
+// before face_plain and the exact threshold below, eight warps of meridian
+// lines with C = 0 made the whole DRIFTE launch 71 us.
 //
 // Compiles for the host too (the arithmetic is tested on the CPU).
 #pragma once
@@ -71,13 +74,33 @@ RG_HD uint32_t max3u(uint32_t a, uint32_t b, uint32_t c) {
   return a > b ? (a > c ? a : c) : (b > c ? b : c);
 #endif
 }
+// smaller and larger of a and b, and whether a is the smaller (or equal):
+// one comparison (from min/max expressions the compiler makes two)
+RG_HD bool sort2(uint64_t a, uint64_t b, uint64_t& lo, uint64_t& hi) {
+#ifdef __CUDA_ARCH__
+  int le;
+  asm("{ .reg .pred p; setp.le.u64 p, %3, %4; selp.b64 %0, %3, %4, p; selp.b64 %1, %4, %3, p; selp.s32 %2, 1, 0, p; }"
+      : "=&l"(lo), "=&l"(hi), "=r"(le) : "l"(a), "l"(b));
+  return le != 0;
+#else
+  lo = a <= b ? a : b;
+  hi = a <= b ? b : a;
+  return a <= b;
+#endif
+}
 // floor(x*y / 2^64) up to one unit low (the low halves' product is left
-// out), for x*y < 2^126 with x or y below 2^63 and the cross products' sum
-// below 2^64
+// out), for x, y whose cross products sum below 2^64
 RG_HD uint64_t mulhi_cross(uint64_t x, uint64_t y) {
   const uint32_t xh = (uint32_t)(x >> 32), xl = (uint32_t)x, yh = (uint32_t)(y >> 32), yl = (uint32_t)y;
   const uint64_t t = (uint64_t)xh * yl + (uint64_t)xl * yh;
+#ifdef __CUDA_ARCH__
+  uint32_t rl, rh;
+  asm("mad.lo.cc.u32 %0, %2, %3, %4; madc.hi.u32 %1, %2, %3, 0;"
+      : "=r"(rl), "=r"(rh) : "r"(xh), "r"(yh), "r"((uint32_t)(t >> 32)));
+  return ((uint64_t)rh << 32) | rl;
+#else
   return (uint64_t)xh * yh + (uint32_t)(t >> 32);
+#endif
 }
 // significand of a normal double with its top bit at 2^63 (sign and
 // exponent shift out), or at 2^62
@@ -85,29 +108,32 @@ RG_HD uint64_t sig_top(uint64_t x) { return (x << 11) | 0x8000000000000000ULL; }
 RG_HD uint64_t sig_62(uint64_t x) { return ((x << 10) & 0x7FFFFFFFFFFFFFFFULL) | 0x4000000000000000ULL; }
 RG_HD int hi32(uint64_t x) { return (int)(x >> 32); }
 
-// (beta - 1) * 2^64 of the limiter's beta (1 <= beta <= 2; 2 gives 2^64 - 1)
+// (beta - 1) * 2^64 of the limiter's beta (1 <= beta <= 2; 2 gives 2^64 - 1).
+// kB32: its low word is zero (beta a multiple of 2^-32, e.g. 1.5), which
+// saves a product; the launchers choose the form.
 RG_HD uint64_t beta_fix(uint64_t beta_bits) {
   return (beta_bits >> 52) >= 1024 ? ~0ULL : (beta_bits << 12);
 }
 // beta * v for v < 2^63
+template <bool kB32>
 RG_HD uint64_t beta_times(uint64_t v, uint64_t betaf) {
   const uint32_t vh = (uint32_t)(v >> 32), vl = (uint32_t)v, bh = (uint32_t)(betaf >> 32), bl = (uint32_t)betaf;
   uint64_t f = (uint64_t)vh * bh + (uint32_t)(((uint64_t)vl * bh) >> 32);
-  if (bl) f += ((uint64_t)vh * bl) >> 32;  // 0 for beta a multiple of 2^-32, e.g. 1.5
+  if (!kB32) f += ((uint64_t)vh * bl) >> 32;
   return v + f;
 }
 
-// The face coefficient C prepared for face_flux: its significand, exponent,
+// The face coefficient prepared for face_flux: C = +-m 2^-62 2^(e-1023), its
 // sign bit and (1 - U) * 2^63; `bad` is negative where the fixed point does
 // not hold (U >= 1, C infinite or NaN).
 struct FaceCoef {
-  uint64_t m;      // sig_62 of C
+  uint64_t m;      // [2^61, 2^63)
   uint64_t a63;    // (1 - U) * 2^63
-  int e;           // biased exponent of C
+  int e;           // exponent
   uint32_t sign;   // sign bit of C
   int bad;
 };
-// U = |C| (the R and P sweeps)
+// From C with U = |C| (the R and P sweeps).
 RG_HD FaceCoef face_coef(uint64_t c) {
   FaceCoef q;
   const uint32_t h = (uint32_t)(c >> 32);
@@ -118,16 +144,75 @@ RG_HD FaceCoef face_coef(uint64_t c) {
   q.a63 = 0x7FFFFFFFFFFFFFFFULL - shr_clamp(q.m, q.bad);
   return q;
 }
+// DRIFTE's coefficient is C = k*v with k > 0 from the energy bin and v from
+// the line, U = |v|*(k/DE): both products are formed here from v.
+struct alignas(16) FaceBin {
+  double k, iw;         // k and 1/WE of the bin
+  uint64_t sk, sy;      // sig_62 of k and of k/DE
+  int e, sh;            // exponent of k less 1022; 2045 less that of k/DE
+  double pad;
+};
+// prod: the significands' product of U, 2^62 <= prod < 2^64, for face_courant.
+RG_HD FaceCoef face_coef_bin(uint64_t v, const FaceBin& b, uint64_t& prod) {
+  FaceCoef q;
+  const uint32_t h = (uint32_t)(v >> 32);
+  const int ev = (int)((h >> 20) & 0x7FFu);
+  const uint64_t sv = sig_62(v);
+  q.sign = h & 0x80000000u;
+  q.e = ev + b.e;
+  q.m = mulhi_cross(sv, b.sk) << 1;
+  prod = mulhi_cross(sv, b.sy) << 2;
+  const int sh = b.sh - ev;
+  q.a63 = 0x7FFFFFFFFFFFFFFFULL - shr_clamp(prod, sh);
+  q.bad = sh | hi32(q.a63) | (2046 - ev);
+  return q;
+}
+// DRIFTMU's coefficient C comes whole; U = C/DMU.
+struct alignas(16) FaceMu {
+  double iw;            // 1/WMU of the bin
+  uint64_t sy;          // sig_62 of 1/DMU
+  int sh, pad0;         // 2045 less the exponent of 1/DMU
+  double pad1;
+};
+RG_HD FaceCoef face_coef_mu(uint64_t c, const FaceMu& b, uint64_t& prod) {
+  FaceCoef q;
+  const uint32_t h = (uint32_t)(c >> 32);
+  q.sign = h & 0x80000000u;
+  q.e = (int)((h >> 20) & 0x7FFu);
+  q.m = sig_62(c);
+  prod = mulhi_cross(q.m, b.sy) << 2;
+  const int sh = b.sh - q.e;
+  q.a63 = 0x7FFFFFFFFFFFFFFFULL - shr_clamp(prod, sh);
+  q.bad = sh | hi32(q.a63) | (2046 - q.e);
+  return q;
+}
+// U as bits, cut to 53 bits: 0 where v is zero or subnormal or U underflows,
+// |v| itself where it is infinite or NaN.
+RG_HD uint64_t face_courant(uint64_t v, int sh, uint64_t prod) {
+  const int ev = (int)((v >> 52) & 0x7FFu), top = (int)(prod >> 63);
+  const int e = ev + 1022 - sh + top;
+  const uint64_t r = ((uint64_t)(uint32_t)e << 52) | ((prod >> (10 + top)) & 0x000FFFFFFFFFFFFFULL);
+  return ev == 0x7FF ? (v & 0x7FFFFFFFFFFFFFFFULL) : (ev == 0 || e <= 0 ? 0ULL : r);
+}
 
-// Cells of 2^180 and more, and products phi below about 2^-820, take the FP64
-// form too: with those limits one sign test of the exponent of phi covers
-// every zero and subnormal operand.
-constexpr uint32_t kFaceTop = (1023u + 180u) << 20;
-constexpr int kFaceLow = 200;
+// Cells of 2^100 and more, and products phi below about 2^-919, are special
+// too: with those limits one sign test of the exponent of phi covers every
+// zero and subnormal operand.
+constexpr uint32_t kFaceTop = (1023u + 100u) << 20;
+constexpr int kFaceLow = 104;
+// Special faces that carry phi = C*u all the same, for cells of [0, 2^100):
+// C = 0 (c: C or a factor of it that vanishes with it), u = 0 (the
+// difference to uu cannot have the sign of that to d), or d and u up to
+// 1e-27 (|d-u| is too).  Loss cones decay to such cells within minutes, whole
+// lines of them, and a dipole's C vanishes along whole meridians.
+RG_HD bool face_plain(uint64_t uu, uint64_t u, uint64_t d, uint64_t c) {
+  const uint32_t hu = (uint32_t)(u >> 32), hd = (uint32_t)(d >> 32), huu = (uint32_t)(uu >> 32);
+  return max3u(hu, hd, huu) < kFaceTop && (u == 0 || (c << 1) == 0 || (hu < 0x3A53CE9Au && hd < 0x3A53CE9Au));
+}
 
 // phi as bits, from the bits of the cells.  kCase: cs is the limiter's
 // branch (0 upwind only, 1 beta*D, 2 X, 3 D, 4 beta*X).
-template <bool kCase>
+template <bool kCase, bool kB32>
 RG_HD uint64_t face_flux(uint64_t uu, uint64_t u, uint64_t d, const FaceCoef& q, uint64_t betaf, bool& special,
                          int& cs) {
   const uint32_t hu = (uint32_t)(u >> 32), hd = (uint32_t)(d >> 32), huu = (uint32_t)(uu >> 32);
@@ -142,18 +227,23 @@ RG_HD uint64_t face_flux(uint64_t uu, uint64_t u, uint64_t d, const FaceCoef& q,
   // |X|, |D| where both have the sign s, one unit low when it is negative
   const uint64_t ax = X ^ sm, adx = D ^ sm;
   bool act = hi32(adx) >= 0;
-  bool undecided = false;
   if (eu < 993) {
     // |X| > 1e-27.  From eu = 993 (u >= 2^-30) on, a difference below the
     // threshold is at most one unit here, whose correction is zero.  Below
-    // eu = 932 (u < 4.1e-28) only an increase to d > 1e-27 can be active.
-    const uint64_t thr = shr_clamp(0x9E74D1B791E08000ULL, eu > 930 ? eu - 929 : 1);  // sig_top of 1e-27
-    undecided = eu < 932 && hd >= 0x3A53CE9Au && act && s == 0;
-    act = act && eu >= 932 && ax > thr;
+    // eu = 932 (u < 4.1e-28) only an increase can pass it: d against u + 1e-27
+    // in units of 2^-151.
+    constexpr uint64_t t27 = 0x9E74D1B791E08000ULL;  // sig_top of 1e-27, exponent 933
+    if (eu >= 932) {
+      act = act && ax > shr_clamp(t27, eu - 929);
+    } else {
+      const int ed = (int)(hd >> 20);
+      act = act && s == 0 &&
+            (ed > 935 || shr_clamp(sig_top(d), 936 - ed) > shr_clamp(sig_top(u), 936 - eu) + (t27 >> 3));
+    }
   }
-  const bool dlo = adx <= ax;
-  const uint64_t lo = dlo ? adx : ax, hi = dlo ? ax : adx;
-  const uint64_t bl = beta_times(lo, betaf);
+  uint64_t lo, hi;
+  const bool dlo = sort2(adx, ax, lo, hi);
+  const uint64_t bl = beta_times<kB32>(lo, betaf);
   const uint64_t lim = bl < hi ? bl : hi;
   if (kCase) {
     const int c = dlo ? (bl <= hi ? 1 : 2) : (hi <= bl ? 3 : (betaf ? 4 : 2));
@@ -161,12 +251,12 @@ RG_HD uint64_t face_flux(uint64_t uu, uint64_t u, uint64_t d, const FaceCoef& q,
   }
   const uint64_t corr = act ? mulhi_cross(lim, q.a63) : 0ULL;
   const uint64_t fb = mu + (corr ^ sm) + (uint32_t)(-s);
-  const uint64_t p = mulhi_cross(fb, q.m);  // < 2^59
+  const uint64_t p = mulhi_cross(fb, q.m);  // < 2^60
   const int tb = top_bit((uint32_t)(p >> 32));
   const int E = eu + q.e + tb - (1049 + kFaceLow);  // exponent field less one, less kFaceLow
   const uint64_t t = p >> ((tb - 21) & 63);
   const uint32_t top = max3u(hu, hd, huu);
-  special = top >= kFaceTop || undecided || (q.bad | E | hi32(fb) | (tb - 21)) < 0;
+  special = top >= kFaceTop || (q.bad | E | hi32(fb) | (tb - 21)) < 0;
   const uint32_t field = ((uint32_t)E << 20) + (q.sign + ((uint32_t)kFaceLow << 20));
   return ((uint64_t)field << 32) + (t >> 1) + (t & 1ULL);
 }

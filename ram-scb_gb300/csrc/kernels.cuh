@@ -53,13 +53,13 @@ __device__ __forceinline__ int stale_ghost_src(const Dev& d, int m, int slot, in
 // rsh: its nibble of the record bytes (4: high, forward half, written
 // first; 0: low, reverse half, ORed in).
 void launch_sweep_r(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec = nullptr,
-                    bool replay = false, int co = 0, int rsh = 0);
+                    bool replay = false, int rsh = 0);
 void launch_sweep_p(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec = nullptr,
-                    bool replay = false, int co = 0, int rsh = 0);
+                    bool replay = false, int rsh = 0);
 void launch_sweep_e(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec = nullptr,
-                    bool replay = false, int co = 0, int rsh = 0);
+                    bool replay = false, int rsh = 0);
 void launch_sweep_mu(const Dev& d, double dts, bool cfl, int loss_mode, const double* loss,
-                     cudaStream_t st, unsigned char* rec = nullptr, bool replay = false, int co = 0, int rsh = 0);
+                     cudaStream_t st, unsigned char* rec = nullptr, bool replay = false, int rsh = 0);
 
 int sweep_max_blocks_per_sm(int w, int blk);
 

@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "face.cuh"
+
 namespace ramgpu {
 
 constexpr double kOME = 7.3E-5;        // Earth's angular velocity, src/ModRamDrift.f90:224
@@ -39,7 +41,7 @@ struct Dev {
   const double *lr2, *sinphi;  // (LZ(I)*RE)**2 (NR+1) and SIN(PHI(J)-PHIOFS) (NT) of the VOLS formula
   const int *upa_atm;   // int(UPA(I)): first loss-cone L (1-based), NR
   const int *upa_mom;   // int(UPA(I)-1): last L of the ANISCH sum, NR
-  // reciprocal grid tables: -0.5/DE, 1/WE, 1/DE (NE); -0.5/DMU, 1/WMU, 1/DMU (NPA)
+  // reciprocal grid tables: -0.5/DE, 1/WE, 1/DE (NE, then the largest 1/DE); -0.5/DMU, 1/WMU, 1/DMU (NPA)
   const double *mhde, *iwe, *ide, *mhdmu, *iwmu, *idmu;
   const double *bmhde, *bmhdmu;  // BetaLim times -0.5/DE and -0.5/DMU (adjoint)
   // per-species grid (ns x NE)
@@ -69,6 +71,8 @@ struct Dev {
   double *p2;             // (ns, NR, NE)
   double *edot;           // (ns, NR, NE)
   double *eb, *ek;        // (ns, NE)
+  FaceBin *ebin;          // (ns, NE): DRIFTE's bin factors (face.cuh), DTs-free
+  double *er, *erq;       // (NR), (ns, NR): DTs/RLZ and 1e3/QS times that
   double *kap;            // (ns, 2): extrapolation factors of F(1), F(0) in DRIFTE
   double *wm;             // (NR,NT,NPA): -CMUDOT*HM, DTs-dependent, species-free
   double *cmudot;         // (NR,NT,NPA): MUDOT(I,L)*BOUNIS/BOUNHS, DTs-dependent
@@ -107,15 +111,15 @@ struct Dev {
   double *mom_part;       // (nm*ns, NT, NR, (NE-1)*4 chunks, 2) moment partials
   double *ppert, *ppart;  // (nm*ns, NR, NT)
   double *sumrc_part;     // (nm*ns, nblk) SUMRC partial sums
-  // face coefficients C and a of the forward sweeps, read back by the
-  // reverse ones: (stored sweeps, 2, coef_items, ncell); coef_slot[w] is
-  // sweep w's place or -1; null when not allocated
-  double *coef;
+  // face coefficients C of a call's first DRIFTE transpose, read back by the
+  // second: (coef_items, ncell); null when not allocated
+  double* coef;
   long long coef_items;
-  int coef_slot[4];
   // work list
   const int2 *items;      // (member, species)
   int nitems;
+  int nlist;  // items of the full list
+  int nsm;    // multiprocessors of the device
   int item0;              // position of items[0] in the full list (a group's view of it)
   // launch shape of the sweeps R, P, E, MU: threads per CTA and, when > 0,
   // a persistent grid of that many CTAs looping over (item, line-block) units
@@ -263,6 +267,8 @@ __device__ __forceinline__ double mul_rn_int(double a, double b) {
 // x < 0.0 exactly as the Fortran test `C.lt.0` (false for -0.0 and NaN with
 // the sign bit clear).
 __device__ __forceinline__ bool is_neg(double x) { return dbits(x) > 0x8000000000000000ULL; }
+// finite
+__device__ __forceinline__ bool abs_lt_inf(double x) { return (hi32(dbits(x)) & 0x7FF00000) != 0x7FF00000; }
 // |x| > 1e-27
 __device__ __forceinline__ bool abs_gt_1em27(double x) {
   const unsigned long long t = 0x3A53CE9A36F23C10ULL;  // bits of 1.0E-27
@@ -310,10 +316,8 @@ constexpr int kClipBit = 8;  // recorded with the case: the updated cell was cli
 // 3 plain and count clip events into Dev::clipq
 constexpr int kRecCount = 3;
 
-// Stored face coefficient array q (0: C, 1: a) of sweep w for work item `it`.
-__device__ __forceinline__ double* coef_ptr(const Dev& d, int w, int q, long long it) {
-  return d.coef + (((long long)(d.coef_slot[w] * 2 + q) * d.coef_items) + d.item0 + it) * d.ncell;
-}
+// Stored DRIFTE face coefficients of work item `it`.
+__device__ __forceinline__ double* coef_ptr(const Dev& d, long long it) { return d.coef + (d.item0 + it) * d.ncell; }
 
 // Face value with the branch taken from a record (frozen-limiter replay):
 // LIMITER*X = beta*D | X | D | beta*X for cases 1..4, FUP for case 0, the

@@ -11,12 +11,16 @@
 //   DRIFTMU src/ModRamDrift.f90:382-473
 // with the face coefficients taken from separable tables built in tables.cu
 // (C = A(I,J) + G(I,J,L)*k(K) etc.).  The FP64 unit was the limit: sign, abs
-// and limiter tests run on bit patterns; in DRIFTR and DRIFTP the whole face
-// flux is formed in 64-bit fixed point (face.cuh), which leaves three FP64
-// operations a face (the coefficient and the two of the update); in DRIFTE
-// and DRIFTMU the products that are only compared (beta*|X|, the CFL
+// and limiter tests run on bit patterns; in DRIFTR, DRIFTP and DRIFTE the
+// whole face flux is formed in 64-bit fixed point (face.cuh), which leaves
+// three FP64 operations a face (the coefficient and the two of the update);
+// in DRIFTMU the products that are only compared (beta*|X|, the CFL
 // quotients) and the flux C*FBND (mul_rn_int, rounded exactly like the FP64
-// multiply) run on the integer pipe, leaving 6 to 7.
+// multiply) run on the integer pipe, leaving 6.
+#include <string.h>
+
+#include <type_traits>
+
 #include "ramgpu_internal.cuh"
 #include "face.cuh"
 #include "kernels.cuh"
@@ -55,75 +59,114 @@ static __device__ __noinline__ PhiCase face_phi_fp64(double x, double dd, double
 }
 
 // Flux of a limited face (face.cuh) with the prepared coefficient q of C.
-// mh: -1/2 (R, P) or -1/2 over the bin width.  kRec 1: cs is the branch
-// taken; 2: the recorded branch cs is applied (the same bits as the
-// recording sweep's where that is the branch the values select).
-template <int kRec>
-__device__ __forceinline__ double face_phi(double uu, double u, double d, double c, const FaceCoef& q, double mh,
-                                           double beta, uint64_t betaf, int& cs) {
+// v: C or a factor of it that vanishes with it; cf(): C, and mh(): -1/2 (R, P)
+// or -1/2 over the bin width, formed only for the FP64 form.  kRec 1: cs is the branch taken; 2: the recorded branch cs
+// is applied (the same bits as the recording sweep's where that is the
+// branch the values select).  over(): called where U >= 1 or C is not finite.
+struct NoOver {
+  __device__ __forceinline__ void operator()() const {}
+};
+template <int kRec, bool kB32, class C, class M, class O = NoOver>
+__device__ __forceinline__ double face_phi(double uu, double u, double d, double v, const FaceCoef& q, double beta,
+                                           uint64_t betaf, int& cs, C&& cf, M&& mh, O&& over = O()) {
   bool special;
   int taken = 0;
-  double phi = bitsd(face_flux<kRec == 1 || kRec == 2>(dbits(uu), dbits(u), dbits(d), q, betaf, special, taken));
+  double phi =
+      bitsd(face_flux<kRec == 1 || kRec == 2, kB32>(dbits(uu), dbits(u), dbits(d), q, betaf, special, taken));
   if (kRec == 2) special = special || taken != cs;
   if (kRec == 1) cs = taken;
   if (special) {
-    const bool neg = hi32(dbits(c)) < 0;
-    const PhiCase r = face_phi_fp64<kRec>(neg ? u - d : d - u, neg ? uu - u : u - uu, u, c, mh, beta, cs);
+    if (q.bad < 0) over();
+    if (kRec != 2 && face_plain(dbits(uu), dbits(u), dbits(d), dbits(v))) {
+      if (kRec == 1) cs = 0;
+      if (q.bad < 0 || (dbits(u) != 0ULL && (dbits(v) << 1) != 0ULL)) return __dmul_rn(cf(), u);
+      return bitsd((bits64)q.sign << 32);
+    }
+    const bool neg = q.sign != 0;
+    const PhiCase r = face_phi_fp64<kRec>(neg ? u - d : d - u, neg ? uu - u : u - uu, u, cf(), mh(), beta, cs);
     phi = r.phi;
     if (kRec == 1) cs = r.cs;
   }
   return phi;
 }
 
+// The line's largest Courant number, as the face with the smallest 1 - U:
+// its quotient is formed once, after the line.  Faces whose U differ by less
+// than 2^-63 count as equal, which moves DtDrift by at most one rounding
+// wherever it is below its cap.
+struct Largest {
+  uint64_t a63 = 1ULL << 63;
+  int at = 0;
+  __device__ __forceinline__ void see(const FaceCoef& q, int f) {
+    const bool less = q.a63 < a63;
+    a63 = less ? q.a63 : a63;
+    at = less ? f : at;
+  }
+};
+
+// Work units are (item, block of lines).  A plain grid of (blocks per item,
+// items) gives one unit per CTA; a persistent grid (one row) loops over them.
+struct Unit {
+  int it, b, bpi;
+  __device__ __forceinline__ Unit(int bpi_) : it(blockIdx.y), b(blockIdx.x), bpi(bpi_) {}
+  __device__ __forceinline__ bool ok(const Dev& d) {
+    while (b >= bpi) {
+      b -= bpi;
+      ++it;
+    }
+    return it < d.nitems;
+  }
+  __device__ __forceinline__ void next(const Dev& d) {
+    b += gridDim.x;
+    if (gridDim.y > 1) it = d.nitems;
+  }
+};
+
 // ----------------------------------------------------------------- DRIFTR
 // Line (J,K,L) along I = 1..NR.  Faces 2..NR-1 (and NR on inflow lines).
-template <bool kCfl, int kRec, int kCo>
+// kCfl (R, P): 1 the largest |C| of the line, 2 of its cells inside the
+// magnetopause, where some lie outside.
+template <int kCfl, int kRec, bool kB32>
 __global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   // the lines of the L window [lw0, lw1) (all of them unless a pipeline
   // runs the step plane chunk by plane chunk): L is the slowest index
   const int line0 = d.lw0 * nt * ne;
   const int nlines = nt * ne * (d.lw1 - d.lw0);
-  // Work units are (item, block of lines).  A grid of (blocks per item,
-  // items) gives one unit per CTA; a persistent grid loops over them.
-  const int bpi = (nlines + blockDim.x - 1) / blockDim.x;
-  const long long nunits = (long long)bpi * d.nitems;
-  for (long long u = blockIdx.x + (long long)blockIdx.y * gridDim.x; u < nunits;
-       u += (long long)gridDim.x * gridDim.y) {
-    const int2 item = d.items[u / bpi];
+  for (Unit u((nlines + blockDim.x - 1) / blockDim.x); u.ok(d); u.next(d)) {
+    const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
-    const int line = line0 + (int)(u % bpi) * blockDim.x + threadIdx.x;
-    unsigned long long q = 0ULL;  // CFL quotient bits
+    const int line = line0 + u.b * blockDim.x + threadIdx.x;
+    unsigned long long q = kBits1em10;  // CFL quotient bits: |C| at least 1e-10
     unsigned nclip = 0;  // clip events (kRec == kRecCount)
     // bounds-checked builds: the line's cells, its GRT and CR rows, the
     // coefficient store's item
     const bool lok = line >= line0 + nlines ||
         rg_ok(d, rg_item(d, item) && rg_span((long long)line * nr, nr, 1, d.ncell) &&
                      rg_span(((long long)(line / (nt * ne)) * nt + line % nt) * nr, nr, 1, (long long)nr * nt * d.npa) &&
-                     rg_span(((long long)item.x * nt + line % nt) * nr, nr, 1, (long long)d.nm * nr * nt) &&
-                     (!kCo || d.item0 + u / bpi < d.coef_items),
+                     rg_span(((long long)item.x * nt + line % nt) * nr, nr, 1, (long long)d.nm * nr * nt),
               kRgSweepR, line);
     if (line < line0 + nlines && lok) {
       const int j = line % nt;
       const int l = line / (nt * ne);
       double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + (long long)line * nr;
       // branch record of the frozen-limiter adjoint: one byte per face/cell
-      unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + (u / bpi) * d.ncell + (long long)line * nr : nullptr;
-      // face coefficients C: stored by the forward sweep, read back by the
-      // reverse one (same DTs, same potential)
-      double* __restrict__ cst = kCo ? coef_ptr(d, 0, 0, u / bpi) + (long long)line * nr : nullptr;
+      unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + u.it * d.ncell + (long long)line * nr : nullptr;
       const double* __restrict__ grt = d.grt + ((long long)l * nt + j) * nr;
       const double* __restrict__ cr = d.cr + ((long long)m * nt + j) * nr;
       const int* __restrict__ outside = d.outside + (long long)j * nr;
       const double p4 = d.p4[s * ne + (line / nt) % ne];
       const double beta = d.betalim;
       const uint64_t betaf = beta_fix(dbits(beta));
+      auto mh = [] { return -0.5; };
+      auto limit = [&](int f, double c) {
+        if (kCfl == 1 || (kCfl == 2 && outside[f - 1] == 0)) q = cfl_bits(c, q);
+      };
       const bool closed = d.flags & 1u;
 
       const int k = (line / nt) % ne;
-      const double cN = (kCo == 2) ? cst[nr - 1] : fma(grt[nr - 1], p4, cr[nr - 1]);
-      const double cNm = (kCo == 2) ? cst[nr - 2] : fma(grt[nr - 2], p4, cr[nr - 2]);
-      if (kCo == 1) { cst[nr - 1] = cN; cst[nr - 2] = cNm; }
+      const double cN = fma(grt[nr - 1], p4, cr[nr - 1]);
+      const double cNm = fma(grt[nr - 2], p4, cr[nr - 2]);
       const bool inflow = is_neg(cN);
       // F(NR+1), F(NR+2): boundary ghosts on inflow lines.  On an outflow line
       // F(NR+1) is read only by face NR-1 when it is upwinded from the right,
@@ -137,20 +180,18 @@ __global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned cha
         g1 = stale_ghost(d, m, slot, j, k, l, p4);
       }
       double gm = fl[0], g0 = fl[1], gp = fl[2];
-      double c = (kCo == 2) ? cst[0] : fma(grt[0], p4, cr[0]);
-      if (kCo == 1) cst[0] = c;
-      if (kCfl && outside[0] == 0) q = umax64(q, cfl_bits(c, kBits1em10));
+      double c = fma(grt[0], p4, cr[0]);
+      limit(1, c);
       // face 1: FBND(1) = 0 (outflow) or F(2) (inflow)
       double phi_prev = c * ((inflow && !closed) ? g0 : 0.0);
       for (int f = 2; f <= nr - 1; ++f) {  // 1-based face f, updates cell f
         const double gpp = (f + 2 <= nr) ? fl[f + 1] : g1;
-        c = (kCo == 2) ? cst[f - 1] : ((f == nr - 1) ? cNm : fma(grt[f - 1], p4, cr[f - 1]));
-        if (kCo == 1) cst[f - 1] = c;
-        if (kCfl && outside[f - 1] == 0) q = umax64(q, cfl_bits(c, kBits1em10));
+        c = ((f == nr - 1) ? cNm : fma(grt[f - 1], p4, cr[f - 1]));
+        limit(f, c);
         const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
         int cs = kRec == 2 ? (int)(rget(rl + (f - 1), rsh) & 7) : 0;
-        const double phi = face_phi<kRec>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), -0.5,
-                                          beta, betaf, cs);
+        const double phi = face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), beta,
+                                                betaf, cs, [&] { return c; }, mh);
         const double raw = (g0 - phi) + phi_prev;
         fl[f - 1] = (kRec == 2) ? clip_frozen(raw, rget(rl + (f - 1), rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
@@ -160,11 +201,11 @@ __global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned cha
       }
       // face NR (g0 = F(NR), gp = F(NR+1)): limited on inflow lines, F(NR)
       // on outflow lines
-      if (kCfl && outside[nr - 1] == 0) q = umax64(q, cfl_bits(cN, kBits1em10));
+      limit(nr, cN);
       int csn = kRec == 2 ? (int)(rget(rl + (nr - 1), rsh) & 7) : 0;
       double phin = 0.0;
       if (!closed)
-        phin = inflow ? face_phi<kRec>(g2, g1, g0, cN, face_coef(dbits(cN)), -0.5, beta, betaf, csn)
+        phin = inflow ? face_phi<kRec, kB32>(g2, g1, g0, cN, face_coef(dbits(cN)), beta, betaf, csn, [&] { return cN; }, mh)
                       : mul_rn_int(cN, g0);
       const double rawn = (g0 - phin) + phi_prev;
       fl[nr - 1] = (kRec == 2) ? clip_frozen(rawn, rget(rl + (nr - 1), rsh)) : clip(rawn);
@@ -178,21 +219,19 @@ __global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned cha
 
 // ----------------------------------------------------------------- DRIFTP
 // Line (I,K,L), I = 2..NR, along J = 1..NT, periodic with J=1 == J=NT.
-template <bool kCfl, int kRec, int kCo>
-__global__ void __launch_bounds__(256) k_sweep_p(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
+// Held to 64 registers (32 warps an SM): on 40x49x70x144 553 us a launch
+// against 608 with 78; running the next face's coefficient one iteration
+// ahead, or unrolling by 2 or 4, took 594 to 703.
+template <int kCfl, int kRec, bool kB32>
+__global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   const int line0 = d.lw0 * (nr - 1) * ne;  // the L window, as in DRIFTR
   const int nlines = (nr - 1) * ne * (d.lw1 - d.lw0);
-  // Work units are (item, block of lines).  A grid of (blocks per item,
-  // items) gives one unit per CTA; a persistent grid loops over them.
-  const int bpi = (nlines + blockDim.x - 1) / blockDim.x;
-  const long long nunits = (long long)bpi * d.nitems;
-  for (long long u = blockIdx.x + (long long)blockIdx.y * gridDim.x; u < nunits;
-       u += (long long)gridDim.x * gridDim.y) {
-    const int2 item = d.items[u / bpi];
+  for (Unit u((nlines + blockDim.x - 1) / blockDim.x); u.ok(d); u.next(d)) {
+    const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
-    const int line = line0 + (int)(u % bpi) * blockDim.x + threadIdx.x;
-    unsigned long long q = 0ULL;  // CFL quotient bits
+    const int line = line0 + u.b * blockDim.x + threadIdx.x;
+    unsigned long long q = kBits1em10;  // CFL quotient bits: |C| at least 1e-10
     unsigned nclip = 0;  // clip events (kRec == kRecCount)
     // bounds-checked builds: the line's cells, its GPT and CA columns, the
     // coefficient store's item
@@ -201,8 +240,7 @@ __global__ void __launch_bounds__(256) k_sweep_p(Dev d, double dts, unsigned cha
                      rg_span((long long)(line / (nr - 1)) * nt * nr + 1 + line % (nr - 1), nt, nr, d.ncell) &&
                      rg_span((long long)(line / (nr - 1) / ne) * nt * nr + 1 + line % (nr - 1), nt, nr,
                              (long long)nr * nt * d.npa) &&
-                     rg_span((long long)item.x * nt * nr + 1 + line % (nr - 1), nt, nr, (long long)d.nm * nr * nt) &&
-                     (!kCo || d.item0 + u / bpi < d.coef_items),
+                     rg_span((long long)item.x * nt * nr + 1 + line % (nr - 1), nt, nr, (long long)d.nm * nr * nt),
               kRgSweepP, line);
     if (line < line0 + nlines && lok) {
       const int i = 1 + line % (nr - 1);
@@ -211,47 +249,40 @@ __global__ void __launch_bounds__(256) k_sweep_p(Dev d, double dts, unsigned cha
       const long long st = nr;  // stride between consecutive J
       double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + ((long long)kl * nt) * nr + i;
       unsigned char* __restrict__ rl =
-          (kRec == 1 || kRec == 2) ? rec + (u / bpi) * d.ncell + ((long long)kl * nt) * nr + i : nullptr;
-      double* __restrict__ cst = kCo ? coef_ptr(d, 1, 0, u / bpi) + ((long long)kl * nt) * nr + i : nullptr;
+          (kRec == 1 || kRec == 2) ? rec + u.it * d.ncell + ((long long)kl * nt) * nr + i : nullptr;
       const double* __restrict__ gpt = d.gpt + ((long long)l * nt) * nr + i;
       const double* __restrict__ ca = d.ca + ((long long)m * nt) * nr + i;
       const int* __restrict__ outside = d.outside + i;
       const double p2 = d.p2[((long long)s * ne + k) * nr + i];
       const double beta = d.betalim;
       const uint64_t betaf = beta_fix(dbits(beta));
+      auto mh = [] { return -0.5; };
   #define GJ(J) fl[(long long)((J)-1) * st]
   #define CJ(J) fma(gpt[(long long)((J)-1) * nr], p2, ca[(long long)((J)-1) * nr])
       const double G1 = GJ(1), G2 = GJ(2), G3 = GJ(3), GNm = GJ(nt - 1), GN = GJ(nt);
       // face NT first: its flux enters cell 2 through FBND(1)=FBND(NT)
-      const double cN = (kCo == 2) ? cst[(long long)(nt - 1) * st] : CJ(nt);
-      if (kCo == 1) cst[(long long)(nt - 1) * st] = cN;
-      if (kCfl && outside[(long long)(nt - 1) * nr] == 0) q = umax64(q, cfl_bits(cN, kBits1em10));
+      const double cN = CJ(nt);
+      auto limit = [&](int J, double c) {
+        if (kCfl == 1 || (kCfl == 2 && outside[(long long)(J - 1) * nr] == 0)) q = cfl_bits(c, q);
+      };
+      limit(nt, cN);
       int csN = kRec == 2 ? (int)(rget(rl + (long long)(nt - 1) * st, rsh) & 7) : 0;
       const bool negN = is_neg(cN);
-      const double phiN = face_phi<kRec>(negN ? G3 : GNm, negN ? G2 : GN, negN ? GN : G2, cN, face_coef(dbits(cN)),
-                                         -0.5, beta, betaf, csN);
+      const double phiN = face_phi<kRec, kB32>(negN ? G3 : GNm, negN ? G2 : GN, negN ? GN : G2, cN, face_coef(dbits(cN)),
+                                               beta, betaf, csN, [&] { return cN; }, mh);
       double phi_prev = phiN;
       double gm = G1, g0 = G2, gp = G3;
-      // The reference's D of face NT-1 against the flow is F(2)-F(1), with
-      // F(1) in the place of F(NT); the two differ only in states that are
-      // not periodic.
-      const bool oddwrap = dbits(G1) != dbits(GN);
-      // the cell two faces ahead is loaded one iteration early, before this
-      // face's store: the compiler cannot move a load past a store to the
-      // line at a run-time stride (DRIFTR's contiguous lines come from L1)
-      double nxt = GJ(4);
-      for (int J = 2; J <= nt - 1; ++J) {
-        const double nn = GJ(min(J + 3, nt));
-        const double gpp = J == nt - 1 ? G2 : nxt;
-        const double c = (kCo == 2) ? cst[(long long)(J - 1) * st] : CJ(J);
-        if (kCo == 1) cst[(long long)(J - 1) * st] = c;
-        if (kCfl && outside[(long long)(J - 1) * nr] == 0) q = umax64(q, cfl_bits(c, kBits1em10));
+      auto step = [&](int J, double c, double gpp, auto wrap) {
+        limit(J, c);
         const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
         const unsigned char* rj = (kRec == 1 || kRec == 2) ? rl + (long long)(J - 1) * st : nullptr;
         int cs = kRec == 2 ? (int)(rget(rj, rsh) & 7) : 0;
-        double phi = face_phi<kRec>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), -0.5, beta,
-                                    betaf, cs);
-        if (J == nt - 1 && neg && oddwrap) {
+        double phi = face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), beta,
+                                          betaf, cs, [&] { return c; }, mh);
+        // The reference's D of face NT-1 against the flow is F(2)-F(1), with
+        // F(1) in the place of F(NT); the two differ only in states that are
+        // not periodic.
+        if (decltype(wrap)::value && neg && dbits(G1) != dbits(GN)) {
           const PhiCase r = face_phi_fp64<kRec>(gp - g0, G2 - G1, gp, c, -0.5, beta,
                                                 kRec == 2 ? (int)(rget(rj, rsh) & 7) : 0);
           phi = r.phi;
@@ -263,8 +294,17 @@ __global__ void __launch_bounds__(256) k_sweep_p(Dev d, double dts, unsigned cha
         if (kRec == 1) rput(rl + ((long long)(J - 1) * st), rsh, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
         gm = g0; g0 = gp; gp = gpp;
+      };
+      // The cell two faces ahead is loaded one iteration early, before this
+      // face's store: the compiler cannot move a load past a store to the
+      // line at a run-time stride.
+      double nxt = GJ(4);
+      for (int J = 2; J <= nt - 2; ++J) {
+        const double nn = GJ(min(J + 3, nt));
+        step(J, CJ(J), nxt, std::false_type());
         nxt = nn;
       }
+      step(nt - 1, CJ(nt - 1), G2, std::true_type());
       const double rawN = (GN - phiN) + phi_prev;
       const double vN = (kRec == 2) ? clip_frozen(rawN, rget(rl + (long long)(nt - 1) * st, rsh)) : clip(rawN);
       if (kRec == kRecCount) nclip += is_neg(rawN);
@@ -282,109 +322,136 @@ __global__ void __launch_bounds__(256) k_sweep_p(Dev d, double dts, unsigned cha
 // ----------------------------------------------------------------- DRIFTE
 // Line (I,J,L), I = 2..NR, along K = 1..NE with extrapolated F(0), F(1)
 // and F(NE+1) = F(NE+2) = 0.  Cell K = 1 is never written.
-template <bool kCfl, int kRec, int kCo>
-__global__ void __launch_bounds__(256) k_sweep_e(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
+// kSplit adjacent lanes share a line: lane r updates the cells b+1..lim of
+// its segment (b = r*S, lim = (r+1)*S with S = NE/kSplit; the first from
+// cell 2, the last to NE) and first forms face b anew, whose flux enters its
+// cells (face 1 for the first lane).  Every old value a lane needs from its
+// neighbours' cells is loaded before a __syncwarp, and no lane writes before
+// it; the flux of a face is the same bits in either lane.  S >= 4, so no
+// lane but the first sees the extrapolated cells.
+template <bool kCfl, int kRec, bool kB32, int kSplit>
+__global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   const int line0 = d.lw0 * (nr - 1) * nt;  // the L window, as in DRIFTR
   const int nlines = (nr - 1) * nt * (d.lw1 - d.lw0);
-  // Work units are (item, block of lines).  A grid of (blocks per item,
-  // items) gives one unit per CTA; a persistent grid loops over them.
-  const int bpi = (nlines + blockDim.x - 1) / blockDim.x;
-  const long long nunits = (long long)bpi * d.nitems;
-  for (long long u = blockIdx.x + (long long)blockIdx.y * gridDim.x; u < nunits;
-       u += (long long)gridDim.x * gridDim.y) {
-    const int2 item = d.items[u / bpi];
+  const int lpb = blockDim.x / kSplit;  // lines per CTA
+  const int r = kSplit > 1 ? (int)threadIdx.x % kSplit : 0, seg = ne / kSplit;
+  const bool last = r == kSplit - 1;
+  const int b = r ? r * seg : 1, lim = last ? ne : (r + 1) * seg;
+  for (Unit u((nlines + lpb - 1) / lpb); u.ok(d); u.next(d)) {
+    const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
-    const int line = line0 + (int)(u % bpi) * blockDim.x + threadIdx.x;
+    const int line = line0 + u.b * lpb + (int)threadIdx.x / kSplit;
     unsigned long long q = 0ULL;  // CFL quotient bits
     unsigned nclip = 0;  // clip events (kRec == kRecCount)
     // bounds-checked builds: the line's cells, its (I,J,L) table entry and
-    // UE, its EDOT column, the coefficient store's item
-    const bool lok = line >= line0 + nlines ||
+    // UE, its line factors (the lanes sharing a line test the same)
+    const bool active = line < line0 + nlines &&
         rg_ok(d, rg_item(d, item) &&
                      rg_span(((long long)(line / (nr - 1) / nt) * ne * nt + (line / (nr - 1)) % nt) * nr + 1 +
                                  line % (nr - 1), ne, (long long)nt * nr, d.ncell) &&
                      rg_span((long long)item.x * nr * nt * d.npa + (long long)(line / (nr - 1)) * nr + 1 +
                                  line % (nr - 1), 1, 1, (long long)d.nm * nr * nt * d.npa) &&
-                     rg_span((long long)item.y * ne * nr + 1 + line % (nr - 1), ne, nr, (long long)d.ns * ne * nr) &&
-                     (!kCo || d.item0 + u / bpi < d.coef_items),
+                     rg_span((long long)item.y * nr + 1 + line % (nr - 1), 1, 1, (long long)d.ns * nr),
               kRgSweepE, line);
-    if (line < line0 + nlines && lok) {
-      const int i = 1 + line % (nr - 1);
-      const int jl = line / (nr - 1);
-      const int j = jl % nt, l = jl / nt;
-      const long long st = (long long)nt * nr;  // stride between consecutive K
-      double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + ((long long)l * ne * nt + j) * nr + i;
-      unsigned char* __restrict__ rl =
-          (kRec == 1 || kRec == 2) ? rec + (u / bpi) * d.ncell + ((long long)l * ne * nt + j) * nr + i : nullptr;
-      double* __restrict__ cst =
-          kCo ? coef_ptr(d, 2, 0, u / bpi) + ((long long)l * ne * nt + j) * nr + i : nullptr;
-      double* __restrict__ ast =
-          kCo ? coef_ptr(d, 2, 1, u / bpi) + ((long long)l * ne * nt + j) * nr + i : nullptr;
-      const long long fij = ((long long)l * nt + j) * nr + i;
-      const double wet = d.wet[fij];
-      const double ue = d.ue[(long long)m * nr * nt * d.npa + fij];
-      const double* __restrict__ edot = d.edot + (long long)s * ne * nr + i;
-      const double* __restrict__ eb = d.eb + s * ne;
-      const double* __restrict__ mhde = d.mhde;
-      const double* __restrict__ iwe = d.iwe;
-      const bool inside = d.outside[(long long)j * nr + i] == 0;
-      const BetaBits beta(d.betalim);
-      const bool closed = d.flags & 1u;
+    const int lc = active ? line : line0;
+    const int i = 1 + lc % (nr - 1);
+    const int jl = lc / (nr - 1);
+    const int j = jl % nt, l = jl / nt;
+    const long long st = (long long)nt * nr;  // stride between consecutive K
+    const long long off = ((long long)l * ne * nt + j) * nr + i;
+    double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + off;
+    unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + u.it * d.ncell + off : nullptr;
+    const FaceBin* __restrict__ bins = d.ebin + s * ne;
   #define GK(K) fl[(long long)((K)-1) * st]
-  #define CK(K) (edot[(long long)((K)-1) * nr] * fma(eb[(K)-1], wet, ue))
-      const double F2v = GK(2);
-      const double G1 = d.kap[2 * s + 1] * F2v;
-      const double G0 = d.kap[2 * s + 0] * G1;
-      const double G2 = F2v, G3 = GK(3);
-      const double X0 = G1 - G0; const bits64 bX0 = babs_bits(beta, X0);
-      const double X1 = G2 - G1; const bits64 bX1 = babs_bits(beta, X1);
-      const double X2 = G3 - G2; const bits64 bX2 = babs_bits(beta, X2);
+    // the window G(b-1..b+2), the next cell, and the two cells past lim
+    double w0 = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0, nxt = 0.0, hA = 0.0, hB = 0.0;
+    if (active) {
+      w2 = GK(b + 1);
+      w3 = GK(b + 2);
+      if (kSplit > 1 && r) {
+        w0 = GK(b - 1);
+        w1 = GK(b);
+      } else {
+        w1 = d.kap[2 * s + 1] * w2;
+        w0 = d.kap[2 * s + 0] * w1;
+      }
+      nxt = GK(b + 3);
+      if (kSplit > 1 && !last) {
+        hA = GK(lim + 1);
+        hB = GK(lim + 2);
+      }
+    }
+    if (kSplit > 1) __syncwarp();
+    if (active) {
+      const long long fij = ((long long)l * nt + j) * nr + i;
+      // C(K) = k(K)*v, v = UE*DTs/RLZ + k*(WET*1e3/QS*DTs/RLZ): k = EBND*(GRBND+1)/
+      // (2 GRBND) comes from the bin's table, so a face's C costs one fma
+      const double wet = d.wet[fij] * d.erq[s * nr + i];
+      const double ue = d.ue[(long long)m * nr * nt * d.npa + fij] * d.er[i];
+      const bool inside = d.outside[(long long)j * nr + i] == 0;
+      const double beta = d.betalim;
+      const uint64_t betaf = beta_fix(dbits(beta));
+      const bool closed = d.flags & 1u;
+      // Face K: its flux.  At face NE against the flow FUP = F(NE+1) = 0: that
+      // flux is zero whatever the other cells (end).
+      Largest big;
+      auto face = [&](int K, const FaceBin& bin, double v, double gm, double g0, double gp, double gpp, int& cs,
+                      auto end) {
+        uint64_t prod;
+        const FaceCoef fc = face_coef_bin(dbits(v), bin, prod);
+        if (kCfl) big.see(fc, K);
+        const bool none = decltype(end)::value && fc.sign && abs_lt_inf(v), neg = fc.sign && !none;
+        const double phi = face_phi<kRec, kB32>(
+            neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, v, fc, beta, betaf, cs, [&] { return bin.k * v; },
+            [&] { return d.mhde[K - 1]; },
+            [&] { if (kCfl && inside) q = umax64(q, face_courant(dbits(v), bin.sh, prod)); });
+        if (none) cs = 0;
+        return none ? 0.0 : phi;
+      };
       double phi_prev;
       {
-        const double c = (kCo == 2) ? cst[0] : CK(1);
-        if (kCfl && inside) q = umax64(q, mul_pos_bits(cfl_bits(c, kBits1em10), d.ide[0]));
-        const bool neg = is_neg(c);
-        const double a = (kCo == 2) ? ast[0] : fma(c, mhde[0], neg ? -0.5 : 0.5);
-        if (kCo == 1) { cst[0] = c; ast[0] = a; }
-        int cs;
-        double fb = (kRec == 2) ? face_value_frozen(X1, neg ? X2 : X0, neg ? G2 : G1, a, beta, cs = rget(rl, rsh) & 7)
-                                : face_value_case(X1, bX1, neg ? X2 : X0, neg ? bX2 : bX0, neg ? G2 : G1, a, cs);
-        if (closed) fb = 0.0;
-        if (kRec == 1) rput(rl, rsh, cs);
-        phi_prev = c * fb;
+        unsigned char* rb = (kRec == 1 || kRec == 2) ? rl + (long long)(b - 1) * st : nullptr;
+        int cs = kRec == 2 ? (int)(rget(rb, rsh) & 7) : 0;
+        phi_prev = face(b, bins[b - 1], fma(bins[b - 1].k, wet, ue), w0, w1, w2, w3, cs, std::false_type());
+        if (closed && r == 0) phi_prev = 0.0;
+        if (kRec == 1 && r == 0) rput(rb, rsh, cs);
       }
-      double g0 = G2, gp = G3, xm = X1, x = X2;
-      bits64 bxm = bX1, bx = bX2;
-      double nxt = GK(4);  // loaded one iteration ahead, as in DRIFTP
-      for (int K = 2; K <= ne; ++K) {
-        const double gpp = (K + 2 <= ne) ? nxt : 0.0;
-        nxt = GK(min(K + 3, ne));
-        const double xp = gpp - gp; const bits64 bxp = babs_bits(beta, xp);
-        const double c = (kCo == 2) ? cst[(long long)(K - 1) * st] : CK(K);
-        if (kCfl && inside) q = umax64(q, mul_pos_bits(cfl_bits(c, kBits1em10), d.ide[K - 1]));
-        const bool neg = is_neg(c);
-        const double a = (kCo == 2) ? ast[(long long)(K - 1) * st] : fma(c, mhde[K - 1], neg ? -0.5 : 0.5);
-        if (kCo == 1) { cst[(long long)(K - 1) * st] = c; ast[(long long)(K - 1) * st] = a; }
-        int cs;
+      double gm = w1, g0 = w2, gp = w3;
+      auto step = [&](int K, double v, double gpp, auto end) {
+        const FaceBin bin = bins[K - 1];
         const unsigned char* rk = (kRec == 1 || kRec == 2) ? rl + (long long)(K - 1) * st : nullptr;
-        double fb = (kRec == 2) ? face_value_frozen(x, neg ? xp : xm, neg ? gp : g0, a, beta, cs = rget(rk, rsh) & 7)
-                                : face_value_case(x, bx, neg ? xp : xm, neg ? bxp : bxm, neg ? gp : g0, a, cs);
-        if (closed && K == ne) fb = 0.0;
-        // loaded coefficients leave this sweep few FP64 operations to hide its
-        // loads behind: the FP64 multiply (uncontracted, bit-equal to mul_rn_int)
-        const double phi = (kCo == 2) ? __dmul_rn(c, fb) : mul_rn_int(c, fb);
-        const double raw = fma(phi_prev - phi, iwe[K - 1], g0);
+        int cs = kRec == 2 ? (int)(rget(rk, rsh) & 7) : 0;
+        double phi = face(K, bin, v, gm, g0, gp, gpp, cs, end);
+        if (decltype(end)::value && closed) phi = 0.0;
+        const double raw = fma(phi_prev - phi, bin.iw, g0);
         GK(K) = (kRec == 2) ? clip_frozen(raw, rget(rk, rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
         if (kRec == 1) rput(rl + ((long long)(K - 1) * st), rsh, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
-        g0 = gp; gp = gpp;
-        xm = x; bxm = bx; x = xp; bx = bxp;
+        gm = g0; g0 = gp; gp = gpp;
+      };
+      // the cell two faces ahead one iteration early, as in DRIFTP
+      for (int K = b + 1; K <= (last ? ne - 1 : lim); ++K) {
+        double nn = hA;
+        if (K + 3 <= lim) nn = GK(K + 3);
+        else hA = hB;
+        step(K, fma(bins[K - 1].k, wet, ue), nxt, std::false_type());
+        nxt = nn;
       }
-  #undef GK
-  #undef CK
+      if (last) step(ne, fma(bins[ne - 1].k, wet, ue), 0.0, std::true_type());
+      if (kCfl && inside) {  // |C|/DE, |C| at least 1e-10
+        q = umax64(q, mul_pos_bits(kBits1em10, d.ide[ne]));
+        if (big.at) {
+          const FaceBin bin = bins[big.at - 1];
+          const double vb = fma(bin.k, wet, ue);
+          uint64_t prod;
+          face_coef_bin(dbits(vb), bin, prod);
+          q = umax64(q, face_courant(dbits(vb), bin.sh, prod));
+        }
+      }
     }
+  #undef GK
     if (kRec == kRecCount) warp_atomic_add(&d.clipq[slot], nclip);
     if (kCfl) warp_atomic_max(&d.cflq[slot * 4 + 2], q);
   }
@@ -405,16 +472,12 @@ __global__ void __launch_bounds__(256) k_sweep_e(Dev d, double dts, unsigned cha
 // past lim) is loaded before a __syncwarp, and no lane writes before it.
 // Segments keep at least 4 cells (2 lanes: NPA >= 12; 4 lanes: NPA >= 24),
 // so no lane but lane 0 sees the F(1) = F(2) rule.
-template <bool kCfl, int kLoss, int kRec, int kCo, int kSplit>
+template <bool kCfl, int kLoss, int kRec, int kSplit>
 __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const double* __restrict__ lossA,
                                                    unsigned char* __restrict__ rec, int rsh) {
   const int nr = d.nr, nt = d.nt, ne = d.ne, npa = d.npa;
   const int nlines = (nr - 1) * nt * ne;
-  // Work units are (item, block of lines).  A grid of (blocks per item,
-  // items) gives one unit per CTA; a persistent grid loops over them.
   const int lpb = blockDim.x / kSplit;  // lines per CTA
-  const int bpi = (nlines + lpb - 1) / lpb;
-  const long long nunits = (long long)bpi * d.nitems;
   // lane pairs: the even lane ends at Lm, the odd one takes the rest
   const int half = kSplit == 2 ? (int)(threadIdx.x & 1) : 0;
   const int Lm = kSplit == 2 ? npa / 2 : npa;  // last cell of the even lane
@@ -423,11 +486,10 @@ __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const doubl
   const int seg4 = npa / 4;
   const int pre = kSplit == 4 ? q4 : half;  // nonzero: the pre-face is recomputed
   const bool last = kSplit == 4 ? q4 == 3 : (half || kSplit == 1);
-  for (long long u = blockIdx.x + (long long)blockIdx.y * gridDim.x; u < nunits;
-       u += (long long)gridDim.x * gridDim.y) {
-    const int2 item = d.items[u / bpi];
+  for (Unit u((nlines + lpb - 1) / lpb); u.ok(d); u.next(d)) {
+    const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
-    const int line = (int)(u % bpi) * lpb + (int)threadIdx.x / kSplit;
+    const int line = u.b * lpb + (int)threadIdx.x / kSplit;
     // bounds-checked builds: the line's cells, its WM and UM columns, the
     // coefficient store's item (the lanes sharing a line test the same)
     const bool active = line < nlines &&
@@ -437,8 +499,7 @@ __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const doubl
                      rg_span((long long)((line / (nr - 1)) % nt) * nr + 1 + line % (nr - 1), npa, (long long)nt * nr,
                              (long long)nr * nt * npa) &&
                      rg_span((long long)item.x * nt * nr * npa + ((line / (nr - 1)) % nt) * nr + 1 + line % (nr - 1),
-                             npa, (long long)nt * nr, (long long)d.nm * nr * nt * npa) &&
-                     (!kCo || d.item0 + u / bpi < d.coef_items),
+                             npa, (long long)nt * nr, (long long)d.nm * nr * nt * npa),
               kRgSweepMu, line);
     unsigned long long q = 0ULL;  // CFL quotient bits
     unsigned nclip = 0;  // clip events (kRec == kRecCount)
@@ -449,9 +510,7 @@ __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const doubl
     const long long st = (long long)ne * nt * nr;  // stride between consecutive L
     const long long off = (long long)jk * nr + i;  // (K*NT + J)*NR + I
     double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + off;
-    unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + (u / bpi) * d.ncell + off : nullptr;
-    double* __restrict__ cst = kCo ? coef_ptr(d, 3, 0, u / bpi) + off : nullptr;
-    double* __restrict__ ast = kCo ? coef_ptr(d, 3, 1, u / bpi) + off : nullptr;
+    unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + u.it * d.ncell + off : nullptr;
     const double* __restrict__ la = lossA ? lossA + (long long)s * d.ncell + off : nullptr;
     const long long sij = (long long)nt * nr;     // stride of (I,J,L) tables in L
     const long long fij = (long long)j * nr + i;
@@ -489,9 +548,9 @@ __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const doubl
       // pre-face: the flux entering this lane's first cell
       double phi_prev;
       {
-        const double c = pre ? ((kCo == 2) ? cst[(long long)(b - 1) * st] : CL(b)) : 0.0;
+        const double c = pre ? CL(b) : 0.0;
         const bool neg = is_neg(c);
-        const double a = (kCo == 2 && pre) ? ast[(long long)(b - 1) * st] : fma(c, mhdmu[b - 1], neg ? -0.5 : 0.5);
+        const double a = fma(c, mhdmu[b - 1], neg ? -0.5 : 0.5);
         const double xm = w1 - w0, x = w2 - w1, xp = w3 - w2;
         int cs;
         const double fb = (kRec == 2)
@@ -518,11 +577,10 @@ __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const doubl
           if (kLoss == 2) gpp *= LA(L + 2);
         }
         const double xp = gpp - gp; const bits64 bxp = babs_bits(beta, xp);
-        const double c = (kCo == 2) ? cst[(long long)(L - 1) * st] : CL(L);
+        const double c = CL(L);
         if (kCfl && inside) q = umax64(q, mul_pos_bits(cfl_bits(c, kBits1em32), d.idmu[L - 1]));
         const bool neg = is_neg(c);
-        const double a = (kCo == 2) ? ast[(long long)(L - 1) * st] : fma(c, mhdmu[L - 1], neg ? -0.5 : 0.5);
-        if (kCo == 1) { cst[(long long)(L - 1) * st] = c; ast[(long long)(L - 1) * st] = a; }
+        const double a = fma(c, mhdmu[L - 1], neg ? -0.5 : 0.5);
         int cs;
         const unsigned char* rq = (kRec == 1 || kRec == 2) ? rl + (long long)(L - 1) * st : nullptr;
         const double fb = (kRec == 2) ? face_value_frozen(x, neg ? xp : xm, neg ? gp : g0, a, beta, cs = rget(rq, rsh) & 7)
@@ -541,8 +599,7 @@ __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const doubl
       // face NPA-1: FBND = F(NPA); cell NPA-1; then the F2(NPA) ghost
       if (last) {
         const int L = npa - 1;
-        const double c = (kCo == 2) ? cst[(long long)(L - 1) * st] : CL(L);
-        if (kCo == 1) cst[(long long)(L - 1) * st] = c;
+        const double c = CL(L);
         if (kCfl && inside) q = umax64(q, mul_pos_bits(cfl_bits(c, kBits1em32), d.idmu[L - 1]));
         const double phi = c * (closed ? 0.0 : gp);
         const double raw = fma(phi_prev - phi, iwmu[L - 1], g0);
@@ -586,89 +643,93 @@ static inline int nlines_of(const Dev& d, int w) {
   }
 }
 
-// co: 0 compute the face coefficients, 1 compute and store them, 2 load
-// the stored ones (needs d.coef; the plain, store and load forms give
-// identical results).
-void launch_sweep_r(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int co,
-                    int rsh) {
-  dim3 g = grid_for(d, 0, nlines_of(d, 0));
-  const int b = d.blk[0];
-  const bool n = d.count_clips;
-  if (rec && replay) k_sweep_r<false, 2, 0><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (rec) k_sweep_r<false, 1, 0><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (co == 1) (n ? k_sweep_r<true, 3, 1> : k_sweep_r<true, 0, 1>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else if (co == 2) (n ? k_sweep_r<false, 3, 2> : k_sweep_r<false, 0, 2>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else if (cfl) (n ? k_sweep_r<true, 3, 0> : k_sweep_r<true, 0, 0>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else (n ? k_sweep_r<false, 3, 0> : k_sweep_r<false, 0, 0>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
+// The limiter's beta has a short fraction (face.cuh beta_times).
+static inline bool beta_b32(const Dev& d) {
+  uint64_t u;
+  memcpy(&u, &d.betalim, sizeof(u));
+  return (uint32_t)beta_fix(u) == 0u;
 }
-void launch_sweep_p(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int co,
-                    int rsh) {
-  dim3 g = grid_for(d, 1, nlines_of(d, 1));
-  const int b = d.blk[1];
-  const bool n = d.count_clips;
-  if (rec && replay) k_sweep_p<false, 2, 0><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (rec) k_sweep_p<false, 1, 0><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (co == 1) (n ? k_sweep_p<true, 3, 1> : k_sweep_p<true, 0, 1>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else if (co == 2) (n ? k_sweep_p<false, 3, 2> : k_sweep_p<false, 0, 2>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else if (cfl) (n ? k_sweep_p<true, 3, 0> : k_sweep_p<true, 0, 0>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else (n ? k_sweep_p<false, 3, 0> : k_sweep_p<false, 0, 0>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
+#define SWEEP_LAUNCHER(NAME, KERNEL, W)                                                                       \
+  template <bool kB>                                                                                          \
+  static void NAME##_b(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay,  \
+                       int rsh) {                                                                             \
+    const dim3 g = grid_for(d, W, nlines_of(d, W));                                                           \
+    const int b = d.blk[W];                                                                                   \
+    const bool n = d.count_clips;                                                                             \
+    if (rec && replay) KERNEL<0, 2, kB><<<g, b, 0, st>>>(d, dts, rec, rsh);                               \
+    else if (rec) KERNEL<0, 1, kB><<<g, b, 0, st>>>(d, dts, rec, rsh);                                    \
+    else if (cfl && (d.flags >> 31))                                                                          \
+      (n ? KERNEL<2, 3, kB> : KERNEL<2, 0, kB>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);                         \
+    else if (cfl) (n ? KERNEL<1, 3, kB> : KERNEL<1, 0, kB>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);             \
+    else (n ? KERNEL<0, 3, kB> : KERNEL<0, 0, kB>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);                      \
+  }                                                                                                           \
+  void NAME(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int rsh) {  \
+    if (beta_b32(d)) NAME##_b<true>(d, dts, cfl, st, rec, replay, rsh);                                       \
+    else NAME##_b<false>(d, dts, cfl, st, rec, replay, rsh);                                                  \
+  }
+SWEEP_LAUNCHER(launch_sweep_r, k_sweep_r, 0)
+SWEEP_LAUNCHER(launch_sweep_p, k_sweep_p, 1)
+#undef SWEEP_LAUNCHER
+
+// Lanes per DRIFTE line.  A line is a serial chain of NE faces; with few
+// lines an SM has too few warps to hide it, and splitting lines gives more,
+// for one extra face and the halo loads per lane.  Measured (GB300, us a
+// launch with 1, 2, 4 lanes): 34.2 k lines (one species, 20x25x35x72) 26.6,
+// 25.2, 25.0, the whole call 0.231, 0.226, 0.225 ms; 136.8 k lines 54, 58,
+// 68; 1.1 M lines (40x49x70x144) 580, 665, 748.  The count is that of the
+// whole work list and every plane: item groups and chunks run side by side.
+static int e_lanes(const Dev& d) {
+  const long long warps = (long long)(d.nr - 1) * d.nt * d.npa * d.nlist / 32;
+  if (d.ne < 16) return 1;  // segments of at least four cells
+  return warps < 4LL * d.nsm ? 4 : (warps < 12LL * d.nsm ? 2 : 1);
 }
-void launch_sweep_e(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int co,
-                    int rsh) {
-  dim3 g = grid_for(d, 2, nlines_of(d, 2));
+template <bool kB, int kS>
+static void e_launch(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int rsh) {
+  const dim3 g = grid_for(d, 2, kS * nlines_of(d, 2));
   const int b = d.blk[2];
   const bool n = d.count_clips;
-  if (rec && replay) k_sweep_e<false, 2, 0><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (rec && co == 1) k_sweep_e<false, 1, 1><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (rec && co == 2) k_sweep_e<false, 1, 2><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (rec) k_sweep_e<false, 1, 0><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (co == 1) (n ? k_sweep_e<true, 3, 1> : k_sweep_e<true, 0, 1>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else if (co == 2) (n ? k_sweep_e<false, 3, 2> : k_sweep_e<false, 0, 2>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else if (cfl) (n ? k_sweep_e<true, 3, 0> : k_sweep_e<true, 0, 0>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else (n ? k_sweep_e<false, 3, 0> : k_sweep_e<false, 0, 0>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
+  if (rec && replay) k_sweep_e<false, 2, kB, kS><<<g, b, 0, st>>>(d, dts, rec, rsh);
+  else if (rec) k_sweep_e<false, 1, kB, kS><<<g, b, 0, st>>>(d, dts, rec, rsh);
+  else if (cfl) (n ? k_sweep_e<true, 3, kB, kS> : k_sweep_e<true, 0, kB, kS>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
+  else (n ? k_sweep_e<false, 3, kB, kS> : k_sweep_e<false, 0, kB, kS>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
 }
-// The clip-counting forms of the plain (unrecorded) pitch-angle sweeps.
-template <int kLoss, int kS>
-static void mu_count(const Dev& d, dim3 g, int b, double dts, const double* loss, cudaStream_t st, bool cfl,
-                     int co) {
-  if (co == 1) k_sweep_mu<true, kLoss, 3, 1, kS><<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
-  else if (co == 2) k_sweep_mu<false, kLoss, 3, 2, kS><<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
-  else if (cfl) k_sweep_mu<true, kLoss, 3, 0, kS><<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
-  else k_sweep_mu<false, kLoss, 3, 0, kS><<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
+void launch_sweep_e(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int rsh) {
+  const int lanes = e_lanes(d);
+  const bool kb = beta_b32(d);
+  if (lanes == 4) (kb ? e_launch<true, 4> : e_launch<false, 4>)(d, dts, cfl, st, rec, replay, rsh);
+  else if (lanes == 2) (kb ? e_launch<true, 2> : e_launch<false, 2>)(d, dts, cfl, st, rec, replay, rsh);
+  else (kb ? e_launch<true, 1> : e_launch<false, 1>)(d, dts, cfl, st, rec, replay, rsh);
 }
 
 template <int kLoss, int kS>
 static void mu_launch(const Dev& d, dim3 g, int b, double dts, const double* loss, cudaStream_t st,
-                      unsigned char* rec, bool replay, bool cfl, int co, int rsh) {
+                      unsigned char* rec, bool replay, bool cfl, int rsh) {
   const bool n = d.count_clips;
-  if (rec && replay) k_sweep_mu<false, kLoss, 2, 0, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
-  else if (rec) k_sweep_mu<false, kLoss, 1, 0, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
-  else if (n) mu_count<kLoss, kS>(d, g, b, dts, loss, st, cfl, co);
-  else if (co == 1) k_sweep_mu<true, kLoss, 0, 1, kS><<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
-  else if (co == 2) k_sweep_mu<false, kLoss, 0, 2, kS><<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
-  else if (cfl) k_sweep_mu<true, kLoss, 0, 0, kS><<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
-  else k_sweep_mu<false, kLoss, 0, 0, kS><<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
+  if (rec && replay) k_sweep_mu<false, kLoss, 2, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
+  else if (rec) k_sweep_mu<false, kLoss, 1, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
+  else if (cfl) (n ? k_sweep_mu<true, kLoss, 3, kS> : k_sweep_mu<true, kLoss, 0, kS>)<<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
+  else (n ? k_sweep_mu<false, kLoss, 3, kS> : k_sweep_mu<false, kLoss, 0, kS>)<<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
 }
 // Lines are split between d.mu_lanes adjacent lanes (2 for NPA >= 12, 4
 // for NPA >= 24: every segment keeps at least four cells, so no lane but
 // the first reads the F(1) rule).
 void launch_sweep_mu(const Dev& d, double dts, bool cfl, int loss_mode, const double* loss,
-                     cudaStream_t st, unsigned char* rec, bool replay, int co, int rsh) {
+                     cudaStream_t st, unsigned char* rec, bool replay, int rsh) {
   const int lanes = (d.mu_lanes == 4 && d.npa >= 24) ? 4 : ((d.mu_lanes >= 2 && d.npa >= 12) ? 2 : 1);
   dim3 g = grid_for(d, 3, lanes * nlines_of(d, 3));
   const int b = d.blk[3];
   if (lanes == 4) {
-    if (loss_mode == 1) mu_launch<1, 4>(d, g, b, dts, loss, st, rec, replay, cfl, co, rsh);
-    else if (loss_mode == 2) mu_launch<2, 4>(d, g, b, dts, loss, st, rec, replay, cfl, co, rsh);
-    else mu_launch<0, 4>(d, g, b, dts, nullptr, st, rec, replay, cfl, co, rsh);
+    if (loss_mode == 1) mu_launch<1, 4>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
+    else if (loss_mode == 2) mu_launch<2, 4>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
+    else mu_launch<0, 4>(d, g, b, dts, nullptr, st, rec, replay, cfl, rsh);
   } else if (lanes == 2) {
-    if (loss_mode == 1) mu_launch<1, 2>(d, g, b, dts, loss, st, rec, replay, cfl, co, rsh);
-    else if (loss_mode == 2) mu_launch<2, 2>(d, g, b, dts, loss, st, rec, replay, cfl, co, rsh);
-    else mu_launch<0, 2>(d, g, b, dts, nullptr, st, rec, replay, cfl, co, rsh);
+    if (loss_mode == 1) mu_launch<1, 2>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
+    else if (loss_mode == 2) mu_launch<2, 2>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
+    else mu_launch<0, 2>(d, g, b, dts, nullptr, st, rec, replay, cfl, rsh);
   } else {
-    if (loss_mode == 1) mu_launch<1, 1>(d, g, b, dts, loss, st, rec, replay, cfl, co, rsh);
-    else if (loss_mode == 2) mu_launch<2, 1>(d, g, b, dts, loss, st, rec, replay, cfl, co, rsh);
-    else mu_launch<0, 1>(d, g, b, dts, nullptr, st, rec, replay, cfl, co, rsh);
+    if (loss_mode == 1) mu_launch<1, 1>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
+    else if (loss_mode == 2) mu_launch<2, 1>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
+    else mu_launch<0, 1>(d, g, b, dts, nullptr, st, rec, replay, cfl, rsh);
   }
 }
 
@@ -677,10 +738,10 @@ int sweep_max_blocks_per_sm(int w, int blk) {
   int n = 0;
   cudaError_t e = cudaSuccess;
   switch (w) {
-    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_r<false, 0, 0>, blk, 0); break;
-    case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_p<false, 0, 0>, blk, 0); break;
-    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_e<false, 0, 0>, blk, 0); break;
-    default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_mu<false, 0, 0, 0, 2>, blk, 0); break;
+    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_r<0, 0, true>, blk, 0); break;
+    case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_p<0, 0, true>, blk, 0); break;
+    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_e<false, 0, true, 1>, blk, 0); break;
+    default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_mu<false, 0, 0, 2>, blk, 0); break;
   }
   return e == cudaSuccess ? n : 0;
 }

@@ -149,6 +149,18 @@ __global__ void k_species_static(Dev d) {
   const double QS = (double)d.qs[s];
   d.eb[t] = EBND(K) * 1e3 * (grbnd[K - 1] + 1) / 2 / grbnd[K - 1] / QS;
   d.ek[t] = EKEV(K) * 1e3 * (grel[K - 1] + 1) / 2 / grel[K - 1] / QS;
+  {  // DRIFTE's bin factors: EDOT and EDT1 share EBND*(GRBND+1)/(2 GRBND)
+    FaceBin b;
+    b.k = EBND(K) * (grbnd[K - 1] + 1) / grbnd[K - 1] / 2.;
+    b.iw = d.iwe[K - 1];
+    const uint64_t uk = dbits(b.k), uy = dbits(b.k * d.ide[K - 1]);
+    b.sk = sig_62(uk);
+    b.sy = sig_62(uy);
+    b.e = (int)(uk >> 52) - 1022;
+    b.sh = 2045 - (int)(uy >> 52);
+    b.pad = 0.0;
+    d.ebin[t] = b;
+  }
   if (K == 1) {
     const double G1 = grel[0], G2 = grel[1];
     d.kap[2 * s + 1] = G1 / G2 * sqrt((G2 * G2 - 1) / (G1 * G1 - 1));
@@ -255,6 +267,10 @@ __global__ void k_dts_small(Dev d, double DTs) {
   if (i == 0) d.p4[s * d.ne + k] = DTs * EKEV(K) * 1000.0 * (g + 1) / g / DPHI / MDR / QS;
   d.p2[t] = DTs * EKEV(K) * 1000 * (g + 1) / g / (RLZ(I) * RLZ(I)) / DPHI / QS;
   d.edot[t] = EBND(K) * DTs / RLZ(I) * (gb + 1) / gb / 2.;
+  if (k == 0) {  // DRIFTE's line factors of UE and WET
+    if (s == 0) d.er[i] = DTs / RLZ(I);
+    d.erq[s * d.nr + i] = 1e3 / QS * DTs / RLZ(I);
+  }
 }
 
 __global__ void k_dts_cells(Dev d, double DTs) {

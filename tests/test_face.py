@@ -20,8 +20,8 @@ extern "C" void flux(long n, const double* uu, const double* u, const double* d,
   for (long i = 0; i < n; ++i) {
     bool s, s2; int k = 0, k2 = 0;
     const FaceCoef q = face_coef(bits(c[i]));
-    const uint64_t a = face_flux<true>(bits(uu[i]), bits(u[i]), bits(d[i]), q, beta_fix(bits(beta)), s, k);
-    const uint64_t b = face_flux<false>(bits(uu[i]), bits(u[i]), bits(d[i]), q, beta_fix(bits(beta)), s2, k2);
+    const uint64_t a = face_flux<true, false>(bits(uu[i]), bits(u[i]), bits(d[i]), q, beta_fix(bits(beta)), s, k);
+    const uint64_t b = face_flux<false, false>(bits(uu[i]), bits(u[i]), bits(d[i]), q, beta_fix(bits(beta)), s2, k2);
     memcpy(&phi[i], &a, 8);
     cs[i] = k;
     special[i] = s | (a != b && !s) << 1 | (s != s2) << 2;  // plain and recording forms: the same bits
@@ -109,7 +109,7 @@ def test_face_flux_arithmetic(flux, kind, beta):
 def test_face_flux_leaves_out(flux):
     """Forms the fixed point does not hold are reported, whatever the other operands."""
     good = [1.0, 1.1, 1.3, 0.1]
-    for bad in (np.inf, np.nan, -1.0, -0.0, -1e-300, 1e60):
+    for bad in (np.inf, np.nan, -1.0, -0.0, -1e-300, 1e31):
         for at in range(3):
             v = list(good)
             v[at] = bad
