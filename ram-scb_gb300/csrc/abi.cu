@@ -1006,7 +1006,7 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   d.betalim = ctx->cfg.betalim;
   const int blk0[4] = {128, 128, 64, 64};
   for (int w = 0; w < 4; ++w) { d.blk[w] = blk0[w]; d.pers[w] = 0; }
-  d.mu_lanes = d.npa >= 12 ? 2 : 1;
+  d.mu_lanes = 0;  // by the number of lines
   d.lw0 = 0;
   d.lw1 = d.npa;
   const size_t nr = d.nr, nt = d.nt, ne = d.ne, npa = d.npa, ns = d.ns, nm = d.nm, nf = d.nf;
@@ -1031,7 +1031,8 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   d.mhde = dalloc<double>(ctx, ne, &ok); d.iwe = dalloc<double>(ctx, ne, &ok);
   d.ide = dalloc<double>(ctx, ne + 1, &ok);
   d.mhdmu = dalloc<double>(ctx, npa, &ok); d.iwmu = dalloc<double>(ctx, npa, &ok);
-  d.idmu = dalloc<double>(ctx, npa, &ok);
+  d.idmu = dalloc<double>(ctx, npa + 1, &ok);
+  d.mubin = dalloc<FaceMu>(ctx, npa, &ok);
   d.bmhde = dalloc<double>(ctx, ne, &ok); d.bmhdmu = dalloc<double>(ctx, npa, &ok);
   d.grel = dalloc<double>(ctx, ns * ne, &ok); d.grbnd = dalloc<double>(ctx, ns * ne, &ok);
   d.vel = dalloc<double>(ctx, ns * ne, &ok); d.epp = dalloc<double>(ctx, ns * ne, &ok);
@@ -1219,12 +1220,22 @@ int ramgpu_set_grid(ramgpu_ctx* ctx, const ramgpu_grid* g) {
   }
   CK(cudaMemcpy((void*)d.upa_atm, ua.data(), sizeof(int) * nr, cudaMemcpyHostToDevice));
   CK(cudaMemcpy((void*)d.upa_mom, um.data(), sizeof(int) * nr, cudaMemcpyHostToDevice));
-  std::vector<double> r1(ne), r2(ne), r3(ne + 1), q1(npa), q2(npa), q3(npa);
+  std::vector<double> r1(ne), r2(ne), r3(ne + 1), q1(npa), q2(npa), q3(npa + 1);
   for (int k = 0; k < ne; ++k) { r1[k] = -0.5 / G.de[k]; r2[k] = 1.0 / G.we[k]; r3[k] = 1.0 / G.de[k]; }
   r3[ne] = *std::max_element(r3.begin(), r3.begin() + ne);
   for (int l = 0; l < npa; ++l) { q1[l] = -0.5 / G.dmu[l]; q2[l] = 1.0 / G.wmu[l]; q3[l] = 1.0 / G.dmu[l]; }
+  q3[npa] = *std::max_element(q3.begin() + 1, q3.begin() + npa - 1);  // over the faces DRIFTMU counts
   CK(up(d.mhde, r1.data(), ne)); CK(up(d.iwe, r2.data(), ne)); CK(up(d.ide, r3.data(), ne + 1));
-  CK(up(d.mhdmu, q1.data(), npa)); CK(up(d.iwmu, q2.data(), npa)); CK(up(d.idmu, q3.data(), npa));
+  CK(up(d.mhdmu, q1.data(), npa)); CK(up(d.iwmu, q2.data(), npa)); CK(up(d.idmu, q3.data(), npa + 1));
+  {  // DRIFTMU's bin factors (face.cuh)
+    std::vector<FaceMu> mb(npa);
+    for (int l = 0; l < npa; ++l) {
+      uint64_t uy;
+      memcpy(&uy, &q3[l], sizeof(uy));
+      mb[l] = FaceMu{q2[l], sig_62(uy), 2045 - (int)(uy >> 52), 0, 0.0};
+    }
+    CK(cudaMemcpy((void*)d.mubin, mb.data(), sizeof(FaceMu) * npa, cudaMemcpyHostToDevice));
+  }
   for (int k = 0; k < ne; ++k) r1[k] *= d.betalim;
   for (int l = 0; l < npa; ++l) q1[l] *= d.betalim;
   CK(up(d.bmhde, r1.data(), ne)); CK(up(d.bmhdmu, q1.data(), npa));

@@ -24,12 +24,13 @@
 //
 // Bound and figures (GB300, one launch over four species on 20x25x35x72): the
 // FP64 sequence held the FP64 pipe, five operations a face in DRIFTR and
-// DRIFTP and up to seven in DRIFTE (phi, beta|X| and the Courant products
-// were integer products already).  Here three remain (the coefficient's fma
+// DRIFTP and up to seven in DRIFTE and DRIFTMU (phi, beta|X| and the Courant
+// products were integer products already).  Here three remain (the coefficient's fma
 // and the update); instruction issue (55-64 %, 170-210 instructions a face),
 // the integer ALU (60 %) and the FP64 pipe (58 %) are about even.  DRIFTR
-// 64.5 -> 52.1 us, DRIFTP 61.8 -> 46.9, DRIFTE 66.8 -> 54.4; on 40x49x70x144
-// DRIFTP 783 -> 543, DRIFTE 875 -> 580.  Normalising the factor and the
+// 64.5 -> 52.1 us, DRIFTP 61.8 -> 46.9, DRIFTE 66.8 -> 54.4, DRIFTMU 68.6 ->
+// 61.5; on 40x49x70x144 DRIFTP 783 -> 543, DRIFTE 875 -> 580, DRIFTMU 946 ->
+// 691.  Normalising the factor and the
 // differences, as the FP64 form's integer products did, took more
 // instructions than aligning the cells once.  The rare forms must stay rare:
 // before face_plain and the exact threshold below, eight warps of meridian

@@ -41,7 +41,8 @@ struct Dev {
   const double *lr2, *sinphi;  // (LZ(I)*RE)**2 (NR+1) and SIN(PHI(J)-PHIOFS) (NT) of the VOLS formula
   const int *upa_atm;   // int(UPA(I)): first loss-cone L (1-based), NR
   const int *upa_mom;   // int(UPA(I)-1): last L of the ANISCH sum, NR
-  // reciprocal grid tables: -0.5/DE, 1/WE, 1/DE (NE, then the largest 1/DE); -0.5/DMU, 1/WMU, 1/DMU (NPA)
+  // reciprocal grid tables: -0.5/DE, 1/WE, 1/DE (NE, then the largest 1/DE); -0.5/DMU, 1/WMU,
+  // 1/DMU (NPA, then the largest 1/DMU of faces 2..NPA-1)
   const double *mhde, *iwe, *ide, *mhdmu, *iwmu, *idmu;
   const double *bmhde, *bmhdmu;  // BetaLim times -0.5/DE and -0.5/DMU (adjoint)
   // per-species grid (ns x NE)
@@ -72,6 +73,7 @@ struct Dev {
   double *edot;           // (ns, NR, NE)
   double *eb, *ek;        // (ns, NE)
   FaceBin *ebin;          // (ns, NE): DRIFTE's bin factors (face.cuh), DTs-free
+  FaceMu *mubin;          // (NPA): DRIFTMU's bin factors
   double *er, *erq;       // (NR), (ns, NR): DTs/RLZ and 1e3/QS times that
   double *kap;            // (ns, 2): extrapolation factors of F(1), F(0) in DRIFTE
   double *wm;             // (NR,NT,NPA): -CMUDOT*HM, DTs-dependent, species-free
@@ -125,7 +127,7 @@ struct Dev {
   // a persistent grid of that many CTAs looping over (item, line-block) units
   int blk[4];
   int pers[4];
-  int mu_lanes;  // lanes per DRIFTMU line: 2 (lane pairs, NPA >= 12) or 1
+  int mu_lanes;  // lanes per DRIFTMU line: 1, 2 or 4 as set, 0 by the number of lines
   // L window of the R, P and E sweeps and the closing copy/mask: planes
   // [lw0, lw1) (0 and NPA: all); a host pipeline runs them chunk by chunk
   int lw0, lw1;

@@ -11,12 +11,10 @@
 //   DRIFTMU src/ModRamDrift.f90:382-473
 // with the face coefficients taken from separable tables built in tables.cu
 // (C = A(I,J) + G(I,J,L)*k(K) etc.).  The FP64 unit was the limit: sign, abs
-// and limiter tests run on bit patterns; in DRIFTR, DRIFTP and DRIFTE the
-// whole face flux is formed in 64-bit fixed point (face.cuh), which leaves
-// three FP64 operations a face (the coefficient and the two of the update);
-// in DRIFTMU the products that are only compared (beta*|X|, the CFL
-// quotients) and the flux C*FBND (mul_rn_int, rounded exactly like the FP64
-// multiply) run on the integer pipe, leaving 6.
+// and limiter tests run on bit patterns and the whole face flux is formed in
+// 64-bit fixed point (face.cuh), which leaves three FP64 operations a face:
+// the coefficient and the two of the update (DRIFTMU's forward half
+// multiplies the loss factor too).
 #include <string.h>
 
 #include <type_traits>
@@ -462,36 +460,26 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
 // faces 2..NPA-2, FBND(NPA-1) = F(NPA), then the F2(NPA) extrapolation.
 // kLoss: 0 none, 1 multiply the result by table lossA (loss after the sweep),
 //        2 multiply the input by lossA (loss before the sweep).
-// kSplit 2 or 4: there are few pitch-angle lines (NR-1)*NT*NE, so kSplit
-// adjacent lanes share one, lane q updating cells b+1..lim of segment q
-// (b = q*S, lim = (q+1)*S with S = NPA/kSplit; lane 0 from cell 2, the last
-// lane to NPA).  All run the same instructions: a "pre-face" (face 1,
-// whose flux is zero, for lane 0; face b, recomputed bit for bit from the
-// old values, for the others), then their faces.  Every old value a lane
-// needs from its neighbours' cells (its entering window and the two cells
-// past lim) is loaded before a __syncwarp, and no lane writes before it.
-// Segments keep at least 4 cells (2 lanes: NPA >= 12; 4 lanes: NPA >= 24),
-// so no lane but lane 0 sees the F(1) = F(2) rule.
-template <bool kCfl, int kLoss, int kRec, int kSplit>
-__global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const double* __restrict__ lossA,
-                                                   unsigned char* __restrict__ rec, int rsh) {
+// kSplit: there are few pitch-angle lines (NR-1)*NT*NE, so kSplit adjacent
+// lanes share one, as in DRIFTE: lane r updates the cells b+1..lim of segment
+// r (b = r*S, lim = (r+1)*S with S = NPA/kSplit; the first from cell 2, the
+// last to NPA) and forms face b anew (the first lane's face 1 carries
+// nothing).  S >= 4, so no lane but the first sees the F(1) = F(2) rule.
+template <bool kCfl, int kLoss, int kRec, bool kB32, int kSplit>
+__global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const double* __restrict__ lossA,
+                                                     unsigned char* __restrict__ rec, int rsh) {
   const int nr = d.nr, nt = d.nt, ne = d.ne, npa = d.npa;
   const int nlines = (nr - 1) * nt * ne;
   const int lpb = blockDim.x / kSplit;  // lines per CTA
-  // lane pairs: the even lane ends at Lm, the odd one takes the rest
-  const int half = kSplit == 2 ? (int)(threadIdx.x & 1) : 0;
-  const int Lm = kSplit == 2 ? npa / 2 : npa;  // last cell of the even lane
-  // four lanes: segment q4 of seg4 cells (the last one to NPA)
-  const int q4 = kSplit == 4 ? (int)(threadIdx.x & 3) : 0;
-  const int seg4 = npa / 4;
-  const int pre = kSplit == 4 ? q4 : half;  // nonzero: the pre-face is recomputed
-  const bool last = kSplit == 4 ? q4 == 3 : (half || kSplit == 1);
+  const int r = kSplit > 1 ? (int)threadIdx.x % kSplit : 0, seg = npa / kSplit;
+  const bool last = r == kSplit - 1;
+  const int b = r ? r * seg : 1, lim = last ? npa : (r + 1) * seg;
   for (Unit u((nlines + lpb - 1) / lpb); u.ok(d); u.next(d)) {
     const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
     const int line = u.b * lpb + (int)threadIdx.x / kSplit;
-    // bounds-checked builds: the line's cells, its WM and UM columns, the
-    // coefficient store's item (the lanes sharing a line test the same)
+    // bounds-checked builds: the line's cells, its WM and UM columns (the
+    // lanes sharing a line test the same)
     const bool active = line < nlines &&
         rg_ok(d, rg_item(d, item) &&
                      rg_span((long long)(line / (nr - 1)) * nr + 1 + line % (nr - 1), npa, (long long)ne * nt * nr,
@@ -512,100 +500,91 @@ __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const doubl
     double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + off;
     unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + u.it * d.ncell + off : nullptr;
     const double* __restrict__ la = lossA ? lossA + (long long)s * d.ncell + off : nullptr;
-    const long long sij = (long long)nt * nr;     // stride of (I,J,L) tables in L
-    const long long fij = (long long)j * nr + i;
-    const double* __restrict__ wm = d.wm + fij;
-    const double* __restrict__ um = d.um + (long long)m * nt * nr * npa + fij;
-    const double ekv = d.ek[s * ne + jk / nt];
-    const double* __restrict__ mhdmu = d.mhdmu;
-    const double* __restrict__ iwmu = d.iwmu;
-    const bool inside = d.outside[fij] == 0;
-    const BetaBits beta(d.betalim);
-    const bool closed = d.flags & 1u;
   #define GL(L) fl[(long long)((L)-1) * st]
   #define LA(L) la[(long long)((L)-1) * st]
   #define GLS(L) (kLoss == 2 ? GL(L) * LA(L) : GL(L))
-  #define CL(L) fma(ekv, wm[(long long)((L)-1) * sij], um[(long long)((L)-1) * sij])
-    // pre-face b (1, Lm or q4*seg4) and its window G(b-1..b+2); the first
-    // lane's F(1) is F(2); lim: last cell of this lane's range (its
-    // look-ahead beyond lim comes from the halo hA = G(lim+1), hB = G(lim+2))
-    const int b = kSplit == 4 ? (q4 ? q4 * seg4 : 1) : (half ? Lm : 1);
-    const int lim = kSplit == 4 ? (q4 == 3 ? npa : (q4 + 1) * seg4) : (half ? npa : Lm);
+    // the window G(b-1..b+2) (the first lane's F(1) is F(2)), the next cell,
+    // and the two cells past lim
     double w0 = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0, nxt = 0.0, hA = 0.0, hB = 0.0;
     if (active) {
-      w0 = GLS(pre ? b - 1 : 2);
-      w1 = GLS(pre ? b : 2);
-      w2 = GLS(b + 1 > 2 ? b + 1 : 2);
+      w2 = GLS(b + 1);
       w3 = GLS(b + 2);
-      nxt = GL(b + 3);
-      if (kSplit > 1) {
-        hA = GLS(min(lim + 1, npa));
-        hB = GLS(min(lim + 2, npa));
+      w0 = w1 = w2;
+      if (kSplit > 1 && r) {
+        w0 = GLS(b - 1);
+        w1 = GLS(b);
+      }
+      nxt = GLS(b + 3);
+      if (kSplit > 1 && !last) {
+        hA = GLS(lim + 1);
+        hB = GLS(lim + 2);
       }
     }
     if (kSplit > 1) __syncwarp();
     if (active) {
-      // pre-face: the flux entering this lane's first cell
-      double phi_prev;
-      {
-        const double c = pre ? CL(b) : 0.0;
-        const bool neg = is_neg(c);
-        const double a = fma(c, mhdmu[b - 1], neg ? -0.5 : 0.5);
-        const double xm = w1 - w0, x = w2 - w1, xp = w3 - w2;
-        int cs;
-        const double fb = (kRec == 2)
-            ? face_value_frozen(x, neg ? xp : xm, neg ? w2 : w1, a, beta, cs = rget(rl + (long long)(b - 1) * st, rsh) & 7)
-            : face_value_case(x, babs_bits(beta, x), neg ? xp : xm, babs_bits(beta, neg ? xp : xm),
-                              neg ? w2 : w1, a, cs);
-        phi_prev = c * fb;
+      const long long sij = (long long)nt * nr;     // stride of (I,J,L) tables in L
+      const long long fij = (long long)j * nr + i;
+      const double* __restrict__ wm = d.wm + fij;
+      const double* __restrict__ um = d.um + (long long)m * nt * nr * npa + fij;
+      const FaceMu* __restrict__ bins = d.mubin;
+      const double ekv = d.ek[s * ne + jk / nt];
+      const bool inside = d.outside[fij] == 0;
+      const double beta = d.betalim;
+      const uint64_t betaf = beta_fix(dbits(beta));
+      const bool closed = d.flags & 1u;
+  #define CL(L) fma(ekv, wm[(long long)((L)-1) * sij], um[(long long)((L)-1) * sij])
+      // face L's flux; the CFL quotient |C|/DMU is the Courant number
+      Largest big;
+      auto quotient = [&](double c, const FaceMu& bin) {
+        uint64_t prod;
+        face_coef_mu(dbits(c), bin, prod);
+        q = umax64(q, face_courant(dbits(c), bin.sh, prod));
+      };
+      auto face = [&](int L, const FaceMu& bin, double c, double gm, double g0, double gp, double gpp, int& cs) {
+        uint64_t prod;
+        const FaceCoef fc = face_coef_mu(dbits(c), bin, prod);
+        if (kCfl) big.see(fc, L);
+        const bool neg = fc.sign;  // C = 0 carries nothing either way
+        return face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, fc, beta, betaf, cs,
+                                    [&] { return c; }, [&] { return d.mhdmu[L - 1]; },
+                                    [&] { if (kCfl && inside) quotient(c, bin); });
+      };
+      double phi_prev = 0.0;
+      if (kSplit > 1) {
+        int cs = kRec == 2 ? (int)(rget(rl + (long long)(b - 1) * st, rsh) & 7) : 0;
+        const double phi = face(b, bins[b - 1], CL(b), w0, w1, w2, w3, cs);
+        if (r) phi_prev = phi;
+        else big = Largest();  // face 1 does not count
       }
-      double g0 = w2, gp = w3;
-      double xm = w2 - w1;
-      bits64 bxm = babs_bits(beta, xm);
-      double x = w3 - w2;
-      bits64 bx = babs_bits(beta, x);
-      const int Lend = last ? npa - 2 : (kSplit == 4 ? lim : Lm);
-      for (int L = b + 1; L <= Lend; ++L) {
-        double gpp;
-        if (kSplit > 1) {
-          gpp = (L + 2 <= lim) ? nxt : (L + 2 == lim + 1 ? hA : hB);
-          if (kLoss == 2 && L + 2 <= lim) gpp *= LA(L + 2);
-          nxt = GL(min(L + 3, lim));
-        } else {
-          gpp = nxt;
-          nxt = GL(min(L + 3, npa));
-          if (kLoss == 2) gpp *= LA(L + 2);
-        }
-        const double xp = gpp - gp; const bits64 bxp = babs_bits(beta, xp);
-        const double c = CL(L);
-        if (kCfl && inside) q = umax64(q, mul_pos_bits(cfl_bits(c, kBits1em32), d.idmu[L - 1]));
-        const bool neg = is_neg(c);
-        const double a = fma(c, mhdmu[L - 1], neg ? -0.5 : 0.5);
-        int cs;
-        const unsigned char* rq = (kRec == 1 || kRec == 2) ? rl + (long long)(L - 1) * st : nullptr;
-        const double fb = (kRec == 2) ? face_value_frozen(x, neg ? xp : xm, neg ? gp : g0, a, beta, cs = rget(rq, rsh) & 7)
-                                      : face_value_case(x, bx, neg ? xp : xm, neg ? bxp : bxm, neg ? gp : g0, a, cs);
-        const double phi = mul_rn_int(c, fb);
-        const double raw = fma(phi_prev - phi, iwmu[L - 1], g0);
+      double gm = w1, g0 = w2, gp = w3;
+      // cell L from its raw value, with its record
+      auto put = [&](int L, double raw, int cs) {
         if (kRec == 1) rput(rl + ((long long)(L - 1) * st), rsh, cs | (is_neg(raw) ? kClipBit : 0));
-        double v = (kRec == 2) ? clip_frozen(raw, rget(rq, rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
+        return (kRec == 2) ? clip_frozen(raw, rget(rl + (long long)(L - 1) * st, rsh)) : clip(raw);
+      };
+      for (int L = b + 1; L <= (last ? npa - 2 : lim); ++L) {
+        double nn = hA;
+        if (L + 3 <= lim) nn = GLS(L + 3);
+        else hA = hB;
+        const FaceMu bin = bins[L - 1];
+        int cs = kRec == 2 ? (int)(rget(rl + (long long)(L - 1) * st, rsh) & 7) : 0;
+        const double phi = face(L, bin, CL(L), gm, g0, gp, nxt, cs);
+        double v = put(L, fma(phi_prev - phi, bin.iw, g0), cs);
         if (kLoss == 1) v *= LA(L);
         GL(L) = v;
         phi_prev = phi;
-        g0 = gp; gp = gpp;
-        xm = x; bxm = bx; x = xp; bx = bxp;
+        gm = g0; g0 = gp; gp = nxt;
+        nxt = nn;
       }
       // face NPA-1: FBND = F(NPA); cell NPA-1; then the F2(NPA) ghost
       if (last) {
         const int L = npa - 1;
+        const FaceMu bin = bins[L - 1];
         const double c = CL(L);
-        if (kCfl && inside) q = umax64(q, mul_pos_bits(cfl_bits(c, kBits1em32), d.idmu[L - 1]));
+        if (kCfl && inside) quotient(c, bin);
         const double phi = c * (closed ? 0.0 : gp);
-        const double raw = fma(phi_prev - phi, iwmu[L - 1], g0);
-        if (kRec == 1) rput(rl + ((long long)(L - 1) * st), rsh, is_neg(raw) ? kClipBit : 0);
-        const double v = (kRec == 2) ? clip_frozen(raw, rget(rl + (long long)(L - 1) * st, rsh)) : clip(raw);
-        if (kRec == kRecCount) nclip += is_neg(raw);
+        const double v = put(L, fma(phi_prev - phi, bin.iw, g0), 0);
         const double vN = v * d.rho[fij];
         if (kLoss == 1) {
           GL(L) = v * LA(L);
@@ -614,6 +593,10 @@ __global__ void __launch_bounds__(256) k_sweep_mu(Dev d, double dts, const doubl
           GL(L) = v;
           GL(npa) = vN;
         }
+      }
+      if (kCfl && inside) {  // |C|/DMU, |C| at least 1e-32
+        q = umax64(q, mul_pos_bits(kBits1em32, d.idmu[npa]));
+        if (big.at) quotient(CL(big.at), bins[big.at - 1]);
       }
     }
   #undef GL
@@ -701,36 +684,52 @@ void launch_sweep_e(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigne
   else (kb ? e_launch<true, 1> : e_launch<false, 1>)(d, dts, cfl, st, rec, replay, rsh);
 }
 
-template <int kLoss, int kS>
-static void mu_launch(const Dev& d, dim3 g, int b, double dts, const double* loss, cudaStream_t st,
-                      unsigned char* rec, bool replay, bool cfl, int rsh) {
-  const bool n = d.count_clips;
-  if (rec && replay) k_sweep_mu<false, kLoss, 2, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
-  else if (rec) k_sweep_mu<false, kLoss, 1, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
-  else if (cfl) (n ? k_sweep_mu<true, kLoss, 3, kS> : k_sweep_mu<true, kLoss, 0, kS>)<<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
-  else (n ? k_sweep_mu<false, kLoss, 3, kS> : k_sweep_mu<false, kLoss, 0, kS>)<<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
+// Lanes per DRIFTMU line: as set, or (0) by the number of lines, as for
+// DRIFTE.  Measured whole calls (GB300, ms with 1, 2, 4 lanes), at 20x25x35x72
+// unless said: one species (3.4 warps an SM with one lane) 0.264, 0.224,
+// 0.203; four (14) 0.422, 0.390, 0.387; two members of four (27) 0.675,
+// 0.679, 0.698; eight (109) 2.52, 2.64, 2.71; 6x9x35x72, four species (1.3)
+// 0.193, 0.153, 0.134, and 0.122 with 8.  Segments keep at least four cells.
+static int mu_lanes(const Dev& d) {
+  int want = d.mu_lanes;
+  if (!want) {
+    const long long warps = (long long)(d.nr - 1) * d.nt * d.ne * d.nlist / 32;
+    want = warps < 2LL * d.nsm ? 8 : (warps < 16LL * d.nsm ? 4 : (warps < 24LL * d.nsm ? 2 : 1));
+  }
+  while (want > 1 && d.npa < 6 * want) want /= 2;
+  return want;
 }
-// Lines are split between d.mu_lanes adjacent lanes (2 for NPA >= 12, 4
-// for NPA >= 24: every segment keeps at least four cells, so no lane but
-// the first reads the F(1) rule).
+template <int kLoss, bool kB, int kS>
+static void mu_launch(const Dev& d, double dts, const double* loss, cudaStream_t st, unsigned char* rec, bool replay,
+                      bool cfl, int rsh) {
+  const dim3 g = grid_for(d, 3, kS * nlines_of(d, 3));
+  const int b = d.blk[3];
+  const bool n = d.count_clips;
+  if (rec && replay) k_sweep_mu<false, kLoss, 2, kB, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
+  else if (rec) k_sweep_mu<false, kLoss, 1, kB, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
+  else if (cfl)
+    (n ? k_sweep_mu<true, kLoss, 3, kB, kS> : k_sweep_mu<true, kLoss, 0, kB, kS>)<<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
+  else
+    (n ? k_sweep_mu<false, kLoss, 3, kB, kS> : k_sweep_mu<false, kLoss, 0, kB, kS>)<<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
+}
+template <int kLoss, bool kB>
+static void mu_lanes_launch(const Dev& d, double dts, const double* loss, cudaStream_t st, unsigned char* rec,
+                            bool replay, bool cfl, int rsh) {
+  const int lanes = mu_lanes(d);
+  if (lanes == 8) mu_launch<kLoss, kB, 8>(d, dts, loss, st, rec, replay, cfl, rsh);
+  else if (lanes == 4) mu_launch<kLoss, kB, 4>(d, dts, loss, st, rec, replay, cfl, rsh);
+  else if (lanes == 2) mu_launch<kLoss, kB, 2>(d, dts, loss, st, rec, replay, cfl, rsh);
+  else mu_launch<kLoss, kB, 1>(d, dts, loss, st, rec, replay, cfl, rsh);
+}
 void launch_sweep_mu(const Dev& d, double dts, bool cfl, int loss_mode, const double* loss,
                      cudaStream_t st, unsigned char* rec, bool replay, int rsh) {
-  const int lanes = (d.mu_lanes == 4 && d.npa >= 24) ? 4 : ((d.mu_lanes >= 2 && d.npa >= 12) ? 2 : 1);
-  dim3 g = grid_for(d, 3, lanes * nlines_of(d, 3));
-  const int b = d.blk[3];
-  if (lanes == 4) {
-    if (loss_mode == 1) mu_launch<1, 4>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
-    else if (loss_mode == 2) mu_launch<2, 4>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
-    else mu_launch<0, 4>(d, g, b, dts, nullptr, st, rec, replay, cfl, rsh);
-  } else if (lanes == 2) {
-    if (loss_mode == 1) mu_launch<1, 2>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
-    else if (loss_mode == 2) mu_launch<2, 2>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
-    else mu_launch<0, 2>(d, g, b, dts, nullptr, st, rec, replay, cfl, rsh);
-  } else {
-    if (loss_mode == 1) mu_launch<1, 1>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
-    else if (loss_mode == 2) mu_launch<2, 1>(d, g, b, dts, loss, st, rec, replay, cfl, rsh);
-    else mu_launch<0, 1>(d, g, b, dts, nullptr, st, rec, replay, cfl, rsh);
-  }
+  const bool kb = beta_b32(d);
+  if (loss_mode == 1)
+    (kb ? mu_lanes_launch<1, true> : mu_lanes_launch<1, false>)(d, dts, loss, st, rec, replay, cfl, rsh);
+  else if (loss_mode == 2)
+    (kb ? mu_lanes_launch<2, true> : mu_lanes_launch<2, false>)(d, dts, loss, st, rec, replay, cfl, rsh);
+  else
+    (kb ? mu_lanes_launch<0, true> : mu_lanes_launch<0, false>)(d, dts, nullptr, st, rec, replay, cfl, rsh);
 }
 
 // Resident CTAs per SM of sweep w at block size blk (for persistent grids).
@@ -741,7 +740,7 @@ int sweep_max_blocks_per_sm(int w, int blk) {
     case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_r<0, 0, true>, blk, 0); break;
     case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_p<0, 0, true>, blk, 0); break;
     case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_e<false, 0, true, 1>, blk, 0); break;
-    default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_mu<false, 0, 0, 2>, blk, 0); break;
+    default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_mu<false, 0, 0, true, 2>, blk, 0); break;
   }
   return e == cudaSuccess ? n : 0;
 }
