@@ -120,12 +120,40 @@ struct Unit {
   }
 };
 
+// V consecutive doubles, 8*V-byte aligned.
+template <int V>
+struct Vec {
+  double x[V];
+  __device__ __forceinline__ void load(const double* p) {
+    if (V == 4)
+      asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                   : "=d"(x[0]), "=d"(x[1]), "=d"(x[V > 2 ? 2 : 0]), "=d"(x[V > 2 ? 3 : 0]) : "l"(p) : "memory");
+    else
+      asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "l"(p) : "memory");
+  }
+  __device__ __forceinline__ void store(double* p) const {
+    if (V == 4)
+      asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x[0]), "d"(x[1]), "d"(x[V > 2 ? 2 : 0]),
+                   "d"(x[V > 2 ? 3 : 0]) : "memory");
+    else
+      asm volatile("st.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(x[0]), "d"(x[1]) : "memory");
+  }
+};
+
 // ----------------------------------------------------------------- DRIFTR
 // Line (J,K,L) along I = 1..NR.  Faces 2..NR-1 (and NR on inflow lines).
 // kCfl (R, P): 1 the largest |C| of the line, 2 of its cells inside the
 // magnetopause, where some lie outside.
-template <int kCfl, int kRec, bool kB32>
-__global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
+// A thread's line is contiguous, the lanes' lines 8*NR bytes apart, so a load
+// or store of one cell a lane touches 32 sectors: with V = 4 or 2 (NR a
+// multiple of it: the lines are aligned) cells, GRT and CR move V at a time,
+// whole sectors for V = 4, through a few slots of shared memory per thread
+// that the face loop reads and writes one at a time (a loop over V unrolled
+// faces does not fit the instruction cache as well).  Cells are loaded two
+// groups ahead.  No barrier: a thread touches its own slots only.
+template <int kCfl, int kRec, bool kB32, int V>
+__global__ void __launch_bounds__(256, 4) k_sweep_r(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
+  extern __shared__ double slots[];
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   // the lines of the L window [lw0, lw1) (all of them unless a pipeline
   // runs the step plane chunk by plane chunk): L is the slowest index
@@ -177,25 +205,81 @@ __global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned cha
       } else if (is_neg(cNm)) {
         g1 = stale_ghost(d, m, slot, j, k, l, p4);
       }
-      double gm = fl[0], g0 = fl[1], gp = fl[2];
-      double c = fma(grt[0], p4, cr[0]);
-      limit(1, c);
+      double gm, g0, gp, phi_prev;
       // face 1: FBND(1) = 0 (outflow) or F(2) (inflow)
-      double phi_prev = c * ((inflow && !closed) ? g0 : 0.0);
-      for (int f = 2; f <= nr - 1; ++f) {  // 1-based face f, updates cell f
-        const double gpp = (f + 2 <= nr) ? fl[f + 1] : g1;
-        c = ((f == nr - 1) ? cNm : fma(grt[f - 1], p4, cr[f - 1]));
+      auto begin = [&](double c) {
+        limit(1, c);
+        phi_prev = c * ((inflow && !closed) ? g0 : 0.0);
+      };
+      // face f, 2 <= f <= NR-1: the new cell f
+      auto step = [&](int f, double c, double gpp) {
         limit(f, c);
         const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
         int cs = kRec == 2 ? (int)(rget(rl + (f - 1), rsh) & 7) : 0;
         const double phi = face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), beta,
                                                 betaf, cs, [&] { return c; }, mh);
         const double raw = (g0 - phi) + phi_prev;
-        fl[f - 1] = (kRec == 2) ? clip_frozen(raw, rget(rl + (f - 1), rsh)) : clip(raw);
+        const double v = (kRec == 2) ? clip_frozen(raw, rget(rl + (f - 1), rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
         if (kRec == 1) rput(rl + (f - 1), rsh, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
         gm = g0; g0 = gp; gp = gpp;
+        return v;
+      };
+      double* slot0 = slots + threadIdx.x;
+      const int bd = blockDim.x, ng = nr / V;
+      if (V == 1) {
+        gm = fl[0]; g0 = fl[1]; gp = fl[2];
+        begin(fma(grt[0], p4, cr[0]));
+        for (int f = 2; f <= nr - 1; ++f) {
+          const double gpp = (f + 2 <= nr) ? fl[f + 1] : g1;
+          fl[f - 1] = step(f, (f == nr - 1) ? cNm : fma(grt[f - 1], p4, cr[f - 1]), gpp);
+        }
+      } else {
+        // slots 0..2V-1: cells, cell n at (n-1) mod 2V; 2V..3V-1: the group's
+        // coefficients, replaced by its new cells
+        constexpr int W = V > 1 ? V : 2;
+        Vec<W> x;
+        auto fill = [&](int g) {  // group g into its half (the ghosts after the last)
+          if (g < ng)
+            for (int t = 0; t < W; ++t) slot0[((g & 1) * W + t) * bd] = x.x[t];
+          else if (g == ng) {
+            slot0[(g & 1) * W * bd] = g1;
+            slot0[((g & 1) * W + 1) * bd] = g2;
+          }
+        };
+        x.load(fl);
+        gm = x.x[0]; g0 = x.x[1];
+        fill(0);
+        if (ng > 1) x.load(fl + W);
+        fill(1);
+        gp = slot0[2 * bd];
+        if (ng > 2) x.load(fl + 2 * W);
+        for (int g = 0; g < ng; ++g) {
+          Vec<W> a, b;
+          a.load(grt + g * W);
+          b.load(cr + g * W);
+          for (int t = 0; t < W; ++t) slot0[(2 * W + t) * bd] = fma(a.x[t], p4, b.x[t]);
+          int t = 0;
+          if (g == 0) {
+            begin(slot0[2 * W * bd]);
+            slot0[2 * W * bd] = gm;  // cell 1 keeps its value
+            t = 1;
+          }
+          const int te = g == ng - 1 ? W - 1 : W;
+#pragma unroll 1
+          for (; t < te; ++t) {
+            double* cell = slot0 + (2 * W + t) * bd;
+            const int f = g * W + t + 1;
+            *cell = step(f, *cell, slot0[((f + 1) & (2 * W - 1)) * bd]);
+          }
+          if (g < ng - 1) {
+            for (int t2 = 0; t2 < W; ++t2) a.x[t2] = slot0[(2 * W + t2) * bd];
+            a.store(fl + g * W);
+            fill(g + 2);
+            if (g + 3 < ng) x.load(fl + (g + 3) * W);
+          }
+        }
       }
       // face NR (g0 = F(NR), gp = F(NR+1)): limited on inflow lines, F(NR)
       // on outflow lines
@@ -206,7 +290,16 @@ __global__ void __launch_bounds__(256) k_sweep_r(Dev d, double dts, unsigned cha
         phin = inflow ? face_phi<kRec, kB32>(g2, g1, g0, cN, face_coef(dbits(cN)), beta, betaf, csn, [&] { return cN; }, mh)
                       : mul_rn_int(cN, g0);
       const double rawn = (g0 - phin) + phi_prev;
-      fl[nr - 1] = (kRec == 2) ? clip_frozen(rawn, rget(rl + (nr - 1), rsh)) : clip(rawn);
+      const double vn = (kRec == 2) ? clip_frozen(rawn, rget(rl + (nr - 1), rsh)) : clip(rawn);
+      if (V == 1) {
+        fl[nr - 1] = vn;
+      } else {
+        constexpr int W = V > 1 ? V : 2;
+        Vec<W> a;
+        for (int t = 0; t < W - 1; ++t) a.x[t] = slot0[(2 * W + t) * bd];
+        a.x[W - 1] = vn;
+        a.store(fl + nr - W);
+      }
       if (kRec == kRecCount) nclip += is_neg(rawn);
       if (kRec == 1) rput(rl + (nr - 1), rsh, csn | (is_neg(rawn) ? kClipBit : 0));
     }
@@ -650,9 +743,36 @@ static inline bool beta_b32(const Dev& d) {
     if (beta_b32(d)) NAME##_b<true>(d, dts, cfl, st, rec, replay, rsh);                                       \
     else NAME##_b<false>(d, dts, cfl, st, rec, replay, rsh);                                                  \
   }
-SWEEP_LAUNCHER(launch_sweep_r, k_sweep_r, 0)
 SWEEP_LAUNCHER(launch_sweep_p, k_sweep_p, 1)
 #undef SWEEP_LAUNCHER
+
+template <bool kB, int V>
+static void r_launch(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int rsh) {
+  const dim3 g = grid_for(d, 0, nlines_of(d, 0));
+  const int b = d.blk[0];
+  const size_t sm = V > 1 ? 3 * V * b * sizeof(double) : 0;
+  const bool n = d.count_clips;
+  if (rec && replay) k_sweep_r<0, 2, kB, V><<<g, b, sm, st>>>(d, dts, rec, rsh);
+  else if (rec) k_sweep_r<0, 1, kB, V><<<g, b, sm, st>>>(d, dts, rec, rsh);
+  else if (cfl && (d.flags >> 31)) (n ? k_sweep_r<2, 3, kB, V> : k_sweep_r<2, 0, kB, V>)<<<g, b, sm, st>>>(d, dts, nullptr, 0);
+  else if (cfl) (n ? k_sweep_r<1, 3, kB, V> : k_sweep_r<1, 0, kB, V>)<<<g, b, sm, st>>>(d, dts, nullptr, 0);
+  else (n ? k_sweep_r<0, 3, kB, V> : k_sweep_r<0, 0, kB, V>)<<<g, b, sm, st>>>(d, dts, nullptr, 0);
+}
+// Cells per access.  While an SM's lines (32 warps of 8*NR bytes a lane) stay
+// in L1 (NR up to 24), cells move one at a time: the wide accesses bring
+// nothing (NR = 20, us a launch over four species: 52.1 with one, 56.7 with
+// two, 51.6 with four; the call 0.386, 0.397, 0.389 ms).  Longer lines fall
+// out of L1 between a lane's cells, and the widest access that divides NR
+// (then every line, GRT and CR row starts on its boundary) reads and writes
+// whole sectors once (NR = 40: 863, 733, 610; L2 traffic down to 0.4).
+static int r_width(const Dev& d) { return d.nr <= 24 || d.nr % 2 ? 1 : (d.nr % 4 ? 2 : 4); }
+void launch_sweep_r(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int rsh) {
+  const bool kb = beta_b32(d);
+  const int v = r_width(d);
+  if (v == 4) (kb ? r_launch<true, 4> : r_launch<false, 4>)(d, dts, cfl, st, rec, replay, rsh);
+  else if (v == 2) (kb ? r_launch<true, 2> : r_launch<false, 2>)(d, dts, cfl, st, rec, replay, rsh);
+  else (kb ? r_launch<true, 1> : r_launch<false, 1>)(d, dts, cfl, st, rec, replay, rsh);
+}
 
 // Lanes per DRIFTE line.  A line is a serial chain of NE faces; with few
 // lines an SM has too few warps to hide it, and splitting lines gives more,
@@ -737,7 +857,7 @@ int sweep_max_blocks_per_sm(int w, int blk) {
   int n = 0;
   cudaError_t e = cudaSuccess;
   switch (w) {
-    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_r<0, 0, true>, blk, 0); break;
+    case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_r<0, 0, true, 4>, blk, 3 * 4 * blk * sizeof(double)); break;
     case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_p<0, 0, true>, blk, 0); break;
     case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_e<false, 0, true, 1>, blk, 0); break;
     default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_mu<false, 0, 0, true, 2>, blk, 0); break;

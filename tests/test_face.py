@@ -180,3 +180,56 @@ def test_sweeps_at_the_limits(kind, beta):
             bad = np.abs(got - ref) > 64 * 2.0 ** -53 * scale
             assert not bad.any(), (which, s, int(bad.sum()), np.argwhere(bad)[:3].tolist())
     gpu.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("field", ["dipole", "perturbed"])
+@pytest.mark.parametrize("nr", [4, 6, 23, 25, 26, 28, 30, 32])
+def test_radial_widths(nr, field):
+    """Grids of every DRIFTR access width (one, two or four cells), at the
+    smallest and at both sides of each rule: two calls against the oracle,
+    1e-12 of the largest cell (the step's parity bar)."""
+    from ramgpu import abi, workload as W
+    import pyoracle
+    g = W.arrays(nr, 9, 35, 72, species=(W.HYDROGEN,), mu_grid_nr=20)
+    f = W.perturbed_fields(g, seed=nr) if field == "perturbed" else W.dipole_fields(g, seed=nr)
+    f2, fg = np.asfortranarray(W.initial_f2(g, f, 0, nr)), W.boundary_fgeos(g, 0)
+    gpu, o = abi.RamGpu(g, f), pyoracle.Oracle(g, f)
+    gpu.upload_f2(0, 0, f2)
+    gpu.set_boundary(0, 0, fg)
+    ref = [f2.copy(order="F")]
+    for c in range(2):
+        gpu.set_kp(0, 3.0 + c)
+        gpu.ram_run(3.0)
+        out = o.ram_run(ref, [fg], 3.0, kp=3.0 + c)
+        got = gpu.download_f2(0, 0)
+        assert np.abs(got - ref[0]).max() <= 1e-12 * np.abs(ref[0]).max()
+        assert abs(gpu.cfl(0, 0)[4] - out["dts_next"]) <= 1e-12 * out["dts_next"]
+    gpu.close()
+
+
+@pytest.mark.gpu
+def test_lane_counts_agree():
+    """DRIFTE and DRIFTMU share a line among 4 and 8 lanes for one member of
+    the reduced grid and among fewer as members join: member 0's F2, moments
+    and Courant limits are the same bits in every list."""
+    from ramgpu import abi, workload as W
+    wl = W.make_workload("tiny_pert")
+    g, ns = wl.grid, len(wl.grid.species)
+    first = None
+    for members in (1, 3, 16, 24):
+        gpu = abi.RamGpu(g, wl.fields, n_members=members)
+        for m in range(members):
+            for s in range(ns):
+                gpu.upload_f2(m, s, np.asfortranarray(wl.f2[s]))
+                gpu.set_boundary(m, s, wl.fgeos[s])
+        gpu.set_kp_all([4.0] * members)
+        for _ in range(3):
+            gpu.ram_run(wl.dts)
+        got = [gpu.download_f2(0, s) for s in range(ns)] + [np.array(gpu.moments(0, s)) for s in range(ns)] \
+            + [gpu.cfl(0, s) for s in range(ns)]
+        gpu.close()
+        if first is None:
+            first = got
+        for a, b in zip(got, first):
+            assert np.array_equal(a, b), members
