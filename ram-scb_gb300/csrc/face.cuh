@@ -153,8 +153,7 @@ struct alignas(16) FaceBin {
   int e, sh;            // exponent of k less 1022; 2045 less that of k/DE
   double pad;
 };
-// prod: the significands' product of U, 2^62 <= prod < 2^64, for face_courant.
-RG_HD FaceCoef face_coef_bin(uint64_t v, const FaceBin& b, uint64_t& prod) {
+RG_HD FaceCoef face_coef_bin(uint64_t v, const FaceBin& b) {
   FaceCoef q;
   const uint32_t h = (uint32_t)(v >> 32);
   const int ev = (int)((h >> 20) & 0x7FFu);
@@ -162,7 +161,7 @@ RG_HD FaceCoef face_coef_bin(uint64_t v, const FaceBin& b, uint64_t& prod) {
   q.sign = h & 0x80000000u;
   q.e = ev + b.e;
   q.m = mulhi_cross(sv, b.sk) << 1;
-  prod = mulhi_cross(sv, b.sy) << 2;
+  const uint64_t prod = mulhi_cross(sv, b.sy) << 2;  // of U, 2^62 <= prod < 2^64
   const int sh = b.sh - ev;
   q.a63 = 0x7FFFFFFFFFFFFFFFULL - shr_clamp(prod, sh);
   q.bad = sh | hi32(q.a63) | (2046 - ev);
@@ -175,27 +174,18 @@ struct alignas(16) FaceMu {
   int sh, pad0;         // 2045 less the exponent of 1/DMU
   double pad1;
 };
-RG_HD FaceCoef face_coef_mu(uint64_t c, const FaceMu& b, uint64_t& prod) {
+RG_HD FaceCoef face_coef_mu(uint64_t c, const FaceMu& b) {
   FaceCoef q;
   const uint32_t h = (uint32_t)(c >> 32);
   q.sign = h & 0x80000000u;
   q.e = (int)((h >> 20) & 0x7FFu);
   q.m = sig_62(c);
-  prod = mulhi_cross(q.m, b.sy) << 2;
+  const uint64_t prod = mulhi_cross(q.m, b.sy) << 2;
   const int sh = b.sh - q.e;
   q.a63 = 0x7FFFFFFFFFFFFFFFULL - shr_clamp(prod, sh);
   q.bad = sh | hi32(q.a63) | (2046 - q.e);
   return q;
 }
-// U as bits, cut to 53 bits: 0 where v is zero or subnormal or U underflows,
-// |v| itself where it is infinite or NaN.
-RG_HD uint64_t face_courant(uint64_t v, int sh, uint64_t prod) {
-  const int ev = (int)((v >> 52) & 0x7FFu), top = (int)(prod >> 63);
-  const int e = ev + 1022 - sh + top;
-  const uint64_t r = ((uint64_t)(uint32_t)e << 52) | ((prod >> (10 + top)) & 0x000FFFFFFFFFFFFFULL);
-  return ev == 0x7FF ? (v & 0x7FFFFFFFFFFFFFFFULL) : (ev == 0 || e <= 0 ? 0ULL : r);
-}
-
 // Cells of 2^100 and more, and products phi below about 2^-919, are special
 // too: with those limits one sign test of the exponent of phi covers every
 // zero and subnormal operand.

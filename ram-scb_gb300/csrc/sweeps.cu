@@ -89,7 +89,8 @@ __device__ __forceinline__ double face_phi(double uu, double u, double d, double
 }
 
 // The line's largest Courant number, as the face with the smallest 1 - U:
-// its quotient is formed once, after the line.  Faces whose U differ by less
+// its quotient is formed once, after the line, in FP64 (a few operations a
+// line; every face's took 16 integer instructions and cut the quotient).  Faces whose U differ by less
 // than 2^-63 count as equal, which moves DtDrift by at most one rounding
 // wherever it is below its cap.
 struct Largest {
@@ -487,16 +488,16 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
       // Face K: its flux.  At face NE against the flow FUP = F(NE+1) = 0: that
       // flux is zero whatever the other cells (end).
       Largest big;
+      auto quotient = [&](int K, double c) { q = umax64(q, dbits(c * d.ide[K - 1]) & kAbsMask); };
       auto face = [&](int K, const FaceBin& bin, double v, double gm, double g0, double gp, double gpp, int& cs,
                       auto end) {
-        uint64_t prod;
-        const FaceCoef fc = face_coef_bin(dbits(v), bin, prod);
+        const FaceCoef fc = face_coef_bin(dbits(v), bin);
         if (kCfl) big.see(fc, K);
         const bool none = decltype(end)::value && fc.sign && abs_lt_inf(v), neg = fc.sign && !none;
         const double phi = face_phi<kRec, kB32>(
             neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, v, fc, beta, betaf, cs, [&] { return bin.k * v; },
             [&] { return d.mhde[K - 1]; },
-            [&] { if (kCfl && inside) q = umax64(q, face_courant(dbits(v), bin.sh, prod)); });
+            [&] { if (kCfl && inside) quotient(K, bin.k * v); });
         if (none) cs = 0;
         return none ? 0.0 : phi;
       };
@@ -534,11 +535,8 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
       if (kCfl && inside) {  // |C|/DE, |C| at least 1e-10
         q = umax64(q, mul_pos_bits(kBits1em10, d.ide[ne]));
         if (big.at) {
-          const FaceBin bin = bins[big.at - 1];
-          const double vb = fma(bin.k, wet, ue);
-          uint64_t prod;
-          face_coef_bin(dbits(vb), bin, prod);
-          q = umax64(q, face_courant(dbits(vb), bin.sh, prod));
+          const double k = bins[big.at - 1].k;
+          quotient(big.at, k * fma(k, wet, ue));
         }
       }
     }
@@ -628,19 +626,14 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
   #define CL(L) fma(ekv, wm[(long long)((L)-1) * sij], um[(long long)((L)-1) * sij])
       // face L's flux; the CFL quotient |C|/DMU is the Courant number
       Largest big;
-      auto quotient = [&](double c, const FaceMu& bin) {
-        uint64_t prod;
-        face_coef_mu(dbits(c), bin, prod);
-        q = umax64(q, face_courant(dbits(c), bin.sh, prod));
-      };
+      auto quotient = [&](int L, double c) { q = umax64(q, dbits(c * d.idmu[L - 1]) & kAbsMask); };
       auto face = [&](int L, const FaceMu& bin, double c, double gm, double g0, double gp, double gpp, int& cs) {
-        uint64_t prod;
-        const FaceCoef fc = face_coef_mu(dbits(c), bin, prod);
+        const FaceCoef fc = face_coef_mu(dbits(c), bin);
         if (kCfl) big.see(fc, L);
         const bool neg = fc.sign;  // C = 0 carries nothing either way
         return face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, fc, beta, betaf, cs,
                                     [&] { return c; }, [&] { return d.mhdmu[L - 1]; },
-                                    [&] { if (kCfl && inside) quotient(c, bin); });
+                                    [&] { if (kCfl && inside) quotient(L, c); });
       };
       double phi_prev = 0.0;
       if (kSplit > 1) {
@@ -675,7 +668,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
         const int L = npa - 1;
         const FaceMu bin = bins[L - 1];
         const double c = CL(L);
-        if (kCfl && inside) quotient(c, bin);
+        if (kCfl && inside) quotient(L, c);
         const double phi = c * (closed ? 0.0 : gp);
         const double v = put(L, fma(phi_prev - phi, bin.iw, g0), 0);
         const double vN = v * d.rho[fij];
@@ -689,7 +682,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
       }
       if (kCfl && inside) {  // |C|/DMU, |C| at least 1e-32
         q = umax64(q, mul_pos_bits(kBits1em32, d.idmu[npa]));
-        if (big.at) quotient(CL(big.at), bins[big.at - 1]);
+        if (big.at) quotient(big.at, CL(big.at));
       }
     }
   #undef GL
