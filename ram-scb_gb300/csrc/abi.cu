@@ -42,8 +42,6 @@ using namespace ramgpu;
 
 namespace {
 thread_local std::string g_create_error;
-constexpr int kSumrcBlocks = 64;
-constexpr int kSumrcStages = 9;  // 0-5 ram_run, 6-7 pitch-angle diffusion, 8 reset
 }  // namespace
 
 struct ramgpu_ctx {
@@ -76,7 +74,8 @@ struct ramgpu_ctx {
   double last_dts = 0.0;
   // loss bookkeeping on the device: per slot {SETRC, LSDR, LSCHA, LSATM, valid}
   double* losses = nullptr;
-  double* sumrc_part = nullptr;
+  double* book_part = nullptr;     // the blocks' partial sums, per slot
+  unsigned* book_done = nullptr;   // blocks done, per slot (0 between launches)
   double* upa_h_dummy = nullptr;
   long long launches = 0;
   long long graph_launch_count = 0;
@@ -371,35 +370,16 @@ static void ensure_coef(ramgpu_ctx* ctx) {
   }
 }
 
-// SUMRC of every item into stage buffer `stage`, then fold into the device
-// accumulators: which = -1 (set SETRC only), 1 LSDR, 2 LSCHA, 3 LSATM,
-// 5 LSWAE (index 4 marks a valid SETRC).
-__global__ void k_losses_fold(Dev d, const double* part, int nblk, double* losses, int which) {
-  const int it = blockIdx.x * blockDim.x + threadIdx.x;
-  if (it >= d.nitems) return;
-  const int2 item = d.items[it];
-  const int slot = item.x * d.ns + item.y;
-  double s = 0.0;
-  for (int b = 0; b < nblk; ++b) s += part[(long long)it * nblk + b];
-  double* L = losses + (long long)slot * 6;
-  if (which >= 1 && L[4] != 0.0) L[which] += L[0] - s;  // ELORC = ENOLD - SETRC
-  L[0] = s;
-  L[4] = 1.0;
-}
-
-static int sumrc_stage(ramgpu_ctx* ctx, int stage, int which) {
-  double* part = ctx->sumrc_part + (size_t)stage * ctx->d.nm * ctx->d.ns * kSumrcBlocks;
+// SETRC of every item, its change booked to channel `which` (tables.cu).
+static int sumrc_stage(ramgpu_ctx* ctx, int which) {
   Timed tm_(ctx, 9);
-  launch_sumrc(ctx->d, part, kSumrcBlocks, ctx->stream);
-  k_losses_fold<<<(ctx->d.nitems + 127) / 128, 128, 0, ctx->stream>>>(ctx->d, part, kSumrcBlocks,
-                                                                     ctx->losses, which);
-  ctx->launches += 2;
+  launch_books(ctx->d, false, ctx->book_part, ctx->book_done, ctx->losses, which, ctx->stream);
+  ctx->launches += 1;
   CKL("sumrc");
   return RAMGPU_OK;
 }
 
-// Forward sweeps with the CFL reduction; when the coefficient store exists
-// they also keep each face's C and CORR factor for the reverse half.
+// Forward sweeps with the CFL reduction.
 static int enqueue_forward(ramgpu_ctx* ctx, double dts, bool loss_fused, const double* loss_table,
                            bool clear_cfl = true) {
   if (clear_cfl)
@@ -414,10 +394,8 @@ static int enqueue_forward(ramgpu_ctx* ctx, double dts, bool loss_fused, const d
   return RAMGPU_OK;
 }
 
-// Reverse sweeps; after_forward: the forward half of the same call ran just
-// before, so its stored face coefficients are read back.
-static int enqueue_reverse(ramgpu_ctx* ctx, double dts, bool loss_fused, const double* loss_table,
-                           bool after_forward) {
+// Reverse sweeps.
+static int enqueue_reverse(ramgpu_ctx* ctx, double dts, bool loss_fused, const double* loss_table) {
   const Dev& d = ctx->d;
   { Timed t(ctx, 5); launch_sweep_mu(d, dts, false, loss_fused ? 2 : 0, loss_table, ctx->stream); }
   { Timed t(ctx, 4); launch_sweep_e(d, dts, false, ctx->stream); }
@@ -438,7 +416,7 @@ static int enqueue_sweeps(ramgpu_ctx* ctx, double dts, bool clear_cfl) {
   if (!losses && !pd) {
     // R,P,E,MU then CEX,ATMOL,ATMOL,CEX folded into the MU store
     if ((rc = enqueue_forward(ctx, dts, true, ctx->d.loss2, clear_cfl))) return rc;
-    if ((rc = enqueue_reverse(ctx, dts, false, nullptr, true))) return rc;
+    if ((rc = enqueue_reverse(ctx, dts, false, nullptr))) return rc;
   } else if (!losses) {
     // R,P,E,MU, WPADIF, CEX,ATMOL,ATMOL,CEX (folded into WPADIF's store), WPADIF, MU,E,P,R
     if ((rc = enqueue_forward(ctx, dts, false, nullptr, clear_cfl))) return rc;
@@ -446,31 +424,28 @@ static int enqueue_sweeps(ramgpu_ctx* ctx, double dts, bool clear_cfl) {
     { Timed t(ctx, 10); launch_padif(ctx->d, nullptr, ctx->stream); }
     ctx->launches += 2;
     CKL("pitch-angle diffusion");
-    if ((rc = enqueue_reverse(ctx, dts, false, nullptr, true))) return rc;
+    if ((rc = enqueue_reverse(ctx, dts, false, nullptr))) return rc;
   } else {
     if ((rc = enqueue_forward(ctx, dts, false, nullptr, clear_cfl))) return rc;
-    if ((rc = sumrc_stage(ctx, 0, 1))) return rc;
+    if ((rc = sumrc_stage(ctx, 1))) return rc;
     if (pd) {
       { Timed t(ctx, 10); launch_padif(ctx->d, nullptr, ctx->stream); }
       ctx->launches += 1;
-      if ((rc = sumrc_stage(ctx, 6, 5))) return rc;
+      if ((rc = sumrc_stage(ctx, 5))) return rc;
     }
-    { Timed t(ctx, 9); launch_loss_apply(ctx->d, ctx->d.charge, ctx->stream); }
-    if ((rc = sumrc_stage(ctx, 1, 2))) return rc;
-    { Timed t(ctx, 9); launch_loss_apply(ctx->d, ctx->d.atm, ctx->stream); }
-    if ((rc = sumrc_stage(ctx, 2, 3))) return rc;
-    { Timed t(ctx, 9); launch_loss_apply(ctx->d, ctx->d.atm, ctx->stream); }
-    if ((rc = sumrc_stage(ctx, 3, 3))) return rc;
-    { Timed t(ctx, 9); launch_loss_apply(ctx->d, ctx->d.charge, ctx->stream); }
-    if ((rc = sumrc_stage(ctx, 4, 2))) return rc;
-    ctx->launches += 4;
+    {
+      Timed t(ctx, 9);
+      launch_books(ctx->d, true, ctx->book_part, ctx->book_done, ctx->losses, 0, ctx->stream);
+    }
+    ctx->launches += 1;
+    CKL("losses");
     if (pd) {
       { Timed t(ctx, 10); launch_padif(ctx->d, nullptr, ctx->stream); }
       ctx->launches += 1;
-      if ((rc = sumrc_stage(ctx, 7, 5))) return rc;
+      if ((rc = sumrc_stage(ctx, 5))) return rc;
     }
-    if ((rc = enqueue_reverse(ctx, dts, false, nullptr, true))) return rc;
-    if ((rc = sumrc_stage(ctx, 5, 1))) return rc;
+    if ((rc = enqueue_reverse(ctx, dts, false, nullptr))) return rc;
+    if ((rc = sumrc_stage(ctx, 1))) return rc;
   }
   { Timed t(ctx, 6); launch_finish(ctx->d, ctx->stream); }
   if (ctx->finish_hook) CK(cudaEventRecord(ctx->finish_hook, ctx->stream));
@@ -525,11 +500,10 @@ static int over_groups(ramgpu_ctx* ctx, int G, F&& fn) {
   return RAMGPU_OK;
 }
 
-// Item groups of a step: 1 with the loss bookkeeping (its partial sums are
-// indexed by list position) and in per-kernel timing passes (the events sit
-// on one stream), else the given count, at most one group per item.
+// Item groups of a step: 1 in per-kernel timing passes (the events sit on
+// one stream), else the given count, at most one group per item.
 static int clamp_groups(const ramgpu_ctx* ctx, int groups) {
-  if ((ctx->cfg.flags & RAMGPU_FLAG_LOSSES) || ctx->timing) return 1;
+  if (ctx->timing) return 1;
   return std::max(1, std::min(groups, ctx->d.nitems));
 }
 
@@ -1097,7 +1071,8 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   d.ppart = dalloc<double>(ctx, nslot * nr * nt, &ok);
   ctx->items_d = dalloc<int2>(ctx, nslot, &ok);
   ctx->losses = dalloc<double>(ctx, nslot * 6, &ok);
-  ctx->sumrc_part = dalloc<double>(ctx, (size_t)kSumrcStages * nslot * kSumrcBlocks, &ok);
+  ctx->book_part = dalloc<double>(ctx, books_part_doubles(nslot), &ok);
+  ctx->book_done = dalloc<unsigned>(ctx, nslot, &ok);
   ctx->status_d = dalloc<unsigned long long>(ctx, 5, &ok);
   ctx->stat_part = dalloc<double>(ctx, kF2StatBlocks, &ok);
   ctx->stat_mm = dalloc<unsigned long long>(ctx, 2, &ok);
@@ -2074,7 +2049,7 @@ int ramgpu_half_step(ramgpu_ctx* ctx, double dts, int order) {
   ctx->launches += 3;
   CKL("member tables");
   if (order == 0) rc = enqueue_forward(ctx, dts, true, ctx->d.loss1);
-  else rc = enqueue_reverse(ctx, dts, true, ctx->d.loss1, false);
+  else rc = enqueue_reverse(ctx, dts, true, ctx->d.loss1);
   if (rc) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   return RAMGPU_OK;
@@ -2214,7 +2189,7 @@ int ramgpu_reset_losses(ramgpu_ctx* ctx) {
       if (rc) return rc;
     }
     if (ctx->d.nitems > 0) {
-      int rc = sumrc_stage(ctx, kSumrcStages - 1, -1);
+      int rc = sumrc_stage(ctx, -1);
       if (rc) return rc;
     }
   }
@@ -2455,7 +2430,7 @@ int ramgpu_autotune(ramgpu_ctx* ctx, double dts, int reps, double* best_ms4) {
   }
   // then the number of concurrent item groups, 1, 2, 4 or 8 (at most one
   // per item), on the chosen shapes
-  if (!(ctx->cfg.flags & RAMGPU_FLAG_LOSSES)) {
+  {
     float best = 1e30f;
     int bg = ctx->step_groups;
     for (int G = 1; G <= 8 && G <= ctx->d.nitems; G *= 2) {

@@ -72,7 +72,9 @@ void launch_loss_apply(const Dev& d, const double* table, cudaStream_t st);
 void launch_finish(const Dev& d, cudaStream_t st);
 void launch_moments(const Dev& d, cudaStream_t st);
 void launch_anisch_state(const Dev& d, cudaStream_t st);
-void launch_sumrc(const Dev& d, double* part, int nblk, cudaStream_t st);
+void launch_books(const Dev& d, bool all_losses, double* part, unsigned* done, double* losses, int which,
+                  cudaStream_t st);
+size_t books_part_doubles(size_t nslot);
 void launch_flux(const Dev& d, int slot, int s, double* out, cudaStream_t st);
 
 // ---- frozen-limiter adjoint (adjoint.cu)

@@ -112,7 +112,6 @@ struct Dev {
   int count_clips;            // the sweeps count clip events (status pass on)
   double *mom_part;       // (nm*ns, NT, NR, (NE-1)*4 chunks, 2) moment partials
   double *ppert, *ppart;  // (nm*ns, NR, NT)
-  double *sumrc_part;     // (nm*ns, nblk) SUMRC partial sums
   // face coefficients C of a call's first DRIFTE transpose, read back by the
   // second: (coef_items, ncell); null when not allocated
   double* coef;

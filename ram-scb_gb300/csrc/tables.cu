@@ -703,37 +703,119 @@ void launch_anisch_state(const Dev& d, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ SUMRC
-// Per-block partial sums of EKEV*F2*WE*WMU over I=2..NR, J=1..NT-1,
-// K=2..NE, L=2..NPA (src/ModRamRun.f90:246-255).  part: (nitems, nblk).
-__global__ void __launch_bounds__(256) k_sumrc(Dev d, double* part, int nblk) {
-  __shared__ double sh[256];
+// The bookkeeping of SUMRC (src/ModRamRun.f90:231-259): SETRC, the sum of
+// EKEV*F2*WE*WMU over I = 2..NR, J = 1..NT-1, K = 2..NE, L = 2..NPA, after
+// each process, its change booked to that process's channel.  kN = 1: one
+// sum of the state as it is.  kN = 4: CHAREXCHANGE, ATMOL, ATMOL,
+// CHAREXCHANGE (src/ModRamRun.f90:136-157) applied in one pass over F2, each
+// product rounded as a pass of its own would, with the sum after each.
+// The two factors are 1 on the planes K = 1 and L = 1, which are left out.
+//
+// A warp takes whole (K, L) planes, NR*NT contiguous cells with one weight,
+// so a cell costs one FP64 add (and its products), no division and no
+// weight.  The last block of an item sums the blocks' partials in order and
+// books them.  Bound by FP64 issue at kN = 4 (8 operations a cell).  Two ions
+// on 20x25x35x72: with one pass a process and one a sum (a division by each
+// size per cell, 64 blocks an item, a fold launch each) the call took 785 us,
+// with these three 395.
+constexpr int kBookBlocks = 152;  // two planes a warp on the standard grid
+template <int kN>
+__global__ void __launch_bounds__(256) k_books(Dev d, double* __restrict__ part, unsigned* __restrict__ done,
+                                               double* __restrict__ losses, int which) {
+  __shared__ double sh[8][kN];
+  __shared__ bool lastblk;
   const int2 item = d.items[blockIdx.y];
-  const int slot = item.x * d.ns + item.y;
-  const double* f = d.f2 + (long long)slot * d.ncell;
-  double acc = 0.0;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < d.ncell;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int I = 1 + (int)(c % d.nr);
-    const int J = 1 + (int)((c / d.nr) % d.nt);
-    const int K = 1 + (int)((c / ((long long)d.nr * d.nt)) % d.ne);
-    const int L = 1 + (int)(c / ((long long)d.nr * d.nt * d.ne));
-    if (I >= 2 && J <= d.nt - 1 && K >= 2 && L >= 2) {
-      const double WEIGHT = f[c] * WE(K) * WMU(L);
-      acc = acc + EKEV(K) * WEIGHT;
+  const int s = item.y, slot = item.x * d.ns + s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ne1 = d.ne - 1, np = ne1 * (d.npa - 1), nr = d.nr;
+  const int ncount = (d.nt - 1) * nr, ncells = d.nt * nr, dr = 32 % nr;
+  double acc[kN];
+#pragma unroll
+  for (int q = 0; q < kN; ++q) acc[q] = 0.0;
+  for (int p = blockIdx.x * 8 + warp; p < np; p += gridDim.x * 8) {
+    const int k = 1 + p % ne1, l = 1 + p / ne1;
+    const long long base = ((long long)l * d.ne + k) * ncells;
+    double* __restrict__ f = d.f2 + (long long)slot * d.ncell + base;
+    const double* __restrict__ ch = d.charge + (long long)s * d.ncell + base;
+    const double* __restrict__ at = d.atm + (long long)s * d.ncell + base;
+    double sum[kN];
+#pragma unroll
+    for (int q = 0; q < kN; ++q) sum[q] = 0.0;
+    int r = lane % nr;  // I - 1 of cell c
+#pragma unroll 4
+    for (int c = lane; c < (kN == 1 ? ncount : ncells); c += 32) {
+      const bool in = r != 0 && (kN == 1 || c < ncount);
+      double v = f[c];
+      if (kN == 1) {
+        sum[0] += in ? v : 0.0;
+      } else {
+        const double x = ch[c], y = at[c];
+        v *= x;
+        sum[0] += in ? v : 0.0;
+        v *= y;
+        sum[1 % kN] += in ? v : 0.0;
+        v *= y;
+        sum[2 % kN] += in ? v : 0.0;
+        v *= x;
+        sum[3 % kN] += in ? v : 0.0;
+        f[c] = v;
+      }
+      r += dr;
+      if (r >= nr) r -= nr;
     }
+    const double w = d.ekev[k] * d.we[k] * d.wmu[l];
+#pragma unroll
+    for (int q = 0; q < kN; ++q) acc[q] += w * sum[q];
   }
-  sh[threadIdx.x] = acc;
+#pragma unroll
+  for (int q = 0; q < kN; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if (lane == 0) sh[warp][q] = acc[q];
+  }
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
+  double* mine = part + (long long)slot * kBookBlocks * 4;
+  if (threadIdx.x < kN) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += sh[w][threadIdx.x];
+    mine[blockIdx.x * 4 + threadIdx.x] = t;
   }
-  if (threadIdx.x == 0) part[(long long)blockIdx.y * nblk + blockIdx.x] = sh[0];
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) lastblk = atomicAdd(&done[slot], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!lastblk) return;
+  __threadfence();
+  if (warp < kN) {  // warp q sums the blocks of channel q
+    double t = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(&mine[b * 4 + warp]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) sh[0][warp] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // {SETRC, LSDR, LSCHA, LSATM, valid, LSWAE}: ELORC = ENOLD - SETRC
+    double* L = losses + (long long)slot * 6;
+    for (int q = 0; q < kN; ++q) {
+      const int ch = kN == 1 ? which : (q == 0 || q == 3 ? 2 : 3);
+      if (ch >= 1 && L[4] != 0.0) L[ch] += L[0] - sh[0][q];
+      L[0] = sh[0][q];
+      L[4] = 1.0;
+    }
+    done[slot] = 0u;
+  }
 }
 
-void launch_sumrc(const Dev& d, double* part, int nblk, cudaStream_t st) {
-  k_sumrc<<<dim3(nblk, d.nitems), 256, 0, st>>>(d, part, nblk);
+// which: the channel of losses the change is booked to (1 LSDR, 5 LSWAE; -1
+// sets SETRC only); all_losses: the four loss processes and their channels.
+void launch_books(const Dev& d, bool all_losses, double* part, unsigned* done, double* losses, int which,
+                  cudaStream_t st) {
+  const dim3 g(kBookBlocks, d.nitems);
+  if (all_losses) k_books<4><<<g, 256, 0, st>>>(d, part, done, losses, 0);
+  else k_books<1><<<g, 256, 0, st>>>(d, part, done, losses, which);
 }
+size_t books_part_doubles(size_t nslot) { return nslot * kBookBlocks * 4; }
 
 // ------------------------------------------------------------------- FLUX
 __global__ void k_flux(Dev d, int slot, int s, double* out) {
