@@ -121,6 +121,18 @@ struct Unit {
   }
 };
 
+// p[i * st], i >= 0, as one multiply-add of 32-bit factors, where a 64-bit
+// index takes five instructions: the stride in cells (below 2^32: a line of
+// larger ones does not fit the memory) or, where it is below 2^29, in bytes.
+template <class T>
+__device__ __forceinline__ T& strided(T* p, int i, unsigned st) {
+  return *(T*)((uintptr_t)p + (uint64_t)((unsigned)i * (unsigned)sizeof(T)) * st);
+}
+template <class T>
+__device__ __forceinline__ T& strided_b(T* p, int i, unsigned bytes) {
+  return *(T*)((uintptr_t)p + (uint64_t)(unsigned)i * bytes);
+}
+
 // V consecutive doubles, 8*V-byte aligned.
 template <int V>
 struct Vec {
@@ -339,6 +351,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
       const int kl = line / (nr - 1);
       const int k = kl % ne, l = kl / ne;
       const long long st = nr;  // stride between consecutive J
+      const unsigned st8 = (unsigned)nr * 8u;
       double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + ((long long)kl * nt) * nr + i;
       unsigned char* __restrict__ rl =
           (kRec == 1 || kRec == 2) ? rec + u.it * d.ncell + ((long long)kl * nt) * nr + i : nullptr;
@@ -383,7 +396,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
         const double raw = (g0 - phi) + phi_prev;
         GJ(J) = (kRec == 2) ? clip_frozen(raw, rget(rj, rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
-        if (kRec == 1) rput(rl + ((long long)(J - 1) * st), rsh, cs | (is_neg(raw) ? kClipBit : 0));
+        if (kRec == 1) rput(rl + (long long)(J - 1) * st, rsh, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
         gm = g0; g0 = gp; gp = gpp;
       };
@@ -402,7 +415,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
       if (kRec == kRecCount) nclip += is_neg(rawN);
       GJ(nt) = vN;
       GJ(1) = vN;
-      if (kRec == 1) rput(rl + ((long long)(nt - 1) * st), rsh, csN | (is_neg(rawN) ? kClipBit : 0));
+      if (kRec == 1) rput(rl + (long long)(nt - 1) * st, rsh, csN | (is_neg(rawN) ? kClipBit : 0));
   #undef GJ
   #undef CJ
     }
@@ -450,12 +463,12 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
     const int i = 1 + lc % (nr - 1);
     const int jl = lc / (nr - 1);
     const int j = jl % nt, l = jl / nt;
-    const long long st = (long long)nt * nr;  // stride between consecutive K
+    const unsigned st = (unsigned)nt * nr;  // stride between consecutive K
     const long long off = ((long long)l * ne * nt + j) * nr + i;
     double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + off;
     unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + u.it * d.ncell + off : nullptr;
     const FaceBin* __restrict__ bins = d.ebin + s * ne;
-  #define GK(K) fl[(long long)((K)-1) * st]
+  #define GK(K) strided_b(fl, (K)-1, st * 8u)
     // the window G(b-1..b+2), the next cell, and the two cells past lim
     double w0 = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0, nxt = 0.0, hA = 0.0, hB = 0.0;
     if (active) {
@@ -503,7 +516,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
       };
       double phi_prev;
       {
-        unsigned char* rb = (kRec == 1 || kRec == 2) ? rl + (long long)(b - 1) * st : nullptr;
+        unsigned char* rb = (kRec == 1 || kRec == 2) ? rl + (uint64_t)(b - 1) * st : nullptr;
         int cs = kRec == 2 ? (int)(rget(rb, rsh) & 7) : 0;
         phi_prev = face(b, bins[b - 1], fma(bins[b - 1].k, wet, ue), w0, w1, w2, w3, cs, std::false_type());
         if (closed && r == 0) phi_prev = 0.0;
@@ -512,14 +525,14 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
       double gm = w1, g0 = w2, gp = w3;
       auto step = [&](int K, double v, double gpp, auto end) {
         const FaceBin bin = bins[K - 1];
-        const unsigned char* rk = (kRec == 1 || kRec == 2) ? rl + (long long)(K - 1) * st : nullptr;
+        const unsigned char* rk = (kRec == 1 || kRec == 2) ? rl + (uint64_t)(K - 1) * st : nullptr;
         int cs = kRec == 2 ? (int)(rget(rk, rsh) & 7) : 0;
         double phi = face(K, bin, v, gm, g0, gp, gpp, cs, end);
         if (decltype(end)::value && closed) phi = 0.0;
         const double raw = fma(phi_prev - phi, bin.iw, g0);
         GK(K) = (kRec == 2) ? clip_frozen(raw, rget(rk, rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
-        if (kRec == 1) rput(rl + ((long long)(K - 1) * st), rsh, cs | (is_neg(raw) ? kClipBit : 0));
+        if (kRec == 1) rput(rl + (uint64_t)(K - 1) * st, rsh, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
         gm = g0; g0 = gp; gp = gpp;
       };
@@ -586,13 +599,13 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
     const int i = 1 + lc % (nr - 1);
     const int jk = lc / (nr - 1);
     const int j = jk % nt;
-    const long long st = (long long)ne * nt * nr;  // stride between consecutive L
+    const unsigned st = (unsigned)ne * nt * nr;  // stride between consecutive L
     const long long off = (long long)jk * nr + i;  // (K*NT + J)*NR + I
     double* __restrict__ fl = d.f2 + (long long)slot * d.ncell + off;
     unsigned char* __restrict__ rl = (kRec == 1 || kRec == 2) ? rec + u.it * d.ncell + off : nullptr;
     const double* __restrict__ la = lossA ? lossA + (long long)s * d.ncell + off : nullptr;
-  #define GL(L) fl[(long long)((L)-1) * st]
-  #define LA(L) la[(long long)((L)-1) * st]
+  #define GL(L) strided(fl, (L)-1, st)
+  #define LA(L) strided(la, (L)-1, st)
   #define GLS(L) (kLoss == 2 ? GL(L) * LA(L) : GL(L))
     // the window G(b-1..b+2) (the first lane's F(1) is F(2)), the next cell,
     // and the two cells past lim
@@ -613,7 +626,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
     }
     if (kSplit > 1) __syncwarp();
     if (active) {
-      const long long sij = (long long)nt * nr;     // stride of (I,J,L) tables in L
+      const unsigned sij = (unsigned)nt * nr * 8u;  // bytes between consecutive L of (I,J,L) tables
       const long long fij = (long long)j * nr + i;
       const double* __restrict__ wm = d.wm + fij;
       const double* __restrict__ um = d.um + (long long)m * nt * nr * npa + fij;
@@ -623,7 +636,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
       const double beta = d.betalim;
       const uint64_t betaf = beta_fix(dbits(beta));
       const bool closed = d.flags & 1u;
-  #define CL(L) fma(ekv, wm[(long long)((L)-1) * sij], um[(long long)((L)-1) * sij])
+  #define CL(L) fma(ekv, strided_b(wm, (L)-1, sij), strided_b(um, (L)-1, sij))
       // face L's flux; the CFL quotient |C|/DMU is the Courant number
       Largest big;
       auto quotient = [&](int L, double c) { q = umax64(q, dbits(c * d.idmu[L - 1]) & kAbsMask); };
@@ -637,7 +650,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
       };
       double phi_prev = 0.0;
       if (kSplit > 1) {
-        int cs = kRec == 2 ? (int)(rget(rl + (long long)(b - 1) * st, rsh) & 7) : 0;
+        int cs = kRec == 2 ? (int)(rget(rl + (uint64_t)(b - 1) * st, rsh) & 7) : 0;
         const double phi = face(b, bins[b - 1], CL(b), w0, w1, w2, w3, cs);
         if (r) phi_prev = phi;
         else big = Largest();  // face 1 does not count
@@ -645,16 +658,16 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
       double gm = w1, g0 = w2, gp = w3;
       // cell L from its raw value, with its record
       auto put = [&](int L, double raw, int cs) {
-        if (kRec == 1) rput(rl + ((long long)(L - 1) * st), rsh, cs | (is_neg(raw) ? kClipBit : 0));
+        if (kRec == 1) rput(rl + (uint64_t)(L - 1) * st, rsh, cs | (is_neg(raw) ? kClipBit : 0));
         if (kRec == kRecCount) nclip += is_neg(raw);
-        return (kRec == 2) ? clip_frozen(raw, rget(rl + (long long)(L - 1) * st, rsh)) : clip(raw);
+        return (kRec == 2) ? clip_frozen(raw, rget(rl + (uint64_t)(L - 1) * st, rsh)) : clip(raw);
       };
       for (int L = b + 1; L <= (last ? npa - 2 : lim); ++L) {
         double nn = hA;
         if (L + 3 <= lim) nn = GLS(L + 3);
         else hA = hB;
         const FaceMu bin = bins[L - 1];
-        int cs = kRec == 2 ? (int)(rget(rl + (long long)(L - 1) * st, rsh) & 7) : 0;
+        int cs = kRec == 2 ? (int)(rget(rl + (uint64_t)(L - 1) * st, rsh) & 7) : 0;
         const double phi = face(L, bin, CL(L), gm, g0, gp, nxt, cs);
         double v = put(L, fma(phi_prev - phi, bin.iw, g0), cs);
         if (kLoss == 1) v *= LA(L);
