@@ -130,6 +130,7 @@ struct ramgpu_ctx {
   int pipe_chunks = -1;  // -1: per call (item groups for per-species arrays, 4 chunks for the reference layout)
   std::vector<cudaEvent_t> chunk_events;
   int step_groups = 4;  // ram_run's concurrent item groups (autotuned)
+  bool groups_set = false;  // by the caller or the autotuner
   cudaGraphExec_t pipe_exec = nullptr;
   std::vector<const void*> pipe_key;
   double pipe_dts = -1.0;
@@ -177,6 +178,11 @@ struct ramgpu_ctx {
   double* stat_part = nullptr;
   unsigned long long* stat_mm = nullptr;
   unsigned long long* status_h = nullptr;
+  // the moments in page-locked host memory, (2, nm*ns, NT, NR): the moment
+  // kernels store every PPERT and PPART there too (Dev::mom_host), so reading
+  // them takes no copy
+  double* mom_h = nullptr;
+  double dmu_last = 0.0;  // DMU(NPA)
   bool check_on = false;
   bool status_valid = false;
   // optional timeline of ramgpu_ram_run_host (diagnostics): start, then per
@@ -500,11 +506,19 @@ static int over_groups(ramgpu_ctx* ctx, int G, F&& fn) {
   return RAMGPU_OK;
 }
 
-// Item groups of a step: 1 in per-kernel timing passes (the events sit on
-// one stream), else the given count, at most one group per item.
+// Item groups: 1 in per-kernel timing passes (the events sit on one stream),
+// else the given count, at most one group per item.
 static int clamp_groups(const ramgpu_ctx* ctx, int groups) {
   if (ctx->timing) return 1;
   return std::max(1, std::min(groups, ctx->d.nitems));
+}
+// The step's item groups.  Until a count is set or tuned, 1 for small lists,
+// whose launches run in one wave (8x9x35x72, four species, ms a call with 1,
+// 2, 4 groups: 0.130, 0.132, 0.135 from the graph, 0.160, 0.163, 0.205
+// launched directly; 20x25x35x72: 0.458, 0.394, 0.385 from the graph).
+static int step_group_count(const ramgpu_ctx* ctx) {
+  if (!ctx->groups_set && ctx->d.ncell * ctx->d.nitems < 1500000) return 1;
+  return clamp_groups(ctx, ctx->step_groups);
 }
 
 // One ram_run step on the device-resident F2.  With more than one item
@@ -523,7 +537,7 @@ static int enqueue_status(ramgpu_ctx* ctx) {
 }
 
 static int enqueue_body(ramgpu_ctx* ctx, double dts) {
-  const int G = clamp_groups(ctx, ctx->step_groups);
+  const int G = step_group_count(ctx);
   int rc = RAMGPU_OK;
   if (G > 1) {
     if ((rc = ensure_group_streams(ctx, G))) return rc;
@@ -555,7 +569,7 @@ static int enqueue_call_rec(ramgpu_ctx* ctx, double dts, unsigned char* rec, boo
   launch_member_coef(ctx->d, dts, ctx->stream);
   launch_ghost(ctx->d, ctx->stream);
   ctx->launches += 3;
-  const int G = clamp_groups(ctx, ctx->step_groups);
+  const int G = step_group_count(ctx);
   if (int rc = ensure_group_streams(ctx, G)) return rc;
   return over_groups(ctx, G, [&](int i0) {
     const Dev& d = ctx->d;
@@ -585,7 +599,7 @@ static int enqueue_call_replay(ramgpu_ctx* ctx, double dts, unsigned char* rec) 
   launch_member_coef(ctx->d, dts, ctx->stream);
   launch_ghost(ctx->d, ctx->stream);
   ctx->launches += 3;
-  const int G = clamp_groups(ctx, ctx->step_groups);
+  const int G = step_group_count(ctx);
   if (int rc = ensure_group_streams(ctx, G)) return rc;
   return over_groups(ctx, G, [&](int i0) {
     const Dev& d = ctx->d;
@@ -1081,6 +1095,13 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
     ctx->status_h = nullptr;
     ok = false;
   }
+  const size_t nmom = 2 * nslot * nr * nt;
+  if (ok && (cudaHostAlloc(&ctx->mom_h, nmom * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
+             cudaHostGetDevicePointer(&d.mom_host, ctx->mom_h, 0) != cudaSuccess)) {
+    cudaGetLastError();
+    ok = false;
+  }
+  if (ok) memset(ctx->mom_h, 0, nmom * sizeof(double));
   if (!ok) {
     ramgpu_destroy(ctx);
     return fail(nullptr, RAMGPU_ERR_NOMEM, "device allocation failed");
@@ -1127,6 +1148,7 @@ int ramgpu_destroy(ramgpu_ctx* ctx) {
   cudaFree(ctx->adj_ring);
   for (cudaEvent_t e : ctx->adj_ring_events) cudaEventDestroy(e);
   if (ctx->status_h) cudaFreeHost(ctx->status_h);
+  if (ctx->mom_h) cudaFreeHost(ctx->mom_h);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return RAMGPU_OK;
@@ -1185,6 +1207,7 @@ int ramgpu_set_grid(ramgpu_ctx* ctx, const ramgpu_grid* g) {
     CK(up(d.sinphi, sp.data(), nt));
   }
   CK(up(d.ekev, G.ekev, ne)); CK(up(d.ebnd, G.ebnd, ne)); CK(up(d.we, G.we, ne)); CK(up(d.de, G.de, ne));
+  ctx->dmu_last = G.dmu[npa - 1];
   CK(up(d.mu, G.mu, npa)); CK(up(d.dmu, G.dmu, npa)); CK(up(d.wmu, G.wmu, npa));
   CK(up(d.rmas, G.rmas, ns));
   std::vector<int> ua(nr), um(nr);
@@ -1321,9 +1344,10 @@ int ramgpu_set_potential(ramgpu_ctx* ctx, int member, const double* vt) {
   if (check_ctx(ctx) || !vt) return fail(ctx, RAMGPU_ERR_ARG, "null argument");
   if (int rc = check_ms(ctx, member, 0)) return rc;
   const size_t n = (size_t)ctx->d.nf * ctx->d.nt;
-  CK(cudaMemcpy(ctx->d.vt + (size_t)member * n, vt, n * sizeof(double), cudaMemcpyHostToDevice));
-  int zero = 0;
-  CK(cudaMemcpy(ctx->d.vt_mode + member, &zero, sizeof(int), cudaMemcpyHostToDevice));
+  // in stream order with the kernels that set Kp
+  CK(cudaMemcpyAsync(ctx->d.vt + (size_t)member * n, vt, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemsetAsync(ctx->d.vt_mode + member, 0, sizeof(int), ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
   return RAMGPU_OK;
 }
 
@@ -1332,6 +1356,14 @@ int ramgpu_set_potential(ramgpu_ctx* ctx, int member, const double* vt) {
 __global__ void k_set_kp(double* kp, int* vt_mode, int m0, int m1, double v) {
   const int m = m0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (m < m1) { kp[m] = v; vt_mode[m] = 1; }
+}
+
+constexpr int kKpArgs = 128;
+struct KpArgs {
+  double kp[kKpArgs];
+};
+__global__ void k_set_kp_list(double* kp, int* vt_mode, int n, KpArgs v) {
+  if ((int)threadIdx.x < n) { kp[threadIdx.x] = v.kp[threadIdx.x]; vt_mode[threadIdx.x] = 1; }
 }
 
 int ramgpu_set_kp(ramgpu_ctx* ctx, int member, double kp) {
@@ -1352,10 +1384,16 @@ int ramgpu_set_kp_all(ramgpu_ctx* ctx, const double* kp) {
   const int nm = ctx->cfg.n_members;
   for (int m = 0; m < nm; ++m)
     if (!isfinite(kp[m])) return fail(ctx, RAMGPU_ERR_ARG, "kp must be finite");
-  std::vector<int> one(nm, 1);
-  CK(cudaMemcpyAsync(ctx->d.kp, kp, sizeof(double) * nm, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->d.vt_mode, one.data(), sizeof(int) * nm, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  // the values travel as kernel arguments: no staging copy, no wait (11-15 us
+  // a call with two copies and a synchronisation, 3 with the launch)
+  for (int m0 = 0; m0 < nm; m0 += kKpArgs) {
+    KpArgs v;
+    const int n = std::min(kKpArgs, nm - m0);
+    memcpy(v.kp, kp + m0, sizeof(double) * n);
+    k_set_kp_list<<<1, kKpArgs, 0, ctx->stream>>>(ctx->d.kp + m0, ctx->d.vt_mode + m0, n, v);
+    ctx->launches += 1;
+  }
+  CKL("set_kp_all");
   return RAMGPU_OK;
 }
 
@@ -1555,8 +1593,9 @@ int ramgpu_pipeline_groups(const ramgpu_ctx* ctx) {
 int ramgpu_set_step_groups(ramgpu_ctx* ctx, int groups) {
   if (check_ctx(ctx)) return RAMGPU_ERR_ARG;
   if (groups < 1 || groups > 8) return fail(ctx, RAMGPU_ERR_ARG, "groups must be 1..8");
-  if (groups != ctx->step_groups) ctx->shape_version += 1;  // ram_run's graph holds the groups
+  if (groups != ctx->step_groups || !ctx->groups_set) ctx->shape_version += 1;  // ram_run's graph holds the groups
   ctx->step_groups = groups;
+  ctx->groups_set = true;
   return RAMGPU_OK;
 }
 
@@ -1885,7 +1924,7 @@ int ramgpu_ram_run_ref(ramgpu_ctx* ctx, double dts, double* const* f2, double* c
   }
   const bool timing = ctx->timing;
   ctx->timing = false;  // one call, one set of streams: no per-kernel events
-  const int G = clamp_groups(ctx, ctx->step_groups);
+  const int G = step_group_count(ctx);
   if ((rc = ensure_group_streams(ctx, G))) {
     ctx->timing = timing;
     return rc;
@@ -2087,9 +2126,10 @@ int ramgpu_moments(ramgpu_ctx* ctx, int member, int s, double* ppert, double* pp
   if (check_ctx(ctx) || !ppert || !ppart) return fail(ctx, RAMGPU_ERR_ARG, "null argument");
   if (int rc = check_ms(ctx, member, s)) return rc;
   const size_t n = (size_t)ctx->d.nr * ctx->d.nt, o = (size_t)(member * ctx->d.ns + s) * n;
+  const double* h = ctx->mom_h + o;  // the moment kernels write it too
   CK(cudaStreamSynchronize(ctx->stream));
-  CK(cudaMemcpy(ppert, ctx->d.ppert + o, n * sizeof(double), cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(ppart, ctx->d.ppart + o, n * sizeof(double), cudaMemcpyDeviceToHost));
+  memcpy(ppert, h, n * sizeof(double));
+  memcpy(ppart, h + (size_t)ctx->d.nm * ctx->d.ns * n, n * sizeof(double));
   return RAMGPU_OK;
 }
 
@@ -2141,8 +2181,7 @@ int ramgpu_cfl(ramgpu_ctx* ctx, int member, int s, double* out5) {
   const double fr = ctx->cfg.fraccfl * ctx->last_dts;
   const double init[4] = {100000.0, 100000.0, 10000.0, 10000.0};
   // smallest 1/DMU(NPA) floor term of DRIFTMU's L = NPA face (CDriftMu = 0 there)
-  double dmu_n = 0.0;
-  CK(cudaMemcpy(&dmu_n, ctx->d.dmu + ctx->d.npa - 1, sizeof(double), cudaMemcpyDeviceToHost));
+  const double dmu_n = ctx->dmu_last;
   double dtsnext = 1e300;
   for (int sp : ctx->member_species[member]) {
     for (int w = 0; w < 4; ++w) {
@@ -2433,6 +2472,7 @@ int ramgpu_autotune(ramgpu_ctx* ctx, double dts, int reps, double* best_ms4) {
   {
     float best = 1e30f;
     int bg = ctx->step_groups;
+    ctx->groups_set = true;
     for (int G = 1; G <= 8 && G <= ctx->d.nitems; G *= 2) {
       ctx->step_groups = G;
       float tbest = 1e30f;
@@ -2664,6 +2704,8 @@ int ramgpu_load_state(ramgpu_ctx* ctx, const char* path, double* time) {
     for (int q = 0; q < 4 && ok; ++q) {
       get(buf.data(), sizeof(double) * cnt[q]);
       if (ok) CK(cudaMemcpy(dst[q], buf.data(), sizeof(double) * cnt[q], cudaMemcpyHostToDevice));
+      if (ok && q >= 2)  // the moments' host copy
+        memcpy(ctx->mom_h + (size_t)((q - 2) * nm * ns + slot) * nm2, buf.data(), sizeof(double) * nm2);
     }
   }
   fclose(f);
@@ -3193,7 +3235,7 @@ int ramgpu_adj_backward(ramgpu_ctx* ctx, double* grad_f2, double* grad_fgeos) {
   if (rc) return rc;
   const size_t nslot = (size_t)d.nm * d.ns, nfg = (size_t)d.nt * d.ne * d.npa;
   const size_t isz = (size_t)d.nitems * d.ncell;
-  const int G = clamp_groups(ctx, ctx->step_groups);
+  const int G = step_group_count(ctx);
   if ((rc = ensure_group_streams(ctx, G))) return rc;
   // the first DRIFTE transpose of each call keeps its face coefficients in
   // the DRIFTE coefficient store for the second

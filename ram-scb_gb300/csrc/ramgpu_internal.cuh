@@ -112,6 +112,7 @@ struct Dev {
   int count_clips;            // the sweeps count clip events (status pass on)
   double *mom_part;       // (nm*ns, NT, NR, (NE-1)*4 chunks, 2) moment partials
   double *ppert, *ppart;  // (nm*ns, NR, NT)
+  double *mom_host;       // the same in mapped host memory: (2, nm*ns, NR, NT)
   // face coefficients C of a call's first DRIFTE transpose, read back by the
   // second: (coef_items, ncell); null when not allocated
   double* coef;

@@ -669,6 +669,8 @@ __global__ void __launch_bounds__(128) k_moments_reduce(Dev d) {
     const long long o = (long long)slot * d.nr * d.nt + (long long)j * d.nr + i;
     d.ppert[o] = e;
     d.ppart[o] = a;
+    d.mom_host[o] = e;
+    d.mom_host[(long long)d.nm * d.ns * d.nr * d.nt + o] = a;
   }
 }
 
