@@ -185,11 +185,7 @@ __device__ __forceinline__ double masked(const double* __restrict__ lam, const u
   return ((__ldg(rl + off) >> rsh) & kClipBit) ? 0.0 : v;
 }
 
-#define WORK_LOOP(NLINES)                                                          \
-  const int bpi = (NLINES + blockDim.x - 1) / blockDim.x;                          \
-  const long long nunits = (long long)bpi * d.nitems;                              \
-  for (long long u = blockIdx.x + (long long)blockIdx.y * gridDim.x; u < nunits;   \
-       u += (long long)gridDim.x * gridDim.y)
+#define WORK_LOOP(NLINES) for (Unit u((NLINES + blockDim.x - 1) / blockDim.x); u.ok(d); u.next(d))
 
 // The loops below are peeled so that no floating-point operation in the
 // main loop depends on the position along the line (the FP64 pipe is the
@@ -223,13 +219,10 @@ __global__ void __launch_bounds__(128) k_adj_r(Dev d, const unsigned char* __res
   const int ts = nr | 1;
   unsigned char* rtile = (unsigned char*)(tile + (size_t)blockDim.x * ts);
   const int nlines = nt * ne * d.npa;
-  const int bpi = (nlines + blockDim.x - 1) / blockDim.x;
-  const long long nunits = (long long)bpi * d.nitems;
-  for (long long u = blockIdx.x + (long long)blockIdx.y * gridDim.x; u < nunits;
-       u += (long long)gridDim.x * gridDim.y) {  // uniform across the CTA
-    const int2 item = d.items[u / bpi];
+  for (Unit u((nlines + blockDim.x - 1) / blockDim.x); u.ok(d); u.next(d)) {  // uniform across the CTA
+    const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
-    const int lfirst = (int)(u % bpi) * blockDim.x;
+    const int lfirst = u.b * blockDim.x;
     const int nl = min((int)blockDim.x, nlines - lfirst);
     // bounds-checked builds: the tile's cells (the whole CTA skips it)
     if (kBoundsChecked) {
@@ -238,7 +231,7 @@ __global__ void __launch_bounds__(128) k_adj_r(Dev d, const unsigned char* __res
       if (!ok) continue;
     }
     double* __restrict__ gl = d.lam + (long long)slot * d.ncell + (long long)lfirst * nr;
-    const unsigned char* __restrict__ gr = rec + (u / bpi) * d.ncell + (long long)lfirst * nr;
+    const unsigned char* __restrict__ gr = rec + u.it * d.ncell + (long long)lfirst * nr;
     for (int e = threadIdx.x; e < nl * nr; e += blockDim.x) {
       const int ln = e / nr;
       tile[ln * ts + (e - ln * nr)] = gl[e];
@@ -337,9 +330,9 @@ __global__ void __launch_bounds__(128) k_adj_p(Dev d, const unsigned char* __res
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   const int nlines = (nr - 1) * ne * d.npa;
   WORK_LOOP(nlines) {
-    const int2 item = d.items[u / bpi];
+    const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
-    const int line = (int)(u % bpi) * blockDim.x + threadIdx.x;
+    const int line = u.b * blockDim.x + threadIdx.x;
     if (line >= nlines) continue;
     const int i = 1 + line % (nr - 1);
     const int kl = line / (nr - 1);
@@ -353,7 +346,7 @@ __global__ void __launch_bounds__(128) k_adj_p(Dev d, const unsigned char* __res
                kRgAdjP, line))
       continue;
     double* __restrict__ lam = d.lam + (long long)slot * d.ncell + base;
-    const unsigned char* __restrict__ rl = rec + (u / bpi) * d.ncell + base;
+    const unsigned char* __restrict__ rl = rec + u.it * d.ncell + base;
     const double* __restrict__ gpt = d.gpt + ((long long)l * nt) * nr + i;
     const double* __restrict__ ca = d.ca + ((long long)m * nt) * nr + i;
     const double p2 = d.p2[((long long)s * ne + k) * nr + i];
@@ -434,9 +427,9 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   const int nlines = (nr - 1) * nt * d.npa;
   WORK_LOOP(nlines) {
-    const int2 item = d.items[u / bpi];
+    const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
-    const int line = (int)(u % bpi) * blockDim.x + threadIdx.x;
+    const int line = u.b * blockDim.x + threadIdx.x;
     if (line >= nlines) continue;
     const int i = 1 + line % (nr - 1);
     const int jl = line / (nr - 1);
@@ -449,12 +442,12 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
                       rg_span((long long)m * nr * nt * d.npa + ((long long)l * nt + j) * nr + i, 1, 1,
                               (long long)d.nm * nr * nt * d.npa) &&
                       rg_span((long long)s * ne * nr + i, ne, nr, (long long)d.ns * ne * nr) &&
-                      (!kCo || d.item0 + u / bpi < d.coef_items),
+                      (!kCo || d.item0 + u.it < d.coef_items),
                kRgAdjE, line))
       continue;
     double* __restrict__ lam = d.lam + (long long)slot * d.ncell + base;
-    const unsigned char* __restrict__ rl = rec + (u / bpi) * d.ncell + base;
-    double* __restrict__ cst = kCo ? coef_ptr(d, u / bpi) + base : nullptr;
+    const unsigned char* __restrict__ rl = rec + u.it * d.ncell + base;
+    double* __restrict__ cst = kCo ? coef_ptr(d, u.it) + base : nullptr;
     const long long fij = ((long long)l * nt + j) * nr + i;
     const double wet = d.wet[fij];
     const double ue = d.ue[(long long)m * nr * nt * d.npa + fij];
@@ -520,30 +513,40 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
 // loss (may be null): the CEX/ATMOL factor table the forward sweep applied
 // to its result (cells L >= 2 of its lines; the table is 1 elsewhere), so
 // lambda is scaled by it as it is read, the transposed loss fused in.
-template <bool kLoss, int rsh>
+// kSplit adjacent lanes share a line (few lines, long serial chains, as in the
+// forward sweep): lane r writes the cells b+1..lim of its segment (b = r*S,
+// lim = (r+1)*S, S = NPA/kSplit; the first from cell 2, the last to NPA).
+// Cell i collects from faces i-2..i+1, so a lane runs the faces b-1..lim+1,
+// three more than its cells.  Every old value a lane needs from its
+// neighbours' cells is loaded before a __syncwarp, no lane writes before it.
+template <bool kLoss, int rsh, int kSplit>
 __global__ void __launch_bounds__(128) k_adj_mu(Dev d, const unsigned char* __restrict__ rec,
                                                 const double* __restrict__ loss) {
   const int nr = d.nr, nt = d.nt, ne = d.ne, npa = d.npa;
   const int nlines = (nr - 1) * nt * ne;
-  WORK_LOOP(nlines) {
-    const int2 item = d.items[u / bpi];
+  const int lpb = blockDim.x / kSplit;
+  const int r = kSplit > 1 ? (int)threadIdx.x % kSplit : 0, seg = npa / kSplit;
+  const bool last = r == kSplit - 1;
+  for (Unit u((nlines + lpb - 1) / lpb); u.ok(d); u.next(d)) {
+    const int2 item = d.items[u.it];
     const int m = item.x, s = item.y, slot = m * d.ns + s;
-    const int line = (int)(u % bpi) * blockDim.x + threadIdx.x;
-    if (line >= nlines) continue;
-    const int i = 1 + line % (nr - 1);
-    const int jk = line / (nr - 1);
+    const int line = u.b * lpb + (int)threadIdx.x / kSplit;
+    const int lc = line < nlines ? line : 0;
+    const int i = 1 + lc % (nr - 1);
+    const int jk = lc / (nr - 1);
     const int j = jk % nt;
     const long long st = (long long)ne * nt * nr;
     const long long off = (long long)jk * nr + i;
-    // bounds-checked builds: the line's cells, its WM and UM columns
-    if (!rg_ok(d, rg_item(d, item) && rg_span(off, npa, st, d.ncell) &&
+    // bounds-checked builds: the line's cells, its WM and UM columns (the
+    // lanes sharing a line test the same)
+    const bool active = line < nlines &&
+        rg_ok(d, rg_item(d, item) && rg_span(off, npa, st, d.ncell) &&
                       rg_span((long long)j * nr + i, npa, (long long)nt * nr, (long long)nr * nt * npa) &&
                       rg_span((long long)m * nt * nr * npa + (long long)j * nr + i, npa, (long long)nt * nr,
                               (long long)d.nm * nr * nt * npa),
-               kRgAdjMu, line))
-      continue;
+               kRgAdjMu, line);
     double* __restrict__ lam = d.lam + (long long)slot * d.ncell + off;
-    const unsigned char* __restrict__ rl = rec + (u / bpi) * d.ncell + off;
+    const unsigned char* __restrict__ rl = rec + u.it * d.ncell + off;
     const long long sij = (long long)nt * nr;
     const long long fij = (long long)j * nr + i;
     const double* __restrict__ wm = d.wm + fij;
@@ -553,6 +556,7 @@ __global__ void __launch_bounds__(128) k_adj_mu(Dev d, const unsigned char* __re
     const BetaBits beta(d.betalim);
     const bool closed = d.flags & 1u;
     const int n = npa;
+    const double* __restrict__ iwmu = d.iwmu;
 #define MC(L) fma(ekv, wm[(long long)((L)-1) * sij], um[(long long)((L)-1) * sij])
     const double* __restrict__ ls = kLoss ? loss + (long long)s * d.ncell + off : nullptr;
     auto lv = [&](int L) {  // lambda of cell L (>= 2), scaled by the loss factor
@@ -563,58 +567,73 @@ __global__ void __launch_bounds__(128) k_adj_mu(Dev d, const unsigned char* __re
       const double v = lv(L);
       return ((__ldg(rl + (long long)(L - 1) * st) >> rsh) & kClipBit) ? 0.0 : v;
     };
-#define MLE(L) mle(L)
-    const double out1 = lam[0];
-    // le(NPA-1) takes rho * lambda(NPA) (F2(NPA) = F2new(NPA-1)*rho)
-    const double leNm = ((rl[(long long)(n - 2) * st] >> rsh) & kClipBit) ? 0.0 : fma(d.rho[fij], lv(n), lv(n - 1));
-    const double le2 = MLE(2), le3 = MLE(3), le4 = MLE(4);
-    double wl0 = le2 * d.iwmu[1], wl1 = le3 * d.iwmu[2], wl2 = le4 * d.iwmu[3];
-    double cm1 = 0.0, c0 = le2, c1 = le3, c2 = le4;
-    auto face = [&](int L) {
-      const double C = MC(L);
-      const bool neg = is_neg(C);
-      const int cs = (rl[(long long)(L - 1) * st] >> rsh) & 7;
-      if (kAdjIntMask & 8u)
-        face_acc_a(adj_mul(8u, C, wl1 - wl0), neg, cs, corr_a_fix(courant_u(C, d.idmu[L - 1]), neg), beta, cm1, c0, c1,
-                   c2);
-      else
-        face_acc(adj_mul(8u, C, wl1 - wl0), neg, cs, face_ak<true>(C, neg, cs, d.mhdmu[L - 1], d.bmhdmu[L - 1], hb),
-                 cm1, c0, c1, c2);
-    };
-    auto shift = [&](double lec, double wl) {
-      cm1 = c0; c0 = c1; c1 = c2; c2 = lec;
-      wl0 = wl1; wl1 = wl2; wl2 = wl;
-    };
-    face(2);
-    const double gb1 = cm1;  // cell 1 -> cell 2 (G(1) = F(2))
-    { const double lec = MLE(5); shift(lec, lec * d.iwmu[4]); }
-    face(3);
-    lam[st] = cm1 + gb1;
-    { const double lec = MLE(6); shift(lec, lec * d.iwmu[5]); }
-    int L = 4;
-    for (; L <= n - 5; ++L) {
-      face(L);
-      lam[(long long)(L - 2) * st] = cm1;
-      const double lec = MLE(L + 3);
-      shift(lec, lec * d.iwmu[L + 2]);
+    // the lane's cells b+1..lim, its faces f0..fe; loads end at cell le1, the
+    // two cells after it are eA, eB: the next lane's first ones, or for the
+    // last lane NPA-1, which takes rho * lambda(NPA) (F2(NPA) = F2new(NPA-1)*rho),
+    // and NPA, which has no term of its own
+    const int b = r ? r * seg : 1, lim = last ? n : (r + 1) * seg;
+    const int f0 = r ? b - 1 : 2, fe = last ? n - 2 : lim + 1, le1 = last ? n - 2 : lim;
+    double eA = 0.0, eB = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0;
+    if (active) {
+      if (last) {
+        eA = ((rl[(long long)(n - 2) * st] >> rsh) & kClipBit) ? 0.0 : fma(d.rho[fij], lv(n), lv(n - 1));
+      } else {
+        eA = mle(lim + 1);
+        eB = mle(lim + 2);
+      }
+      v0 = mle(f0);      // cells f0, f0+1, f0+2
+      v1 = mle(f0 + 1);
+      v2 = mle(f0 + 2);
     }
-    face(n - 4);  // cell NPA-1 enters
-    lam[(long long)(n - 6) * st] = cm1;
-    shift(leNm, leNm * d.iwmu[n - 2]);
-    for (L = n - 3; L <= n - 2; ++L) {
-      face(L);
-      lam[(long long)(L - 2) * st] = cm1;
-      shift(0.0, 0.0);
+    if (kSplit > 1) __syncwarp();
+    if (active) {
+      double wl0 = v0 * iwmu[f0 - 1], wl1 = v1 * iwmu[f0], wl2 = v2 * iwmu[f0 + 1];
+      // window: cells f-1..f+2 (a cell before b+1 is another lane's)
+      double cm1 = 0.0, c0 = r ? 0.0 : v0, c1 = r ? 0.0 : v1, c2 = v2;
+      double first = 0.0;  // cell 1 -> cell 2 (G(1) = F(2))
+      for (int f = f0; f <= fe; ++f) {
+        const double C = MC(f);
+        const bool neg = is_neg(C);
+        const int cs = (rl[(long long)(f - 1) * st] >> rsh) & 7;
+        // the cell entering next
+        double lec = eA;
+        if (f + 3 <= le1) {
+          lec = mle(f + 3);
+        } else {
+          eA = eB;
+          eB = 0.0;
+        }
+        if (kAdjIntMask & 8u)
+          face_acc_a(adj_mul(8u, C, wl1 - wl0), neg, cs, corr_a_fix(courant_u(C, d.idmu[f - 1]), neg), beta, cm1, c0,
+                     c1, c2);
+        else
+          face_acc(adj_mul(8u, C, wl1 - wl0), neg, cs, face_ak<true>(C, neg, cs, d.mhdmu[f - 1], d.bmhdmu[f - 1], hb),
+                   cm1, c0, c1, c2);
+        if (r == 0 && f == 2) first = cm1;
+        if (f - 1 > b) lam[(long long)(f - 2) * st] = (r == 0 && f == 3) ? cm1 + first : cm1;
+        cm1 = c0; c0 = c1; c1 = c2; c2 = lec;
+        wl0 = wl1; wl1 = wl2; wl2 = lec * iwmu[min(f + 3, n) - 1];
+      }
+      if (last) {
+        // window: cells NPA-2, NPA-1, NPA; FBND(NPA-1) = F(NPA): Pb(NPA-1) = -le(NPA-1)/WMU
+        if (!closed) c1 -= MC(n - 1) * wl0;
+        lam[(long long)(n - 3) * st] = cm1;
+        lam[(long long)(n - 2) * st] = c0;
+        lam[(long long)(n - 1) * st] = c1;
+      }
     }
-    // window: cells NPA-2, NPA-1, NPA; FBND(NPA-1) = F(NPA): Pb(NPA-1) = -le(NPA-1)/WMU
-    if (!closed) c1 -= MC(n - 1) * wl0;
-    lam[(long long)(n - 3) * st] = cm1;
-    lam[(long long)(n - 2) * st] = c0;
-    lam[(long long)(n - 1) * st] = c1;
-    lam[0] = out1;
 #undef MC
-#undef MLE
   }
+}
+
+// Lanes per transposed pitch-angle line, by the number of lines.  Measured
+// backward ms a call (GB300, 20x25x35x72) with 1, 2, 4 lanes: one species
+// (3.4 warps an SM with one lane) 0.374, 0.315, 0.291; four (14) 0.608, 0.560,
+// 0.588; four members of four (55) 2.05, 2.10, 2.28.
+static int adj_mu_lanes(const Dev& d) {
+  const long long warps = (long long)(d.nr - 1) * d.nt * d.ne * d.nlist / 32;
+  if (d.npa < 24) return 1;  // segments of at least six cells
+  return warps < 8LL * d.nsm ? 4 : (warps < 24LL * d.nsm ? 2 : 1);
 }
 
 void launch_adj_sweep(const Dev& d, int w, const unsigned char* rec, int rsh, cudaStream_t st, int co,
@@ -639,10 +658,21 @@ void launch_adj_sweep(const Dev& d, int w, const unsigned char* rec, int rsh, cu
         else if (co == 2) k_adj_e<2, R><<<g, blk, 0, st>>>(d, rec);
         else k_adj_e<0, R><<<g, blk, 0, st>>>(d, rec);
         break;
-      default:
-        if (loss) k_adj_mu<true, R><<<g, blk, 0, st>>>(d, rec, loss);
-        else k_adj_mu<false, R><<<g, blk, 0, st>>>(d, rec, nullptr);
+      default: {
+        const int lanes = adj_mu_lanes(d);
+        const dim3 gm((nl * lanes + blk - 1) / blk, d.nitems, 1);
+        if (lanes == 4) {
+          if (loss) k_adj_mu<true, R, 4><<<gm, blk, 0, st>>>(d, rec, loss);
+          else k_adj_mu<false, R, 4><<<gm, blk, 0, st>>>(d, rec, nullptr);
+        } else if (lanes == 2) {
+          if (loss) k_adj_mu<true, R, 2><<<gm, blk, 0, st>>>(d, rec, loss);
+          else k_adj_mu<false, R, 2><<<gm, blk, 0, st>>>(d, rec, nullptr);
+        } else {
+          if (loss) k_adj_mu<true, R, 1><<<gm, blk, 0, st>>>(d, rec, loss);
+          else k_adj_mu<false, R, 1><<<gm, blk, 0, st>>>(d, rec, nullptr);
+        }
         break;
+      }
     }
   };
   if (rsh) go(std::integral_constant<int, 4>());

@@ -157,6 +157,24 @@ __device__ __forceinline__ bool rg_ok(const Dev& d, bool ok, int check, long lon
 #else
 __device__ __forceinline__ bool rg_ok(const Dev&, bool, int, long long) { return true; }
 #endif
+// Work units are (item, block of lines).  A plain grid of (blocks per item,
+// items) gives one unit per CTA; a persistent grid (one row) loops over them.
+struct Unit {
+  int it, b, bpi;
+  __device__ __forceinline__ Unit(int bpi_) : it(blockIdx.y), b(blockIdx.x), bpi(bpi_) {}
+  __device__ __forceinline__ bool ok(const Dev& d) {
+    while (b >= bpi) {
+      b -= bpi;
+      ++it;
+    }
+    return it < d.nitems;
+  }
+  __device__ __forceinline__ void next(const Dev& d) {
+    b += gridDim.x;
+    if (gridDim.y > 1) it = d.nitems;
+  }
+};
+
 // [first, first + (n - 1) * stride] inside [0, size)
 __device__ __forceinline__ bool rg_span(long long first, long long n, long long stride, long long size) {
   return first >= 0 && n >= 1 && first + (n - 1) * stride < size;

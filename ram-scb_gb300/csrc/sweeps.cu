@@ -103,24 +103,6 @@ struct Largest {
   }
 };
 
-// Work units are (item, block of lines).  A plain grid of (blocks per item,
-// items) gives one unit per CTA; a persistent grid (one row) loops over them.
-struct Unit {
-  int it, b, bpi;
-  __device__ __forceinline__ Unit(int bpi_) : it(blockIdx.y), b(blockIdx.x), bpi(bpi_) {}
-  __device__ __forceinline__ bool ok(const Dev& d) {
-    while (b >= bpi) {
-      b -= bpi;
-      ++it;
-    }
-    return it < d.nitems;
-  }
-  __device__ __forceinline__ void next(const Dev& d) {
-    b += gridDim.x;
-    if (gridDim.y > 1) it = d.nitems;
-  }
-};
-
 // p[i * st], i >= 0, as one multiply-add of 32-bit factors, where a 64-bit
 // index takes five instructions: the stride in cells (below 2^32: a line of
 // larger ones does not fit the memory) or, where it is below 2^29, in bytes.

@@ -233,3 +233,29 @@ def test_lane_counts_agree():
             first = got
         for a, b in zip(got, first):
             assert np.array_equal(a, b), members
+
+
+@pytest.mark.gpu
+def test_transposed_lane_counts_agree():
+    """The DRIFTMU transpose shares a line among 4, 2 or 1 lanes as members
+    join: member 0's misfit and dJ/dF2 are the same bits (a cell collects its
+    faces in the same order), dJ/dFGEOS to the rounding of its atomics."""
+    from ramgpu import abi, workload as W
+    wl = W.make_workload("tiny_pert")
+    g, ns = wl.grid, len(wl.grid.species)
+    obs = [{"member": 0, "s": s, "call": c, "k": 10 + 3 * s, "l": 1 + c, "lshell": 3.0 + 0.5 * s, "mlt": 6.0 * c,
+            "log_obs": 0.0} for s in range(ns) for c in range(2)]
+    first = None
+    for members in (1, 9, 24):
+        gpu = abi.RamGpu(g, wl.fields, n_members=members)
+        for m in range(members):
+            for s in range(ns):
+                gpu.upload_f2(m, s, np.asfortranarray(wl.f2[s]))
+                gpu.set_boundary(m, s, wl.fgeos[s])
+        j = gpu.adj_forward(2, wl.dts, np.full((2, members), 4.0), 1, obs)[0]
+        gf, gb = gpu.adj_backward()
+        gpu.close()
+        if first is None:
+            first = (j, gf[0], gb[0])
+        assert j == first[0] and np.array_equal(gf[0], first[1])
+        assert np.abs(gb[0] - first[2]).max() <= 1e-13 * np.abs(first[2]).max()
