@@ -456,7 +456,7 @@ static int enqueue_sweeps(ramgpu_ctx* ctx, double dts, bool clear_cfl) {
   { Timed t(ctx, 6); launch_finish(ctx->d, ctx->stream); }
   if (ctx->finish_hook) CK(cudaEventRecord(ctx->finish_hook, ctx->stream));
   { Timed t(ctx, 7); launch_moments(ctx->d, ctx->stream); }
-  ctx->launches += 3;
+  ctx->launches += 2;
   CKL("finish/moments");
   return RAMGPU_OK;
 }
@@ -586,7 +586,7 @@ static int enqueue_call_rec(ramgpu_ctx* ctx, double dts, unsigned char* rec, boo
     launch_finish(d, st);
     if (moments) launch_moments(d, st);
     else launch_anisch_state(d, st);
-    ctx->launches += moments ? 11 : 10;
+    ctx->launches += 10;
     CKL("recorded ram_run");
     return RAMGPU_OK;
   });
@@ -862,7 +862,7 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
     CK(cudaStreamWaitEvent(main, ev[3 * c + 2], 0));
   }
   { NvtxRange r("ANISCH"); launch_moments(full, main); }
-  ctx->launches += 2;
+  ctx->launches += 1;
   CKL("moments");
   if ((rc = tail(main))) return rc;
   if (ctx->check_on) rc = enqueue_status(ctx);
@@ -1080,7 +1080,8 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   d.cflq = dalloc<unsigned long long>(ctx, nslot * 5, &ok);
   d.clipq = d.cflq ? d.cflq + 4 * nslot : nullptr;
   d.count_clips = 0;
-  d.mom_part = dalloc<double>(ctx, nslot * 4 * nr * nt * ne * 2, &ok);
+  d.mom_part = dalloc<double>(ctx, mom_part_doubles(d), &ok);
+  d.mom_done = dalloc<unsigned>(ctx, mom_done_count(d), &ok);
   d.ppert = dalloc<double>(ctx, nslot * nr * nt, &ok);
   d.ppart = dalloc<double>(ctx, nslot * nr * nt, &ok);
   ctx->items_d = dalloc<int2>(ctx, nslot, &ok);
@@ -1211,11 +1212,15 @@ int ramgpu_set_grid(ramgpu_ctx* ctx, const ramgpu_grid* g) {
   CK(up(d.mu, G.mu, npa)); CK(up(d.dmu, G.dmu, npa)); CK(up(d.wmu, G.wmu, npa));
   CK(up(d.rmas, G.rmas, ns));
   std::vector<int> ua(nr), um(nr);
+  int lmax = 1;
   for (int i = 0; i < nr; ++i) {
     ua[i] = (int)G.upa[i];          // int(UPA(I)) in ATMOL
     um[i] = (int)(G.upa[i] - 1);    // int(UPA(I)-1) in ANISCH
     if (ua[i] < 2 || ua[i] > npa + 1) return fail(ctx, RAMGPU_ERR_ARG, "UPA out of range");
+    lmax = std::max(lmax, std::min(um[i], npa));
   }
+  if (lmax != d.mom_lmax) ctx->shape_version += 1;  // the moment kernel's grid
+  d.mom_lmax = lmax;
   CK(cudaMemcpy((void*)d.upa_atm, ua.data(), sizeof(int) * nr, cudaMemcpyHostToDevice));
   CK(cudaMemcpy((void*)d.upa_mom, um.data(), sizeof(int) * nr, cudaMemcpyHostToDevice));
   std::vector<double> r1(ne), r2(ne), r3(ne + 1), q1(npa), q2(npa), q3(npa + 1);
@@ -2112,7 +2117,7 @@ int ramgpu_apply_op(ramgpu_ctx* ctx, double dts, int op, int cfl) {
     case 3: launch_sweep_mu(ctx->d, dts, cfl != 0, 0, nullptr, ctx->stream); break;
     case 4: launch_loss_apply(ctx->d, ctx->d.charge, ctx->stream); break;
     case 5: launch_loss_apply(ctx->d, ctx->d.atm, ctx->stream); break;
-    case 6: launch_moments(ctx->d, ctx->stream); ctx->launches += 1; break;
+    case 6: launch_moments(ctx->d, ctx->stream); break;
     case 7: launch_padif(ctx->d, nullptr, ctx->stream); break;
     default: break;
   }

@@ -71,6 +71,8 @@ void launch_ghost(const Dev& d, cudaStream_t st);
 void launch_loss_apply(const Dev& d, const double* table, cudaStream_t st);
 void launch_finish(const Dev& d, cudaStream_t st);
 void launch_moments(const Dev& d, cudaStream_t st);
+size_t mom_part_doubles(const Dev& d);
+size_t mom_done_count(const Dev& d);
 void launch_anisch_state(const Dev& d, cudaStream_t st);
 void launch_books(const Dev& d, bool all_losses, double* part, unsigned* done, double* losses, int which,
                   cudaStream_t st);

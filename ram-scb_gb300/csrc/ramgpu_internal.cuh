@@ -66,7 +66,7 @@ struct Dev {
   double *mw_be, *mw_ba;  // (NPA, NT, NR): ANISCH weights WMU/FNHS*(1-MU^2), 2*WMU/FNHS*MU^2
   double *mws_a;          // (ns, NE, NR): RFAC*EPP(K)*MU(2)/FFACTOR(L=2), the separable species factor
   double *mws_be, *mws_ba;  // (NPA, NT, NR): mw_be, mw_ba over MU'(L) (MU'(1) = MU(2))
-  int mom_sep;            // FFACTOR has the separable ARRAYS form: two-fma moment sums
+  int mom_sep;            // FFACTOR has the separable ARRAYS form: two-index moment weights
   // DTs-dependent per-species small tables
   double *p4;             // (ns, NE)
   double *p2;             // (ns, NR, NE)
@@ -110,7 +110,9 @@ struct Dev {
   unsigned long long *cflq;  // (nm*ns, 4): max over cells of the CFL quotient, as bits
   unsigned long long *clipq;  // (nm*ns): clip events of the last call (follows cflq)
   int count_clips;            // the sweeps count clip events (status pass on)
-  double *mom_part;       // (nm*ns, NT, NR, (NE-1)*4 chunks, 2) moment partials
+  double *mom_part;       // moment partials, per slot, tile and L block
+  unsigned *mom_done;     // L blocks done, per slot and tile (0 between launches)
+  int mom_lmax;           // largest L of the moment sums
   double *ppert, *ppart;  // (nm*ns, NR, NT)
   double *mom_host;       // the same in mapped host memory: (2, nm*ns, NR, NT)
   // face coefficients C of a call's first DRIFTE transpose, read back by the

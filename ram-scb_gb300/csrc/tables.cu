@@ -183,7 +183,8 @@ __global__ void k_species_static(Dev d) {
 // species factor leaves the L-sum,
 //   mws_a(S,K,I)    = RFAC*EPP(S,K)*MU(2)/FFACTOR(S,I,K,2)
 //   mws_be(L,J,I)   = mw_be/MU'(L),  mws_ba = mw_ba/MU'(L),  MU'(1) = MU(2),
-// PPERT = sum over K of mws_a * sum over L of F2*mws_be: two fma per cell.
+// PPERT = sum over L of mws_be * sum over K of F2*mws_a, 72 times fewer
+// species weights to read.
 // k_mom_sep_check measures how far the given FFACTOR is from that form.
 // The reference sums the same products band by band (khi = 6,10,25,30,NE)
 // and scales each band by RFAC; the orders differ by rounding only.  All
@@ -591,95 +592,116 @@ void launch_finish(const Dev& d, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------- ANISCH moments
-// Stage 1: one thread per (I>=2, J, K>=2, L-chunk): the L=1 side effect
-// F2(S,I,J,K,1) = F2(S,I,J,K,2) (chunk 0; src/ModRamRun.f90:366) and the
-// chunk's share of both weighted pitch-angle sums, L = 1..int(UPA(I)-1)
-// split into kMomChunks equal runs.  Partials: (slot, J, I, Q) pairs of
-// doubles, Q = (K-2)*kMomChunks + chunk, so each (I,J) owns one contiguous
-// run for stage 2.
-constexpr int kMomChunks = 4;
-template <bool kSep>
-__global__ void __launch_bounds__(128) k_moments_part(Dev d) {
-  const int nr1 = d.nr - 1, ne1 = d.ne - 1;
-  const long long n = (long long)nr1 * d.nt * ne1 * kMomChunks;
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= n) return;
+// PPERT = sum over L of be(L,J,I) * sum over K of a(K,I)*F2, PPART with ba
+// (src/ModRamRun.f90:343-404; the weights above), L = 1..int(UPA(I)-1), K >= 2,
+// and the L = 1 side effect F2(S,I,J,K,1) = F2(S,I,J,K,2) (:366).  The energy
+// sum comes first, so a cell costs one FP64 fma whether FFACTOR is separable
+// (a of (K,I)) or not (a of (L,K,I)); the two pitch-angle weights meet the 34
+// times fewer energy sums.
+//
+// A thread takes one (I,J,L) and walks K; a block 32 consecutive (I,J) and 8
+// L.  The last of a tile's L blocks to finish adds their partials in order
+// and stores the tile's moments: one launch, no second pass.  Bound by FP64
+// issue and the F2 read.  One-stream launches with their events, two launches
+// and two fma a cell against this: four species on 20x25x35x72 35.5, 24.6 us;
+// on 40x49x70x144 304, 206 us.
+constexpr int kMomL = 8;
+__global__ void __launch_bounds__(32 * kMomL) k_moments(Dev d, int nlb, unsigned* __restrict__ done) {
+  __shared__ double2 sh[kMomL][32];
+  __shared__ bool lastblk;
+  const int nr1 = d.nr - 1, npair = nr1 * d.nt;
   const int2 item = d.items[blockIdx.y];
   const int s = item.y, slot = item.x * d.ns + s;
-  const int i = 1 + (int)(t % nr1);
-  const int j = (int)((t / nr1) % d.nt);
-  const int k = 1 + (int)((t / ((long long)nr1 * d.nt)) % ne1);
-  const int ch = (int)(t / ((long long)nr1 * d.nt * ne1));
-  const long long st = (long long)d.ne * d.nt * d.nr;
-  const long long off = ((long long)k * d.nt + j) * d.nr + i;
-  double* f = d.f2 + (long long)slot * d.ncell + off;
-  const long long sa = (long long)d.ne * d.nr, sb = (long long)d.nt * d.nr;  // L strides
-  const double* __restrict__ wa = d.mw_a + (long long)s * d.npa * sa + (long long)k * d.nr + i;
-  const double* __restrict__ be = (kSep ? d.mws_be : d.mw_be) + (long long)j * d.nr + i;
-  const double* __restrict__ ba = (kSep ? d.mws_ba : d.mw_ba) + (long long)j * d.nr + i;
-  const double f2 = f[st];
-  if (ch == 0) f[0] = f2;
-  const int u = d.upa_mom[i];
-  const int cl = (u + kMomChunks - 1) / kMomChunks;
-  const int l0 = 1 + ch * cl, l1 = min(u, (ch + 1) * cl);
-  double sume = 0.0, suma = 0.0;
-#pragma unroll 4
-  for (int L = l0; L <= l1; ++L) {
-    const double v = (L == 1) ? f2 : f[(long long)(L - 1) * st];
-    const double g = kSep ? v : v * wa[(long long)(L - 1) * sa];
-    sume = fma(g, be[(long long)(L - 1) * sb], sume);
-    suma = fma(g, ba[(long long)(L - 1) * sb], suma);
-  }
-  if (kSep) {  // the species factor of (S, I, K), once per partial
-    const double ws = d.mws_a[((long long)s * d.ne + k) * d.nr + i];
-    sume *= ws;
-    suma *= ws;
-  }
-  const int nq = ne1 * kMomChunks;
-  double2* part = reinterpret_cast<double2*>(d.mom_part) +
-                  (((long long)slot * d.nt + j) * d.nr + i) * nq + (k - 1) * kMomChunks + ch;
-  *part = make_double2(sume, suma);
-}
-
-// Stage 2: one warp per (I>=2, J): lanes sum strided runs of the (I,J)'s
-// partials, then an xor butterfly (every lane ends with the same sums).
-__global__ void __launch_bounds__(128) k_moments_reduce(Dev d) {
-  const int nr1 = d.nr - 1;
-  const int lane = threadIdx.x & 31;
-  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= nr1 * d.nt) return;  // uniform per warp
-  const int2 item = d.items[blockIdx.y];
-  const int slot = item.x * d.ns + item.y;
-  const int i = 1 + w % nr1, j = w / nr1;
-  const int nq = (d.ne - 1) * kMomChunks;
-  const double2* __restrict__ p =
-      reinterpret_cast<const double2*>(d.mom_part) + (((long long)slot * d.nt + j) * d.nr + i) * nq;
+  const int tile = (int)blockIdx.x / nlb, lb = (int)blockIdx.x % nlb;
+  const int pair = tile * 32 + threadIdx.x, L = 1 + lb * kMomL + threadIdx.y;  // L 1-based
+  const int ntile = (npair + 31) / 32;
   double e = 0.0, a = 0.0;
-  for (int q = lane; q < nq; q += 32) {
-    const double2 v = p[q];
-    e += v.x;
-    a += v.y;
-  }
+  if (pair < npair) {
+    const int i = 1 + pair % nr1, j = pair / nr1;
+    if (L <= d.upa_mom[i] || L == 1) {
+      const unsigned sk = (unsigned)d.nt * d.nr;  // K stride of F2
+      const long long sl = (long long)d.ne * sk;
+      double* f = d.f2 + (long long)slot * d.ncell + sk + (long long)j * d.nr + i;  // K = 2
+      const double* __restrict__ src = f + (L == 1 ? sl : (L - 1) * sl);
+      const double* __restrict__ wa = d.mom_sep ? d.mws_a + (long long)s * d.ne * d.nr + d.nr + i
+                                                : d.mw_a + ((long long)(s * d.npa + L - 1) * d.ne + 1) * d.nr + i;
+      const int nk = d.ne - 1;
+      double h[4] = {0.0, 0.0, 0.0, 0.0};  // four chains: an fma's result takes 64 cycles
+      for (int k = 0; k < nk; k += 8) {
+        double v[8];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    e += __shfl_xor_sync(0xffffffffu, e, o);
-    a += __shfl_xor_sync(0xffffffffu, a, o);
+        for (int q = 0; q < 8; ++q)
+          if (k + q < nk) v[q] = src[(uint64_t)(k + q) * sk];
+        if (L == 1) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (k + q < nk) f[(uint64_t)(k + q) * sk] = v[q];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (k + q < nk) h[q & 3] = fma(v[q], wa[(k + q) * d.nr], h[q & 3]);
+      }
+      const long long o = ((long long)(L - 1) * d.nt + j) * d.nr + i;
+      const double hk = (h[0] + h[1]) + (h[2] + h[3]);
+      e = hk * (d.mom_sep ? d.mws_be : d.mw_be)[o];
+      a = hk * (d.mom_sep ? d.mws_ba : d.mw_ba)[o];
+    }
   }
-  if (lane == 0) {
-    const long long o = (long long)slot * d.nr * d.nt + (long long)j * d.nr + i;
-    d.ppert[o] = e;
-    d.ppart[o] = a;
-    d.mom_host[o] = e;
-    d.mom_host[(long long)d.nm * d.ns * d.nr * d.nt + o] = a;
+  sh[threadIdx.y][threadIdx.x] = make_double2(e, a);
+  __syncthreads();
+  // both sums in pairs of pairs: the fewest roundings at full size
+  auto tree = [&](int x) {
+    double2 v[kMomL];
+#pragma unroll
+    for (int y = 0; y < kMomL; ++y) v[y] = sh[y][x];
+#pragma unroll
+    for (int n = kMomL / 2; n; n /= 2)
+#pragma unroll
+      for (int y = 0; y < n; ++y) {
+        v[y].x += v[y + n].x;
+        v[y].y += v[y + n].y;
+      }
+    return v[0];
+  };
+  double2* part = reinterpret_cast<double2*>(d.mom_part) + ((long long)slot * ntile + tile) * nlb * 32;
+  if (threadIdx.y == 0) {
+    part[lb * 32 + threadIdx.x] = tree(threadIdx.x);
+    __threadfence();
+    __syncwarp();
+    if (threadIdx.x == 0) {
+      unsigned* q = done + (long long)slot * ntile + tile;
+      lastblk = atomicAdd(q, 1u) == (unsigned)nlb - 1;
+      if (lastblk) *q = 0u;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (!lastblk) return;
+  e = a = 0.0;
+  for (int b = threadIdx.y; b < nlb; b += kMomL) {
+    e += __ldcg(&part[b * 32 + threadIdx.x].x);
+    a += __ldcg(&part[b * 32 + threadIdx.x].y);
+  }
+  sh[threadIdx.y][threadIdx.x] = make_double2(e, a);
+  __syncthreads();
+  if (threadIdx.y == 0 && pair < npair) {
+    const double2 t = tree(threadIdx.x);
+    const long long o = (long long)slot * d.nr * d.nt + (long long)(pair / nr1) * d.nr + 1 + pair % nr1;
+    d.ppert[o] = t.x;
+    d.ppart[o] = t.y;
+    d.mom_host[o] = t.x;
+    d.mom_host[(long long)d.nm * d.ns * d.nr * d.nt + o] = t.y;
   }
 }
 
+static int mom_lblocks(const Dev& d) { return (d.npa + kMomL - 1) / kMomL; }
+static int mom_tiles(const Dev& d) { return ((d.nr - 1) * d.nt + 31) / 32; }
+size_t mom_part_doubles(const Dev& d) { return (size_t)d.nm * d.ns * mom_tiles(d) * mom_lblocks(d) * 64; }
+size_t mom_done_count(const Dev& d) { return (size_t)d.nm * d.ns * mom_tiles(d); }
 void launch_moments(const Dev& d, cudaStream_t st) {
-  long long n = (long long)(d.nr - 1) * d.nt * (d.ne - 1) * kMomChunks;
-  if (d.mom_sep) k_moments_part<true><<<dim3((unsigned)((n + 127) / 128), d.nitems), 128, 0, st>>>(d);
-  else k_moments_part<false><<<dim3((unsigned)((n + 127) / 128), d.nitems), 128, 0, st>>>(d);
-  int n2 = (d.nr - 1) * d.nt;
-  k_moments_reduce<<<dim3((n2 + 3) / 4, d.nitems), 128, 0, st>>>(d);
+  // pitch angles past the largest UPA carry nothing
+  const int nlb = (d.mom_lmax + kMomL - 1) / kMomL;
+  k_moments<<<dim3((unsigned)(mom_tiles(d) * nlb), d.nitems), dim3(32, kMomL), 0, st>>>(d, nlb, d.mom_done);
 }
 
 // ANISCH's only effect on F2, F2(I,J,K,1) = F2(I,J,K,2) for I, K >= 2
