@@ -8,7 +8,7 @@
 //   R, P, E, MU (+ fused CEX/ATMOL)      4   (forward half, CFL tracked)
 //   MU, E, P, R                          4   (reverse half)
 //   periodic copy + magnetopause mask    1
-//   ANISCH moments                       2
+//   ANISCH moments                       1
 // mirroring the species loop of src/ModRamRun.f90:64-222; optionally the
 // status pass (1).  The whole call is one CUDA graph when graphs are on.
 //
@@ -386,10 +386,7 @@ static int sumrc_stage(ramgpu_ctx* ctx, int which) {
 }
 
 // Forward sweeps with the CFL reduction.
-static int enqueue_forward(ramgpu_ctx* ctx, double dts, bool loss_fused, const double* loss_table,
-                           bool clear_cfl = true) {
-  if (clear_cfl)
-    CK(cudaMemsetAsync(ctx->d.cflq, 0, sizeof(unsigned long long) * 5 * ctx->d.nm * ctx->d.ns, ctx->stream));
+static int enqueue_forward(ramgpu_ctx* ctx, double dts, bool loss_fused, const double* loss_table) {
   const Dev& d = ctx->d;
   { Timed t(ctx, 2); launch_sweep_r(d, dts, true, ctx->stream); }
   { Timed t(ctx, 3); launch_sweep_p(d, dts, true, ctx->stream); }
@@ -413,26 +410,26 @@ static int enqueue_reverse(ramgpu_ctx* ctx, double dts, bool loss_fused, const d
 }
 
 // The sweeps, losses and tail of one ram_run call for the work items of
-// ctx->d (the per-member tables and ghost planes are enqueued before);
-// clear_cfl: reset the CFL accumulators first.
-static int enqueue_sweeps(ramgpu_ctx* ctx, double dts, bool clear_cfl) {
+// ctx->d (the per-member tables, which reset the CFL accumulators, and the
+// ghost planes are enqueued before).
+static int enqueue_sweeps(ramgpu_ctx* ctx, double dts) {
   int rc = RAMGPU_OK;
   const bool losses = ctx->cfg.flags & RAMGPU_FLAG_LOSSES;
   const bool pd = ctx->pd_any();
   if (!losses && !pd) {
     // R,P,E,MU then CEX,ATMOL,ATMOL,CEX folded into the MU store
-    if ((rc = enqueue_forward(ctx, dts, true, ctx->d.loss2, clear_cfl))) return rc;
+    if ((rc = enqueue_forward(ctx, dts, true, ctx->d.loss2))) return rc;
     if ((rc = enqueue_reverse(ctx, dts, false, nullptr))) return rc;
   } else if (!losses) {
     // R,P,E,MU, WPADIF, CEX,ATMOL,ATMOL,CEX (folded into WPADIF's store), WPADIF, MU,E,P,R
-    if ((rc = enqueue_forward(ctx, dts, false, nullptr, clear_cfl))) return rc;
+    if ((rc = enqueue_forward(ctx, dts, false, nullptr))) return rc;
     { Timed t(ctx, 10); launch_padif(ctx->d, ctx->d.loss2, ctx->stream); }
     { Timed t(ctx, 10); launch_padif(ctx->d, nullptr, ctx->stream); }
     ctx->launches += 2;
     CKL("pitch-angle diffusion");
     if ((rc = enqueue_reverse(ctx, dts, false, nullptr))) return rc;
   } else {
-    if ((rc = enqueue_forward(ctx, dts, false, nullptr, clear_cfl))) return rc;
+    if ((rc = enqueue_forward(ctx, dts, false, nullptr))) return rc;
     if ((rc = sumrc_stage(ctx, 1))) return rc;
     if (pd) {
       { Timed t(ctx, 10); launch_padif(ctx->d, nullptr, ctx->stream); }
@@ -462,7 +459,7 @@ static int enqueue_sweeps(ramgpu_ctx* ctx, double dts, bool clear_cfl) {
 }
 
 static int enqueue_tables(ramgpu_ctx* ctx, double dts) {
-  { Timed t(ctx, 0); launch_member_coef(ctx->d, dts, ctx->stream); }
+  { Timed t(ctx, 0); launch_member_coef(ctx->d, dts, ctx->stream, true); }
   { Timed t(ctx, 1); launch_ghost(ctx->d, ctx->stream); }
   ctx->launches += 3;
   CKL("member tables");
@@ -544,7 +541,7 @@ static int enqueue_body(ramgpu_ctx* ctx, double dts) {
     rc = enqueue_pipeline(ctx, dts, nullptr, nullptr, nullptr, G, {});
   } else {
     if ((rc = enqueue_tables(ctx, dts))) return rc;
-    rc = enqueue_sweeps(ctx, dts, true);
+    rc = enqueue_sweeps(ctx, dts);
   }
   if (!rc && ctx->check_on) rc = enqueue_status(ctx);
   return rc;
@@ -818,7 +815,6 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
   int rc = RAMGPU_OK;
   CK(cudaEventRecord(ev_start, main));
   if ((rc = enqueue_tables(ctx, dts))) return rc;
-  CK(cudaMemsetAsync(full.cflq, 0, sizeof(unsigned long long) * 5 * full.nm * full.ns, main));
   CK(cudaEventRecord(ev_tab, main));
   for (int c = 0; c < C; ++c) {
     cudaStream_t st = ctx->pipe_streams[c];
@@ -919,7 +915,6 @@ static int enqueue_pipeline(ramgpu_ctx* ctx, double dts, double* const* f2, doub
   }
   // per-member tables and ghost planes of every item, CFL accumulators
   if (int rc = enqueue_tables(ctx, dts)) return rc;
-  CK(cudaMemsetAsync(full.cflq, 0, sizeof(unsigned long long) * 5 * full.nm * full.ns, main));
   CK(cudaEventRecord(ev_tab, main));
   for (int g = 0; g < G; ++g) {
     const int i0 = (int)((long long)nit * g / G), i1 = (int)((long long)nit * (g + 1) / G);
@@ -930,7 +925,7 @@ static int enqueue_pipeline(ramgpu_ctx* ctx, double dts, double* const* f2, doub
     ctx->d.nitems = i1 - i0;
     ctx->d.item0 = i0;
     ctx->finish_hook = f2 ? ctx->pipe_fin_events[g] : nullptr;
-    const int rc = enqueue_sweeps(ctx, dts, false);
+    const int rc = enqueue_sweeps(ctx, dts);
     ctx->finish_hook = nullptr;
     ctx->d = full;
     ctx->stream = main;
@@ -1841,7 +1836,6 @@ static int enqueue_ref(ramgpu_ctx* ctx, double dts, const std::vector<RefMem>& m
   for (int m = 0; m < nm; ++m)
     if (mem[m].f2 && (rc = ref_in(ctx, mem[m].f2, mem[m].f2r, full.f2 + (size_t)m * ns * n, n, n, main))) return rc;
   if ((rc = enqueue_tables(ctx, dts))) return rc;
-  CK(cudaMemsetAsync(full.cflq, 0, sizeof(unsigned long long) * 5 * full.nm * full.ns, main));
   cudaEvent_t ev_tab = ctx->pipe_events[2 * G + 1];
   CK(cudaEventRecord(ev_tab, main));
   for (int g = 0; g < G; ++g) {
@@ -1853,7 +1847,7 @@ static int enqueue_ref(ramgpu_ctx* ctx, double dts, const std::vector<RefMem>& m
     ctx->d.nitems = i1 - i0;
     ctx->d.item0 = i0;
     ctx->finish_hook = staged ? nullptr : ctx->pipe_fin_events[g];
-    rc = enqueue_sweeps(ctx, dts, false);
+    rc = enqueue_sweeps(ctx, dts);
     ctx->finish_hook = nullptr;
     ctx->d = full;
     ctx->stream = main;
@@ -2088,7 +2082,7 @@ int ramgpu_half_step(ramgpu_ctx* ctx, double dts, int order) {
   if (rc) return rc;
   ctx->last_dts = dts;
   if (ctx->d.nitems == 0) return RAMGPU_OK;
-  launch_member_coef(ctx->d, dts, ctx->stream);
+  launch_member_coef(ctx->d, dts, ctx->stream, order == 0);
   launch_ghost(ctx->d, ctx->stream);
   ctx->launches += 3;
   CKL("member tables");
@@ -2106,10 +2100,9 @@ int ramgpu_apply_op(ramgpu_ctx* ctx, double dts, int op, int cfl) {
   if (rc) return rc;
   ctx->last_dts = dts;
   if (ctx->d.nitems == 0) return RAMGPU_OK;
-  launch_member_coef(ctx->d, dts, ctx->stream);
+  launch_member_coef(ctx->d, dts, ctx->stream, cfl != 0);
   launch_ghost(ctx->d, ctx->stream);
   ctx->launches += 3;
-  if (cfl) CK(cudaMemsetAsync(ctx->d.cflq, 0, sizeof(unsigned long long) * 5 * ctx->d.nm * ctx->d.ns, ctx->stream));
   switch (op) {
     case 0: launch_sweep_r(ctx->d, dts, cfl != 0, ctx->stream); break;
     case 1: launch_sweep_p(ctx->d, dts, cfl != 0, ctx->stream); break;

@@ -66,7 +66,7 @@ int sweep_max_blocks_per_sm(int w, int blk);
 void launch_field_tables(const Dev& d, cudaStream_t st);
 void launch_species_static(const Dev& d, unsigned long long* sep_dev, cudaStream_t st);
 void launch_dts_tables(const Dev& d, double dts, cudaStream_t st);
-void launch_member_coef(const Dev& d, double dts, cudaStream_t st);
+void launch_member_coef(const Dev& d, double dts, cudaStream_t st, bool clear_cfl = false);
 void launch_ghost(const Dev& d, cudaStream_t st);
 void launch_loss_apply(const Dev& d, const double* table, cudaStream_t st);
 void launch_finish(const Dev& d, cudaStream_t st);
