@@ -1048,6 +1048,7 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   d.kap = dalloc<double>(ctx, ns * 2, &ok);
   d.ebin = dalloc<FaceBin>(ctx, ns * ne, &ok);
   d.er = dalloc<double>(ctx, nr, &ok); d.erq = dalloc<double>(ctx, ns * nr, &ok);
+  d.cexv = dalloc<double>(ctx, ns * ne, &ok);
   d.loss1 = dalloc<double>(ctx, ns * ncell, &ok); d.loss2 = dalloc<double>(ctx, ns * ncell, &ok);
   d.charge = dalloc<double>(ctx, ns * ncell, &ok); d.atm = dalloc<double>(ctx, ns * ncell, &ok);
   d.kp = dalloc<double>(ctx, nm, &ok); d.vt_mode = dalloc<int>(ctx, nm, &ok);

@@ -78,6 +78,7 @@ struct Dev {
   double *kap;            // (ns, 2): extrapolation factors of F(1), F(0) in DRIFTE
   double *wm;             // (NR,NT,NPA): -CMUDOT*HM, DTs-dependent, species-free
   double *cmudot;         // (NR,NT,NPA): MUDOT(I,L)*BOUNIS/BOUNHS, DTs-dependent
+  double *cexv;           // (ns, NE): charge exchange rate 10**Y*V of CEPARA
   double *loss1;          // (ns, ncell): CHARGE*ATLOS^(1/FNHS) (one half step)
   double *loss2;          // (ns, ncell): ((CHARGE*ATM)*ATM)*CHARGE (both halves)
   double *charge, *atm;   // (ns, ncell): separate factors for the bookkeeping path
