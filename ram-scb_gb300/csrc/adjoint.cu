@@ -422,6 +422,11 @@ __global__ void __launch_bounds__(128) k_adj_p(Dev d, const unsigned char* __res
 // transposes (of the reverse and the forward half) share C (same DTs and
 // potential), so the first keeps it for the second, as the forward sweeps
 // do; the stored value is the recomputed one, so the results do not change.
+// A warp's instructions issue in order: the cell entering the window was
+// masked, and so waited for, where it was loaded, an L2 round trip per face.
+// Loading a face ahead, backward ms a call with and without (one species,
+// four species on 20x25x35x72): 0.291 -> 0.277, 0.560 -> 0.546, with DRIFTMU^T
+// alike 0.270, 0.532.
 template <int kCo, int rsh>
 __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __restrict__ rec) {
   const int nr = d.nr, nt = d.nt, ne = d.ne;
@@ -457,18 +462,36 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
     const BetaBits beta(d.betalim);
     const bool closed = d.flags & 1u;
     const int n = ne;
-#define EC(K) adj_mul(4u, edot[(long long)((K)-1) * nr], fma(eb[(K)-1], wet, ue))
-#define ELE(K) masked(lam, rl, (long long)((K)-1) * st, rsh)
     const double out1 = lam[0];
+    // what face K needs is loaded while face K-1 is worked on: its EDOT (or
+    // the stored coefficient), the lambda and the record byte of the cell
+    // entering, K+3; the record bytes of faces K..K+2 wait in recs
+    auto rb = [&](int c) { return (unsigned)__ldg(rl + (long long)(c - 1) * st); };
+    unsigned recs = rb(1) | rb(2) << 8 | rb(3) << 16;
     // wl(K) = le(K)/WE(K) for K = 2..NE, 0 elsewhere; window = cells K-1..K+2
-    const double le2 = ELE(2), le3 = ELE(3);
+    const double le2 = masked(lam, rl, st, rsh), le3 = masked(lam, rl, 2 * st, rsh);
+    double nc, nlam;
+    unsigned nrec;
+    auto ahead = [&](int K) {
+      const long long o = (long long)(min(K, n) - 1) * st;
+      nc = (kCo == 2) ? cst[o] : edot[(long long)(min(K, n) - 1) * nr];
+      const int c = min(K + 3, n);
+      nlam = lam[(long long)(c - 1) * st];
+      nrec = rb(c);
+    };
+    ahead(1);
     double wl0 = 0.0, wl1 = le2 * d.iwe[1], wl2 = le3 * d.iwe[2];
     double cm1 = 0.0, c0 = 0.0, c1 = le2, c2 = le3;
+    double vin;  // the masked lambda of cell K+3 as face(K) leaves it
     auto face = [&](int K) {
-      const double C = (kCo == 2) ? cst[(long long)(K - 1) * st] : EC(K);
+      const double C = (kCo == 2) ? nc : adj_mul(4u, nc, fma(eb[K - 1], wet, ue));
       if (kCo == 1) cst[(long long)(K - 1) * st] = C;
+      recs |= nrec << 24;
+      vin = ((nrec >> rsh) & kClipBit) ? 0.0 : nlam;
+      ahead(K + 1);
       const bool neg = is_neg(C);
-      const int cs = (rl[(long long)(K - 1) * st] >> rsh) & 7;
+      const int cs = (recs >> rsh) & 7;
+      recs >>= 8;
       face_acc(adj_mul(kCo == 2 ? 0u : 4u, C, wl1 - wl0), neg, cs,
                face_ak<true>(C, neg, cs, d.mhde[K - 1], d.bmhde[K - 1], hb), cm1, c0, c1, c2);
     };
@@ -476,20 +499,26 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
       cm1 = c0; c0 = c1; c1 = c2; c2 = lec;
       wl0 = wl1; wl1 = wl2; wl2 = wl;
     };
-    if (!closed) face(1);
+    if (!closed) {
+      face(1);
+    } else {
+      recs = recs >> 8 | nrec << 16;
+      vin = ((nrec >> rsh) & kClipBit) ? 0.0 : nlam;
+      ahead(2);
+    }
     const double g0 = cm1;  // cell 0
-    { const double lec = ELE(4); shift(lec, lec * d.iwe[3]); }
+    { const double lec = vin; shift(lec, lec * d.iwe[3]); }
     face(2);
     const double g1 = fma(d.kap[2 * s + 0], g0, cm1);  // cell 1 (+ kap0 * cell 0)
-    { const double lec = ELE(5); shift(lec, lec * d.iwe[4]); }
+    { const double lec = vin; shift(lec, lec * d.iwe[4]); }
     face(3);
     lam[st] = fma(d.kap[2 * s + 1], g1, cm1);  // cell 2 (+ kap1 * cell 1)
-    { const double lec = ELE(6); shift(lec, lec * d.iwe[5]); }
+    { const double lec = vin; shift(lec, lec * d.iwe[5]); }
     int K = 4;
     for (; K <= n - 3; ++K) {
       face(K);
       lam[(long long)(K - 2) * st] = cm1;
-      const double lec = ELE(K + 3);
+      const double lec = vin;
       shift(lec, lec * d.iwe[K + 2]);
     }
     for (; K <= n - 1; ++K) {
@@ -501,8 +530,6 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
     lam[(long long)(n - 2) * st] = cm1;
     lam[(long long)(n - 1) * st] = c0;
     lam[0] = out1;
-#undef EC
-#undef ELE
   }
 }
 
@@ -591,18 +618,40 @@ __global__ void __launch_bounds__(128) k_adj_mu(Dev d, const unsigned char* __re
       // window: cells f-1..f+2 (a cell before b+1 is another lane's)
       double cm1 = 0.0, c0 = r ? 0.0 : v0, c1 = r ? 0.0 : v1, c2 = v2;
       double first = 0.0;  // cell 1 -> cell 2 (G(1) = F(2))
+      // what face f needs is loaded while face f-1 is worked on: its WM and
+      // UM, the cell entering (its lambda, factor and record byte, for the
+      // clip; cells past le1 are read at le1 and not used); the record bytes
+      // of faces f..f+2 wait in recs
+      auto rb = [&](int c) { return (unsigned)__ldg(rl + (long long)(c - 1) * st); };
+      unsigned recs = rb(f0) | rb(f0 + 1) << 8 | rb(f0 + 2) << 16;
+      double nwm, num, nlam, nls = 1.0;
+      unsigned nrec;
+      auto ahead = [&](int f) {
+        const int fc = min(f, fe), c = min(f + 3, le1);
+        const long long o = (long long)(c - 1) * st;
+        nwm = wm[(long long)(fc - 1) * sij];
+        num = um[(long long)(fc - 1) * sij];
+        nlam = lam[o];
+        if (kLoss) nls = ls[o];
+        nrec = rb(min(f + 3, n));
+      };
+      ahead(f0);
       for (int f = f0; f <= fe; ++f) {
-        const double C = MC(f);
+        const double C = fma(ekv, nwm, num);
+        const double vin = nlam, lin = nls;
+        recs |= nrec << 24;
+        ahead(f + 1);
         const bool neg = is_neg(C);
-        const int cs = (rl[(long long)(f - 1) * st] >> rsh) & 7;
+        const int cs = (recs >> rsh) & 7;
         // the cell entering next
         double lec = eA;
         if (f + 3 <= le1) {
-          lec = mle(f + 3);
+          lec = ((recs >> (24 + rsh)) & kClipBit) ? 0.0 : (kLoss ? vin * lin : vin);
         } else {
           eA = eB;
           eB = 0.0;
         }
+        recs >>= 8;
         if (kAdjIntMask & 8u)
           face_acc_a(adj_mul(8u, C, wl1 - wl0), neg, cs, corr_a_fix(courant_u(C, d.idmu[f - 1]), neg), beta, cm1, c0,
                      c1, c2);
