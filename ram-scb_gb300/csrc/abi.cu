@@ -1016,7 +1016,6 @@ int ramgpu_create(const ramgpu_config* cfg, ramgpu_ctx** out) {
   d.mhdmu = dalloc<double>(ctx, npa, &ok); d.iwmu = dalloc<double>(ctx, npa, &ok);
   d.idmu = dalloc<double>(ctx, npa + 1, &ok);
   d.mubin = dalloc<FaceMu>(ctx, npa, &ok);
-  d.bmhde = dalloc<double>(ctx, ne, &ok); d.bmhdmu = dalloc<double>(ctx, npa, &ok);
   d.grel = dalloc<double>(ctx, ns * ne, &ok); d.grbnd = dalloc<double>(ctx, ns * ne, &ok);
   d.vel = dalloc<double>(ctx, ns * ne, &ok); d.epp = dalloc<double>(ctx, ns * ne, &ok);
   d.rmas = dalloc<double>(ctx, ns, &ok);
@@ -1235,9 +1234,6 @@ int ramgpu_set_grid(ramgpu_ctx* ctx, const ramgpu_grid* g) {
     }
     CK(cudaMemcpy((void*)d.mubin, mb.data(), sizeof(FaceMu) * npa, cudaMemcpyHostToDevice));
   }
-  for (int k = 0; k < ne; ++k) r1[k] *= d.betalim;
-  for (int l = 0; l < npa; ++l) q1[l] *= d.betalim;
-  CK(up(d.bmhde, r1.data(), ne)); CK(up(d.bmhdmu, q1.data(), npa));
   // (NS,NE) Fortran -> [s][k]
   std::vector<double> t(ns * ne);
   auto tr2 = [&](const double* dst, const double* src) {

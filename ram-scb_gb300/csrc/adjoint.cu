@@ -19,6 +19,7 @@
 
 #include <type_traits>
 
+#include "face.cuh"
 #include "kernels.cuh"
 
 namespace ramgpu {
@@ -33,107 +34,54 @@ namespace ramgpu {
 // streamed once with a rolling window of four cell accumulators in
 // registers: after face f, cell f-1 is final and is written out.
 
-// Scatter of one face into the window (cm1, c0, c1, c2) = cells f-1..f+2.
 // FBND(f) = FUP + a LX depends on adjacent cells only: with C >= 0 (FUP =
 // F(f)) on (f-1, f) for LX = D, (f, f+1) for LX = X; with C < 0 (FUP =
-// F(f+1)) on (f, f+1) for LX = X, (f+1, f+2) for LX = D; its derivatives on
-// that pair are (-ak, 1+ak) when the pair ends at the upwind cell and
-// (1-ak, ak) when it starts there (upwind only: (1, 0)), with ak = a
-// (cases 2, 3) or beta*a (cases 1, 4).  The pair and the signed
-// coefficients are picked by integer selects, so a face costs one add and
-// two fma on the FP64 pipe whatever its case.
-__device__ __forceinline__ void face_acc(double FBb, bool neg, int cs, double ak, double& cm1,
-                                         double& c0, double& c1, double& c2) {
-  const bool xt = (cs == 2) | (cs == 4);  // LX = X (f, f+1)
-  const bool dt = (cs == 1) | (cs == 3);  // LX = D (f-1, f) or (f+1, f+2)
-  const bool ends = (dt & !neg) | (xt & neg);  // pair ends at the upwind cell
-  const bool starts = (xt & !neg) | (dt & neg);
-  const double sak = ends ? bitsd(dbits(ak) ^ kSignMask) : (starts ? ak : 0.0);
-  const double m = 1.0 - sak;
-  const double b0 = ends ? sak : m, b1 = ends ? m : sak;
-  // first cell of the pair in the window: 0 = f-1, 1 = f, 2 = f+1
-  const int p = neg ? (ends ? 1 : 2) : (ends ? 0 : 1);
-  const double p0 = p == 0 ? cm1 : (p == 1 ? c0 : c1);
-  const double p1 = p == 0 ? c0 : (p == 1 ? c1 : c2);
-  const double t0 = fma(b0, FBb, p0);
-  const double t1 = fma(b1, FBb, p1);
-  cm1 = p == 0 ? t0 : cm1;
-  c0 = p == 0 ? t1 : (p == 1 ? t0 : c0);
-  c1 = p == 1 ? t1 : (p == 2 ? t0 : c1);
-  c2 = p == 2 ? t1 : c2;
-}
+// F(f+1)) on (f, f+1) for LX = X, (f+1, f+2) for LX = D.  The pair and its
+// two weights, which add up to 1, are picked by integer selects, so a face
+// costs two fma on the FP64 pipe whatever its case.
+//
+// The transposes are bound by the FP64 unit, so the two FP64 operations that
+// form the weights move to integer instructions (as in face.cuh).  Backward
+// ms a call on 20x25x35x72, one species and four: 0.270 -> 0.262, 0.532 ->
+// 0.502.  That is FP64 for 81 % of the time with four species; forming the
+// product FBb = C*DL on the integer pipe as well was slower or even in every
+// sweep.
 
-// ---- the face weights on the integer pipe
-// The transposed sweeps are bound by the FP64 unit with three quarters of
-// their issue slots free (one FP64 warp instruction holds its pipe about as
-// long as 65 issue slots), so the two FP64 operations per face that form
-// the weights of face_acc, ak = k*a and m = 1 - sak, can move to integer
-// instructions where the sweep has the latency to spare (kAdjIntMask).
-// The fixed point is a signed 64-bit integer with 2^52 as 1: it keeps every
-// bit of its input down to 2^-52, so a and m differ from the FP64 fma and
-// add they replace by at most 2^-53 and 2^-52 absolute; they scale FBb in
-// the two accumulations, whose own rounding is of that size.  Courant
-// numbers of 1024 and more, inf and NaN give NaN weights.
-
-// Sweeps (bit w: R, P, E, MU) whose transposes form ak and m on the
-// integer pipe.
-constexpr unsigned kAdjIntMask = 0xBu;
-// Sweeps whose transposes form the face product FBb = C*DL (and, in E, the
-// coefficient's EDOT product) with mul_rn_int, the FP64 product bit for bit
-// on the integer pipe.  Measured on GB300: the DRIFTE transposes that form
-// C gain, the one that loads C (fewer FP64 operations left) loses and keeps
-// the FP64 product (the bits are the same either way); R (shared-memory
-// tiles, integer weights) loses over the whole adjoint window; P (bit 2) is
-// neutral and MU (bit 8) loses (backward 0.720-0.731 s with E alone, 0.725
-// with E and P, 0.736 with E and MU, 0.755 with all three, on one box).
-constexpr unsigned kAdjMulIntMask = 0x4u;
-__device__ __forceinline__ double adj_mul(unsigned bit, double a, double b) {
-  return (kAdjMulIntMask & bit) ? mul_rn_int(a, b) : a * b;
-}
-constexpr bits64 kNaNBits = 0x7FF8000000000000ULL;
-
-// |v| 2^-52 (v < 2^63) as the bits of a double with the given sign.
-__device__ __forceinline__ bits64 fix52_to_bits(bits64 v, bool neg) {
+// v 2^-64 as a double, rounded.
+__device__ __forceinline__ double fix64_to_double(uint64_t v) {
   const int lz = __clzll((long long)(v | 1ULL));
-  const bits64 r = ((bits64)(1034 - lz) << 52) | (((v << lz) >> 11) & kMantMask);
-  return (neg ? kSignMask : 0ULL) | (v ? r : 0ULL);
+  const uint64_t r = ((uint64_t)(1021 - lz) << 52) + ((((v << lz) >> 10) + 1) >> 1);
+  return bitsd(v ? r : 0ULL);
 }
-// |x| 2^52 for the bits of a double with |x| < 1024 (lower bits cut).
-__device__ __forceinline__ bits64 bits_to_fix52(bits64 x) {
-  const int e = (int)((x >> 52) & 0x7FF);
-  const bits64 mant = (x & kMantMask) | (e ? kImplicit : 0ULL);
-  const int sh = e - 1023;
-  return sh >= 0 ? (mant << (sh < 10 ? sh : 10)) : (mant >> (-sh < 63 ? -sh : 63));
-}
-// The CORR factor a = s*0.5*(1 - u) (s = -1 for neg) as bits, from the bits
-// ub of the Courant number u >= 0.
-__device__ __forceinline__ bits64 corr_a_fix(bits64 ub, bool neg) {
-  const long long D = (long long)(1ULL << 52) - (long long)bits_to_fix52(ub);  // (1 - u) 2^52
-  const bits64 r = fix52_to_bits((bits64)(D < 0 ? -D : D), neg != (D < 0));
-  const bits64 half = (r << 1) ? r - (1ULL << 52) : r;  // r / 2
-  return (ub >> 52) >= 1033 ? kNaNBits : half;
-}
-// 1 - x for the bits of x (|x| < 1024) as bits.
-__device__ __forceinline__ bits64 one_minus_bits(bits64 x) {
-  const bits64 X = bits_to_fix52(x);
-  const long long M = (x >> 63) ? (long long)((1ULL << 52) + X) : (long long)(1ULL << 52) - (long long)X;
-  const bits64 r = fix52_to_bits((bits64)(M < 0 ? -M : M), M < 0);
-  return ((x >> 52) & 0x7FF) >= 1033 ? kNaNBits : r;
-}
-// face_acc with ak = k*a from the CORR factor a (bits; k = beta for cases
-// 1, 4 by babs_bits) and m = 1 - sak, both on the integer pipe.
-__device__ __forceinline__ void face_acc_a(double FBb, bool neg, int cs, bits64 a, const BetaBits& beta,
-                                           double& cm1, double& c0, double& c1, double& c2) {
-  const bool xt = (cs == 2) | (cs == 4);
-  const bool dt = (cs == 1) | (cs == 3);
-  const bool ends = (dt & !neg) | (xt & neg);
-  const bool starts = (xt & !neg) | (dt & neg);
+// Scatter of one face of coefficient C into the window (cm1, c0, c1, c2) =
+// cells f-1..f+2, from q, C as the forward sweeps prepare it.  The pair's
+// weights are (1-w, w) where it starts at the upwind cell, (w, 1-w) where it
+// ends there, with w = ak for LX = X, -ak for LX = D, ak = k/2 (1 - U) (k =
+// beta in cases 1 and 4), 0 with upwind only.  Both are formed in fixed
+// point with 2^64 as 1 and rounded once; Courant numbers of 1 and more, inf
+// and NaN take the FP64 form (y: U = |C| y).
+__device__ __forceinline__ void face_acc_q(double FBb, double C, double y, const FaceCoef& q, int cs, uint64_t betaf,
+                                           double betalim, double& cm1, double& c0, double& c1, double& c2) {
+  const bool neg = is_neg(C);
+  const bool dt = (cs & 1) != 0;  // LX = D (f-1, f) or (f+1, f+2)
   const bool kb = (cs == 1) | (cs == 4);
-  const bits64 ak = kb ? ((a & kSignMask) | babs_bits(beta, bitsd(a))) : a;
-  const bits64 sak = ends ? (ak ^ kSignMask) : (starts ? ak : 0ULL);
-  const bits64 m = one_minus_bits(sak);
-  const double b0 = bitsd(ends ? sak : m), b1 = bitsd(ends ? m : sak);
-  const int p = neg ? (ends ? 1 : 2) : (ends ? 0 : 1);
+  const bool ends = dt != neg;  // (upwind only: either side, w = 0)
+  double w, m;
+  if (q.bad >= 0) {
+    uint64_t A = kb ? beta_times<false>(q.a63, betaf) : q.a63;
+    if (cs == 0) A = 0ULL;
+    w = bitsd(dbits(fix64_to_double(A)) ^ (dt ? kSignMask : 0ULL));
+    const uint64_t up = 0x3FF0000000000000ULL + (((A >> 11) + 1) >> 1);  // 1 + ak
+    m = (dt | (A == 0ULL)) ? bitsd(up) : fix64_to_double(0ULL - A);
+  } else {
+    const double k = kb ? 0.5 * betalim : 0.5;
+    const double ak = fma(fabs(C), -k * y, k);
+    w = cs == 0 ? 0.0 : (dt ? -ak : ak);
+    m = 1.0 - w;
+  }
+  const double b0 = ends ? w : m, b1 = ends ? m : w;
+  // first cell of the pair in the window: 0 = f-1, 1 = f, 2 = f+1
+  const int p = (int)neg + (int)!ends;
   const double p0 = p == 0 ? cm1 : (p == 1 ? c0 : c1);
   const double p1 = p == 0 ? c0 : (p == 1 ? c1 : c2);
   const double t0 = fma(b0, FBb, p0);
@@ -143,37 +91,13 @@ __device__ __forceinline__ void face_acc_a(double FBb, bool neg, int cs, bits64 
   c1 = p == 1 ? t1 : (p == 2 ? t0 : c1);
   c2 = p == 2 ? t1 : c2;
 }
-// Bits of the Courant number |c|*y (y = 1/DE or 1/DMU, positive normal):
-// the significands' product cut to 53 bits (as mul_pos_bits), 0 for zero,
-// subnormal or underflowing |c|*y, inf when it overflows or c is not finite.
-__device__ __forceinline__ bits64 courant_u(double c, double y) {
-  const bits64 ax = dbits(c) & kAbsMask, uy = dbits(y);
-  const int ex = (int)(ax >> 52);
-  const bits64 p = __umul64hi(((ax & kMantMask) | kImplicit) << 11, ((uy & kMantMask) | kImplicit) << 11);
-  const int hi = (int)(p >> 63);
-  const int e = ex + (int)(uy >> 52) - 1023 + hi;
-  const bits64 r = ((bits64)e << 52) | ((p >> (10 + hi)) & kMantMask);
-  return (ex == 0x7FF || e >= 0x7FF) ? 0x7FF0000000000000ULL : ((ax < kImplicit || e <= 0) ? 0ULL : r);
-}
 
-// ak = LIMITER weight times the CORR factor a = -0.5*(C*q - s) of a face:
-// fma(C, -0.5*k*q, 0.5*k*s) with k = beta for cases 1, 4 and 1 otherwise
-// (q = 1 for R and P; -0.5*q comes from the -0.5/DE, -0.5/DMU tables).
-// 0.5*k*s is formed either as a select of four constants or by flipping
-// the sign bit of 0.5*k; the two give the same value, and the compiler's
-// schedule is measurably faster with the first in the R and P transposes
-// and with the second in E and MU (hb = 0.5*beta).
-template <bool kXorSign>
-__device__ __forceinline__ double face_ak(double C, bool neg, int cs, double mh, double bmh, double hb) {
-  const bool kb = (cs == 1) | (cs == 4);
-  double shk;
-  if (kXorSign) {
-    const double hk = kb ? hb : 0.5;
-    shk = bitsd(dbits(hk) ^ (neg ? kSignMask : 0ULL));
-  } else {
-    shk = neg ? (kb ? -hb : -0.5) : (kb ? hb : 0.5);
-  }
-  return fma(C, kb ? bmh : mh, shk);
+// ak = LIMITER weight times the CORR factor a = -0.5*(C - s) of a face of
+// DRIFTP: fma(C, -0.5*k, 0.5*k*s) with k = beta for cases 1, 4 and 1
+// otherwise (the two faces that wrap around; hb = 0.5*beta).
+__device__ __forceinline__ double face_ak(double C, bool neg, int cs, double hb) {
+  const double hk = (cs == 1) | (cs == 4) ? hb : 0.5;
+  return fma(C, -hk, neg ? -hk : hk);
 }
 
 // lambda of cell c of a line (stride st) masked by the clip bit.  Both
@@ -252,8 +176,7 @@ __global__ void __launch_bounds__(128) k_adj_r(Dev d, const unsigned char* __res
       const double* __restrict__ grt = d.grt + ((long long)l * nt + j) * nr;
       const double* __restrict__ cr = d.cr + ((long long)m * nt + j) * nr;
       const double p4 = d.p4[s * ne + k];
-      const double hb = 0.5 * d.betalim, bmh = -hb;
-      const BetaBits beta(d.betalim);
+      const uint64_t betaf = beta_fix(dbits(d.betalim));
       const bool closed = d.flags & 1u;
       const int n = nr;  // >= 4
       auto mk = [&](int c) { return ((rl[c] >> rsh) & kClipBit) ? 0.0 : lam[c]; };  // masked lambda
@@ -264,13 +187,8 @@ __global__ void __launch_bounds__(128) k_adj_r(Dev d, const unsigned char* __res
       double cm1 = lam[0], c0 = le0, c1 = le1, c2 = le2;
       if (inflow && !closed) c0 += fma(grt[0], p4, cr[0]) * le0;  // FBND(1) = F(2)
       auto face = [&](int f, double C) {
-        const bool neg = is_neg(C);
         const int cs = (rl[f - 1] >> rsh) & 7;
-        if (kAdjIntMask & 1u)
-          face_acc_a(adj_mul(1u, C, le1 - le0), neg, cs, corr_a_fix(dbits(C) & kAbsMask, neg), beta, cm1, c0, c1,
-                     c2);
-        else
-          face_acc(adj_mul(1u, C, le1 - le0), neg, cs, face_ak<false>(C, neg, cs, -0.5, bmh, hb), cm1, c0, c1, c2);
+        face_acc_q(C * (le1 - le0), C, 1.0, face_coef(dbits(C)), cs, betaf, d.betalim, cm1, c0, c1, c2);
       };
       auto advance = [&](int f, double le3) {  // cell f-1 is final; cell f+3 enters
         lam[f - 2] = cm1;
@@ -350,8 +268,8 @@ __global__ void __launch_bounds__(128) k_adj_p(Dev d, const unsigned char* __res
     const double* __restrict__ gpt = d.gpt + ((long long)l * nt) * nr + i;
     const double* __restrict__ ca = d.ca + ((long long)m * nt) * nr + i;
     const double p2 = d.p2[((long long)s * ne + k) * nr + i];
-    const double hb = 0.5 * d.betalim, bmh = -hb;
-    const BetaBits beta(d.betalim);
+    const double hb = 0.5 * d.betalim;
+    const uint64_t betaf = beta_fix(dbits(d.betalim));
     const int n = nt;
 #define PC(J) fma(gpt[(long long)((J)-1) * nr], p2, ca[(long long)((J)-1) * nr])
 #define PLE(J) masked(lam, rl, (long long)((J)-1) * st, rsh)
@@ -364,8 +282,8 @@ __global__ void __launch_bounds__(128) k_adj_p(Dev d, const unsigned char* __res
       const double C = PC(n - 1);
       const bool neg = is_neg(C);
       const int cs = (rl[(long long)(n - 2) * st] >> rsh) & 7;
-      const double FBb = adj_mul(2u, C, leN - leNm);
-      const double V = face_ak<false>(C, neg, cs, -0.5, bmh, hb) * FBb;
+      const double FBb = C * (leN - leNm);
+      const double V = face_ak(C, neg, cs, hb) * FBb;
       if (neg) tN += FBb; else tNm1 += FBb;
       if (cs == 2 || cs == 4) { tN += V; tNm1 -= V; }
       else if (cs && !neg) { tNm1 += V; tNm2 -= V; }
@@ -375,8 +293,8 @@ __global__ void __launch_bounds__(128) k_adj_p(Dev d, const unsigned char* __res
       const double C = PC(n);
       const bool neg = is_neg(C);
       const int cs = (rl[(long long)(n - 1) * st] >> rsh) & 7;
-      const double FBb = adj_mul(2u, C, le2 - leN);  // Pb(NT) = -le(NT) + Pb(1), Pb(1) = le(2)
-      const double V = face_ak<false>(C, neg, cs, -0.5, bmh, hb) * FBb;
+      const double FBb = C * (le2 - leN);  // Pb(NT) = -le(NT) + Pb(1), Pb(1) = le(2)
+      const double V = face_ak(C, neg, cs, hb) * FBb;
       if (neg) w2 += FBb; else tN += FBb;
       if (cs == 2 || cs == 4) { w2 += V; tN -= V; }
       else if (cs && !neg) { tN += V; tNm1 -= V; }
@@ -387,12 +305,8 @@ __global__ void __launch_bounds__(128) k_adj_p(Dev d, const unsigned char* __res
     double cm1 = w1, c0 = le2 + w2, c1 = le1 + w3, c2 = lnext;
     auto step = [&](int J, double add, double lec) {  // face J, then cell J+3 enters
       const double C = PC(J);
-      const bool neg = is_neg(C);
       const int cs = (rl[(long long)(J - 1) * st] >> rsh) & 7;
-      if (kAdjIntMask & 2u)
-        face_acc_a(adj_mul(2u, C, le1 - le0), neg, cs, corr_a_fix(dbits(C) & kAbsMask, neg), beta, cm1, c0, c1, c2);
-      else
-        face_acc(adj_mul(2u, C, le1 - le0), neg, cs, face_ak<false>(C, neg, cs, -0.5, bmh, hb), cm1, c0, c1, c2);
+      face_acc_q(C * (le1 - le0), C, 1.0, face_coef(dbits(C)), cs, betaf, d.betalim, cm1, c0, c1, c2);
       lam[(long long)(J - 2) * st] = cm1;
       cm1 = c0; c0 = c1; c1 = c2; c2 = add;
       le0 = le1; le1 = lnext; lnext = lec;
@@ -458,8 +372,7 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
     const double ue = d.ue[(long long)m * nr * nt * d.npa + fij];
     const double* __restrict__ edot = d.edot + (long long)s * ne * nr + i;
     const double* __restrict__ eb = d.eb + s * ne;
-    const double hb = 0.5 * d.betalim;
-    const BetaBits beta(d.betalim);
+    const uint64_t betaf = beta_fix(dbits(d.betalim));
     const bool closed = d.flags & 1u;
     const int n = ne;
     const double out1 = lam[0];
@@ -484,16 +397,19 @@ __global__ void __launch_bounds__(128) k_adj_e(Dev d, const unsigned char* __res
     double cm1 = 0.0, c0 = 0.0, c1 = le2, c2 = le3;
     double vin;  // the masked lambda of cell K+3 as face(K) leaves it
     auto face = [&](int K) {
-      const double C = (kCo == 2) ? nc : adj_mul(4u, nc, fma(eb[K - 1], wet, ue));
+      const double C = (kCo == 2) ? nc : nc * fma(eb[K - 1], wet, ue);
       if (kCo == 1) cst[(long long)(K - 1) * st] = C;
       recs |= nrec << 24;
       vin = ((nrec >> rsh) & kClipBit) ? 0.0 : nlam;
       ahead(K + 1);
-      const bool neg = is_neg(C);
       const int cs = (recs >> rsh) & 7;
       recs >>= 8;
-      face_acc(adj_mul(kCo == 2 ? 0u : 4u, C, wl1 - wl0), neg, cs,
-               face_ak<true>(C, neg, cs, d.mhde[K - 1], d.bmhde[K - 1], hb), cm1, c0, c1, c2);
+      const double y = d.ide[K - 1];
+      FaceMu fm;
+      fm.sy = sig_62(dbits(y));
+      fm.sh = 2045 - (int)(dbits(y) >> 52);
+      face_acc_q(C * (wl1 - wl0), C, y, face_coef_mu(dbits(C), fm), cs, betaf, d.betalim, cm1,
+                 c0, c1, c2);
     };
     auto shift = [&](double lec, double wl) {
       cm1 = c0; c0 = c1; c1 = c2; c2 = lec;
@@ -579,8 +495,7 @@ __global__ void __launch_bounds__(128) k_adj_mu(Dev d, const unsigned char* __re
     const double* __restrict__ wm = d.wm + fij;
     const double* __restrict__ um = d.um + (long long)m * nt * nr * npa + fij;
     const double ekv = d.ek[s * ne + jk / nt];
-    const double hb = 0.5 * d.betalim;
-    const BetaBits beta(d.betalim);
+    const uint64_t betaf = beta_fix(dbits(d.betalim));
     const bool closed = d.flags & 1u;
     const int n = npa;
     const double* __restrict__ iwmu = d.iwmu;
@@ -641,7 +556,6 @@ __global__ void __launch_bounds__(128) k_adj_mu(Dev d, const unsigned char* __re
         const double vin = nlam, lin = nls;
         recs |= nrec << 24;
         ahead(f + 1);
-        const bool neg = is_neg(C);
         const int cs = (recs >> rsh) & 7;
         // the cell entering next
         double lec = eA;
@@ -652,12 +566,8 @@ __global__ void __launch_bounds__(128) k_adj_mu(Dev d, const unsigned char* __re
           eB = 0.0;
         }
         recs >>= 8;
-        if (kAdjIntMask & 8u)
-          face_acc_a(adj_mul(8u, C, wl1 - wl0), neg, cs, corr_a_fix(courant_u(C, d.idmu[f - 1]), neg), beta, cm1, c0,
-                     c1, c2);
-        else
-          face_acc(adj_mul(8u, C, wl1 - wl0), neg, cs, face_ak<true>(C, neg, cs, d.mhdmu[f - 1], d.bmhdmu[f - 1], hb),
-                   cm1, c0, c1, c2);
+        face_acc_q(C * (wl1 - wl0), C, d.idmu[f - 1], face_coef_mu(dbits(C), d.mubin[f - 1]), cs, betaf,
+                   d.betalim, cm1, c0, c1, c2);
         if (r == 0 && f == 2) first = cm1;
         if (f - 1 > b) lam[(long long)(f - 2) * st] = (r == 0 && f == 3) ? cm1 + first : cm1;
         cm1 = c0; c0 = c1; c1 = c2; c2 = lec;

@@ -44,7 +44,6 @@ struct Dev {
   // reciprocal grid tables: -0.5/DE, 1/WE, 1/DE (NE, then the largest 1/DE); -0.5/DMU, 1/WMU,
   // 1/DMU (NPA, then the largest 1/DMU of faces 2..NPA-1)
   const double *mhde, *iwe, *ide, *mhdmu, *iwmu, *idmu;
-  const double *bmhde, *bmhdmu;  // BetaLim times -0.5/DE and -0.5/DMU (adjoint)
   // per-species grid (ns x NE)
   const double *grel, *grbnd, *vel;
   const double *epp;

@@ -259,3 +259,35 @@ def test_transposed_lane_counts_agree():
             first = (j, gf[0], gb[0])
         assert j == first[0] and np.array_equal(gf[0], first[1])
         assert np.abs(gb[0] - first[2]).max() <= 1e-13 * np.abs(first[2]).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("beta", [1.0, 1.3, 1.5, 2.0])
+@pytest.mark.parametrize("dts", [5.0, 400.0])
+def test_transposes_at_the_limits(dts, beta):
+    """The transposes' fixed-point weights, and at the long step the FP64
+    ones of faces with Courant numbers above 1: one call's misfit and
+    gradients against the oracle at the window test's bars (1e-12, 1e-9)."""
+    from ramgpu import abi, workload as W
+    import pyoracle
+    wl = W.make_workload("tiny_pert8")
+    g, ns = wl.grid, len(wl.grid.species)
+    obs = [{"member": 0, "s": s, "call": 0, "k": 6 + 5 * n, "l": 1 + 9 * n, "lshell": 3.0 + 0.7 * n, "mlt": 5.0 * n,
+            "log_obs": 0.0} for s in range(ns) for n in range(5)]
+    gpu, o = abi.RamGpu(g, wl.fields, betalim=beta), pyoracle.Oracle(g, wl.fields, betalim=beta)
+    try:
+        for s in range(ns):
+            gpu.upload_f2(0, s, np.asfortranarray(wl.f2[s]))
+            gpu.set_boundary(0, s, wl.fgeos[s])
+        j = gpu.adj_forward(1, dts, np.full((1, 1), 4.0), 1, obs)[0]
+        gf, gb = gpu.adj_backward()
+        gpu.ram_run(dts)  # (a recorded call keeps no limits)
+        assert (gpu.cfl(0, 1).min() < 0.8 * dts) == (dts > 100.0)  # Courant numbers above 1 at the long step
+    finally:
+        gpu.close()
+    jc, cf, cb = o.window_gradient([np.asfortranarray(a) for a in wl.f2], [np.asfortranarray(a) for a in wl.fgeos], dts,
+                                   [4.0], obs)
+    assert abs(j - jc) <= 1e-12 * jc
+    for s in range(ns):
+        assert np.abs(gf[0, s] - cf[s]).max() <= 1e-9 * np.abs(cf[s]).max(), s
+        assert np.abs(gb[0, s] - cb[s]).max() <= 1e-9 * max(np.abs(cb[s]).max(), 1e-300), s
