@@ -533,15 +533,17 @@ static int enqueue_status(ramgpu_ctx* ctx) {
   return RAMGPU_OK;
 }
 
-static int enqueue_body(ramgpu_ctx* ctx, double dts) {
+static int enqueue_body(ramgpu_ctx* ctx, double dts, bool chained) {
   const int G = step_group_count(ctx);
   int rc = RAMGPU_OK;
   if (G > 1) {
     if ((rc = ensure_group_streams(ctx, G))) return rc;
     rc = enqueue_pipeline(ctx, dts, nullptr, nullptr, nullptr, G, {});
   } else {
-    if ((rc = enqueue_tables(ctx, dts))) return rc;
-    rc = enqueue_sweeps(ctx, dts);
+    ctx->d.chained = chained;
+    rc = enqueue_tables(ctx, dts);
+    if (!rc) rc = enqueue_sweeps(ctx, dts);
+    ctx->d.chained = 0;
   }
   if (!rc && ctx->check_on) rc = enqueue_status(ctx);
   return rc;
@@ -648,7 +650,14 @@ static int enqueue_ram_run(ramgpu_ctx* ctx, double dts) {
   if (rc) return rc;
   ctx->last_dts = dts;
   if (ctx->d.nitems == 0) return RAMGPU_OK;
-  if (!ctx->graph_on || ctx->timing) return enqueue_body(ctx, dts);
+  if (!ctx->graph_on || ctx->timing) {
+    // chained (launch_k) unless events come between the launches or the
+    // caller's capture takes them
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool chained = !ctx->timing && cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess &&
+                         cap == cudaStreamCaptureStatusNone;
+    return enqueue_body(ctx, dts, chained);
+  }
   // CUDA graph: capture once per (dts, work list, flags, launch shapes), replay
   if (!ctx->graph_exec || ctx->graph_dts != dts || ctx->graph_items != ctx->items_version ||
       ctx->graph_flags != ctx->d.flags || ctx->graph_shape != ctx->shape_version) {
@@ -656,7 +665,7 @@ static int enqueue_ram_run(ramgpu_ctx* ctx, double dts) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     const long long l0 = ctx->launches;
-    rc = enqueue_body(ctx, dts);
+    rc = enqueue_body(ctx, dts, false);
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
     if (rc) {
       if (g) cudaGraphDestroy(g);
@@ -2440,7 +2449,7 @@ int ramgpu_autotune(ramgpu_ctx* ctx, double dts, int reps, double* best_ms4) {
         float tbest = 1e30f;
         for (int r = 0; r <= reps; ++r) {
           cudaEventRecord(e0, ctx->stream);
-          if (int rc2 = enqueue_body(ctx, dts)) {
+          if (int rc2 = enqueue_body(ctx, dts, !ctx->graph_on)) {
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
             cudaFree(snap);
@@ -2473,7 +2482,7 @@ int ramgpu_autotune(ramgpu_ctx* ctx, double dts, int reps, double* best_ms4) {
       float tbest = 1e30f;
       for (int r = 0; r <= reps; ++r) {
         cudaEventRecord(e0, ctx->stream);
-        if (int rc2 = enqueue_body(ctx, dts)) {
+        if (int rc2 = enqueue_body(ctx, dts, !ctx->graph_on)) {
           cudaEventDestroy(e0);
           cudaEventDestroy(e1);
           cudaFree(snap);

@@ -148,6 +148,7 @@ struct Vec {
 // groups ahead.  No barrier: a thread touches its own slots only.
 template <int kCfl, int kRec, bool kB32, int V>
 __global__ void __launch_bounds__(256, 4) k_sweep_r(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
+  chain_enter();
   extern __shared__ double slots[];
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   // the lines of the L window [lw0, lw1) (all of them unless a pipeline
@@ -310,6 +311,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_r(Dev d, double dts, unsigned 
 // ahead, or unrolling by 2 or 4, took 594 to 703.
 template <int kCfl, int kRec, bool kB32>
 __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
+  chain_enter();
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   const int line0 = d.lw0 * (nr - 1) * ne;  // the L window, as in DRIFTR
   const int nlines = (nr - 1) * ne * (d.lw1 - d.lw0);
@@ -418,6 +420,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
 // lane but the first sees the extrapolated cells.
 template <bool kCfl, int kRec, bool kB32, int kSplit>
 __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
+  chain_enter();
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   const int line0 = d.lw0 * (nr - 1) * nt;  // the L window, as in DRIFTR
   const int nlines = (nr - 1) * nt * (d.lw1 - d.lw0);
@@ -554,6 +557,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
 template <bool kCfl, int kLoss, int kRec, bool kB32, int kSplit>
 __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const double* __restrict__ lossA,
                                                      unsigned char* __restrict__ rec, int rsh) {
+  chain_enter();
   const int nr = d.nr, nt = d.nt, ne = d.ne, npa = d.npa;
   const int nlines = (nr - 1) * nt * ne;
   const int lpb = blockDim.x / kSplit;  // lines per CTA
@@ -720,12 +724,12 @@ static inline bool beta_b32(const Dev& d) {
     const dim3 g = grid_for(d, W, nlines_of(d, W));                                                           \
     const int b = d.blk[W];                                                                                   \
     const bool n = d.count_clips;                                                                             \
-    if (rec && replay) KERNEL<0, 2, kB><<<g, b, 0, st>>>(d, dts, rec, rsh);                               \
-    else if (rec) KERNEL<0, 1, kB><<<g, b, 0, st>>>(d, dts, rec, rsh);                                    \
+    if (rec && replay) launch_k(d.chained, KERNEL<0, 2, kB>, g, b, 0, st, d, dts, rec, rsh);                               \
+    else if (rec) launch_k(d.chained, KERNEL<0, 1, kB>, g, b, 0, st, d, dts, rec, rsh);                                    \
     else if (cfl && (d.flags >> 31))                                                                          \
-      (n ? KERNEL<2, 3, kB> : KERNEL<2, 0, kB>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);                         \
-    else if (cfl) (n ? KERNEL<1, 3, kB> : KERNEL<1, 0, kB>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);             \
-    else (n ? KERNEL<0, 3, kB> : KERNEL<0, 0, kB>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);                      \
+      launch_k(d.chained, n ? KERNEL<2, 3, kB> : KERNEL<2, 0, kB>, g, b, 0, st, d, dts, nullptr, 0);                         \
+    else if (cfl) launch_k(d.chained, n ? KERNEL<1, 3, kB> : KERNEL<1, 0, kB>, g, b, 0, st, d, dts, nullptr, 0);             \
+    else launch_k(d.chained, n ? KERNEL<0, 3, kB> : KERNEL<0, 0, kB>, g, b, 0, st, d, dts, nullptr, 0);                      \
   }                                                                                                           \
   void NAME(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int rsh) {  \
     if (beta_b32(d)) NAME##_b<true>(d, dts, cfl, st, rec, replay, rsh);                                       \
@@ -740,11 +744,11 @@ static void r_launch(const Dev& d, double dts, bool cfl, cudaStream_t st, unsign
   const int b = d.blk[0];
   const size_t sm = V > 1 ? 3 * V * b * sizeof(double) : 0;
   const bool n = d.count_clips;
-  if (rec && replay) k_sweep_r<0, 2, kB, V><<<g, b, sm, st>>>(d, dts, rec, rsh);
-  else if (rec) k_sweep_r<0, 1, kB, V><<<g, b, sm, st>>>(d, dts, rec, rsh);
-  else if (cfl && (d.flags >> 31)) (n ? k_sweep_r<2, 3, kB, V> : k_sweep_r<2, 0, kB, V>)<<<g, b, sm, st>>>(d, dts, nullptr, 0);
-  else if (cfl) (n ? k_sweep_r<1, 3, kB, V> : k_sweep_r<1, 0, kB, V>)<<<g, b, sm, st>>>(d, dts, nullptr, 0);
-  else (n ? k_sweep_r<0, 3, kB, V> : k_sweep_r<0, 0, kB, V>)<<<g, b, sm, st>>>(d, dts, nullptr, 0);
+  if (rec && replay) launch_k(d.chained, k_sweep_r<0, 2, kB, V>, g, b, sm, st, d, dts, rec, rsh);
+  else if (rec) launch_k(d.chained, k_sweep_r<0, 1, kB, V>, g, b, sm, st, d, dts, rec, rsh);
+  else if (cfl && (d.flags >> 31)) launch_k(d.chained, n ? k_sweep_r<2, 3, kB, V> : k_sweep_r<2, 0, kB, V>, g, b, sm, st, d, dts, nullptr, 0);
+  else if (cfl) launch_k(d.chained, n ? k_sweep_r<1, 3, kB, V> : k_sweep_r<1, 0, kB, V>, g, b, sm, st, d, dts, nullptr, 0);
+  else launch_k(d.chained, n ? k_sweep_r<0, 3, kB, V> : k_sweep_r<0, 0, kB, V>, g, b, sm, st, d, dts, nullptr, 0);
 }
 // Cells per access.  While an SM's lines (32 warps of 8*NR bytes a lane) stay
 // in L1 (NR up to 24), cells move one at a time: the wide accesses bring
@@ -779,10 +783,10 @@ static void e_launch(const Dev& d, double dts, bool cfl, cudaStream_t st, unsign
   const dim3 g = grid_for(d, 2, kS * nlines_of(d, 2));
   const int b = d.blk[2];
   const bool n = d.count_clips;
-  if (rec && replay) k_sweep_e<false, 2, kB, kS><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (rec) k_sweep_e<false, 1, kB, kS><<<g, b, 0, st>>>(d, dts, rec, rsh);
-  else if (cfl) (n ? k_sweep_e<true, 3, kB, kS> : k_sweep_e<true, 0, kB, kS>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
-  else (n ? k_sweep_e<false, 3, kB, kS> : k_sweep_e<false, 0, kB, kS>)<<<g, b, 0, st>>>(d, dts, nullptr, 0);
+  if (rec && replay) launch_k(d.chained, k_sweep_e<false, 2, kB, kS>, g, b, 0, st, d, dts, rec, rsh);
+  else if (rec) launch_k(d.chained, k_sweep_e<false, 1, kB, kS>, g, b, 0, st, d, dts, rec, rsh);
+  else if (cfl) launch_k(d.chained, n ? k_sweep_e<true, 3, kB, kS> : k_sweep_e<true, 0, kB, kS>, g, b, 0, st, d, dts, nullptr, 0);
+  else launch_k(d.chained, n ? k_sweep_e<false, 3, kB, kS> : k_sweep_e<false, 0, kB, kS>, g, b, 0, st, d, dts, nullptr, 0);
 }
 void launch_sweep_e(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int rsh) {
   const int lanes = e_lanes(d);
@@ -813,12 +817,12 @@ static void mu_launch(const Dev& d, double dts, const double* loss, cudaStream_t
   const dim3 g = grid_for(d, 3, kS * nlines_of(d, 3));
   const int b = d.blk[3];
   const bool n = d.count_clips;
-  if (rec && replay) k_sweep_mu<false, kLoss, 2, kB, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
-  else if (rec) k_sweep_mu<false, kLoss, 1, kB, kS><<<g, b, 0, st>>>(d, dts, loss, rec, rsh);
+  if (rec && replay) launch_k(d.chained, k_sweep_mu<false, kLoss, 2, kB, kS>, g, b, 0, st, d, dts, loss, rec, rsh);
+  else if (rec) launch_k(d.chained, k_sweep_mu<false, kLoss, 1, kB, kS>, g, b, 0, st, d, dts, loss, rec, rsh);
   else if (cfl)
-    (n ? k_sweep_mu<true, kLoss, 3, kB, kS> : k_sweep_mu<true, kLoss, 0, kB, kS>)<<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
+    launch_k(d.chained, n ? k_sweep_mu<true, kLoss, 3, kB, kS> : k_sweep_mu<true, kLoss, 0, kB, kS>, g, b, 0, st, d, dts, loss, nullptr, 0);
   else
-    (n ? k_sweep_mu<false, kLoss, 3, kB, kS> : k_sweep_mu<false, kLoss, 0, kB, kS>)<<<g, b, 0, st>>>(d, dts, loss, nullptr, 0);
+    launch_k(d.chained, n ? k_sweep_mu<false, kLoss, 3, kB, kS> : k_sweep_mu<false, kLoss, 0, kB, kS>, g, b, 0, st, d, dts, loss, nullptr, 0);
 }
 template <int kLoss, bool kB>
 static void mu_lanes_launch(const Dev& d, double dts, const double* loss, cudaStream_t st, unsigned char* rec,

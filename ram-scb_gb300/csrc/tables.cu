@@ -410,6 +410,7 @@ struct VtSource {
 // from the graph 0.111 -> 0.107 ms on 6x9x35x72, 0.196 -> 0.191 for one
 // species on 20x25x35x72, 0.376 -> 0.369 for four).
 __global__ void k_member_ij(Dev d, bool clear_cfl) {
+  chain_enter();
   const int per = d.nr * d.nt;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (clear_cfl && blockIdx.x == 0)
@@ -470,6 +471,7 @@ __device__ __forceinline__ void ghost_plane(const Dev& d, int it, int p) {
 // Per (member, I, J, L): UE and UM from the (I,J) factors; the blocks past
 // nb_ijl find the ghost planes of every work item (4 planes per block).
 __global__ void __launch_bounds__(128) k_member_ijl(Dev d, int nb_ijl) {
+  chain_enter();
   if ((int)blockIdx.x >= nb_ijl) {
     const int np = d.ne * d.npa, bpi = (np + 3) / 4;
     const int b = (int)blockIdx.x - nb_ijl;
@@ -502,7 +504,7 @@ void launch_member_coef(const Dev& d, double dts, cudaStream_t st, bool clear_cf
   const long long n = (long long)d.nm * d.nr * d.nt * d.npa;
   const int nb_ijl = (int)((n + 127) / 128);
   const int nb_ghost = ((d.ne * d.npa + 3) / 4) * d.nitems;
-  k_member_ijl<<<(unsigned)(nb_ijl + nb_ghost), 128, 0, st>>>(d, nb_ijl);
+  launch_k(d.chained, k_member_ijl, nb_ijl + nb_ghost, 128, 0, st, d, nb_ijl);
 }
 
 // Exclusive "last defined" scan over planes: one block per work item.
@@ -520,6 +522,7 @@ __device__ __forceinline__ void last_scan_warp(int& h, double& v, int& src) {
 }
 
 __global__ void __launch_bounds__(1024) k_ghost_scan(Dev d) {
+  chain_enter();
   __shared__ int s_h[32];
   __shared__ double s_v[32];
   __shared__ int s_s[32];
@@ -570,7 +573,7 @@ __global__ void __launch_bounds__(1024) k_ghost_scan(Dev d) {
 }
 
 // The planes themselves are found in launch_member_coef's second kernel.
-void launch_ghost(const Dev& d, cudaStream_t st) { k_ghost_scan<<<d.nitems, 1024, 0, st>>>(d); }
+void launch_ghost(const Dev& d, cudaStream_t st) { launch_k(d.chained, k_ghost_scan, d.nitems, 1024, 0, st, d); }
 
 // -------------------------------------------------- loss factor (bookkeeping path)
 __global__ void k_loss_apply(Dev d, const double* __restrict__ table) {
@@ -588,6 +591,7 @@ void launch_loss_apply(const Dev& d, const double* table, cudaStream_t st) {
 
 // ------------------------------------ periodic copy + magnetopause mask
 __global__ void k_finish(Dev d, int any_outside) {
+  chain_enter();
   // the (I, K, L) of the L window [lw0, lw1)
   const long long n = (long long)d.nr * d.ne * (d.lw1 - d.lw0);
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x + (long long)d.lw0 * d.nr * d.ne;
@@ -606,7 +610,7 @@ __global__ void k_finish(Dev d, int any_outside) {
 void launch_finish(const Dev& d, cudaStream_t st) {
   // any_outside is folded into the flags word bit 31 by the host
   long long n = (long long)d.nr * d.ne * (d.lw1 - d.lw0);
-  k_finish<<<dim3((unsigned)((n + 255) / 256), d.nitems), 256, 0, st>>>(d, (d.flags >> 31) & 1u);
+  launch_k(d.chained, k_finish, dim3((unsigned)((n + 255) / 256), d.nitems), 256, 0, st, d, (d.flags >> 31) & 1u);
 }
 
 // ---------------------------------------------------------- ANISCH moments
@@ -625,6 +629,7 @@ void launch_finish(const Dev& d, cudaStream_t st) {
 // on 40x49x70x144 304, 206 us.
 constexpr int kMomL = 8;
 __global__ void __launch_bounds__(32 * kMomL) k_moments(Dev d, int nlb, unsigned* __restrict__ done) {
+  chain_enter();
   __shared__ double2 sh[kMomL][32];
   __shared__ bool lastblk;
   const int nr1 = d.nr - 1, npair = nr1 * d.nt;
@@ -719,7 +724,7 @@ size_t mom_done_count(const Dev& d) { return (size_t)d.nm * d.ns * mom_tiles(d);
 void launch_moments(const Dev& d, cudaStream_t st) {
   // pitch angles past the largest UPA carry nothing
   const int nlb = (d.mom_lmax + kMomL - 1) / kMomL;
-  k_moments<<<dim3((unsigned)(mom_tiles(d) * nlb), d.nitems), dim3(32, kMomL), 0, st>>>(d, nlb, d.mom_done);
+  launch_k(d.chained, k_moments, dim3((unsigned)(mom_tiles(d) * nlb), d.nitems), dim3(32, kMomL), 0, st, d, nlb, d.mom_done);
 }
 
 // ANISCH's only effect on F2, F2(I,J,K,1) = F2(I,J,K,2) for I, K >= 2
