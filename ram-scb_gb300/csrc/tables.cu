@@ -602,9 +602,17 @@ __global__ void k_finish(Dev d, int any_outside) {
   const long long kl = t / d.nr;  // K + NE*L
   double* f = d.f2 + (long long)slot * d.ncell + kl * d.nt * d.nr + i;
   f[(long long)(d.nt - 1) * d.nr] = f[0];  // F2(:,:,NT,:,:) = F2(:,:,1,:,:)
+  // the flags of 8 J at a time, before their stores (one by one, each flag
+  // waited for the store before it: 12.0 us a launch against 6.0 on 23x30x37x69)
   if (any_outside)
-    for (int j = 0; j < d.nt; ++j)
-      if (d.outside[(long long)j * d.nr + i] == 1) f[(long long)j * d.nr] = 1.e-31;
+    for (int j0 = 0; j0 < d.nt; j0 += 8) {
+      int out[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) out[q] = j0 + q < d.nt ? d.outside[(long long)(j0 + q) * d.nr + i] : 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (out[q] == 1) f[(long long)(j0 + q) * d.nr] = 1.e-31;
+    }
 }
 
 void launch_finish(const Dev& d, cudaStream_t st) {
