@@ -793,7 +793,11 @@ static int ensure_group_streams(ramgpu_ctx* ctx, int G) {
 // the next chunk's arrive over the host link), the pitch-angle sweeps
 // (whose lines span every plane) run once all chunks are in, and the
 // reverse E, P, R and the copy/mask of chunk c are followed at once by its
-// read-back (while the next chunk computes).  ANISCH, which rewrites the
+// read-back (while the next chunk computes: chunk c + 1 starts its reverse
+// sweeps after the first of chunk c's, so that the read-backs spread over
+// the time of the sweeps; a four-species call from the pageable reference
+// array 787 -> 768 us, 775 and 771 when it waits for the second and the
+// third).  ANISCH, which rewrites the
 // L = 1 plane, runs last; that plane and the moments go back after it.
 // Streams: chunk c on its own stream; inputs chained in chunk order (they
 // share the link); the per-member tables, ghost planes and pitch-angle
@@ -803,7 +807,7 @@ static int ensure_group_streams(ramgpu_ctx* ctx, int G) {
 // planes write disjoint cells, and CFL maxima and clip counts combine by
 // atomic max/add, so results equal the resident step's bit for bit.
 static int ensure_chunk_events(ramgpu_ctx* ctx, int C) {
-  while ((int)ctx->chunk_events.size() < 3 * C + 3) {
+  while ((int)ctx->chunk_events.size() < 4 * C + 3) {
     cudaEvent_t e = nullptr;
     CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     ctx->chunk_events.push_back(e);
@@ -856,7 +860,11 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
     Dev dc = full;
     dc.lw0 = lo(c);
     dc.lw1 = lo(c + 1);
+    // a chunk's E waits for the one before: side by side all chunks would
+    // finish, and queue for the link, at the same time
+    if (c > 0) CK(cudaStreamWaitEvent(st, ev[3 * C + 2 + c], 0));
     { NvtxRange r("DRIFTE"); launch_sweep_e(dc, dts, false, st); }
+    CK(cudaEventRecord(ev[3 * C + 3 + c], st));
     { NvtxRange r("DRIFTP"); launch_sweep_p(dc, dts, false, st); }
     { NvtxRange r("DRIFTR"); launch_sweep_r(dc, dts, false, st); }
     launch_finish(dc, st);
@@ -880,7 +888,8 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
 // auto_chunks: the count used while the setting is automatic (-1).  Measured
 // on the four-species step: per-species page-locked arrays go faster over
 // the item-group pipeline (0.69 ms per call against 0.93-1.07 ms chunked),
-// the reference layout over 4 chunks (0.88 ms against 0.91 ms unchunked).
+// the reference layout over 4 chunks (us a call with 2, 3, 4, 5, 6, 8: 805,
+// 770, 772, 791, 790, 790; unchunked 807).
 static int chunk_count(const ramgpu_ctx* ctx, int auto_chunks) {
   const int want = ctx->pipe_chunks < 0 ? auto_chunks : ctx->pipe_chunks;
   if (want <= 0 || (ctx->cfg.flags & RAMGPU_FLAG_LOSSES) || ctx->pd_any() || ctx->pipe_trace) return 0;
@@ -1520,7 +1529,7 @@ static int ref_in(ramgpu_ctx* ctx, const double* host, const double* r, double* 
     CK(cudaMemcpyAsync(ctx->ref_stage, host, sizeof(double) * ns * ncell, cudaMemcpyHostToDevice, st));
     r = ctx->ref_stage;
   }
-  launch_ref_gather(r, slots, ns, stride, 0, ncell, ctx->nsm, st);
+  launch_ref_gather(r, slots, ns, stride, 0, ncell, 2 * ctx->nsm, st);
   ctx->launches += 1;
   CKL("reference-layout gather");
   return RAMGPU_OK;
@@ -1533,14 +1542,14 @@ static int ref_out(ramgpu_ctx* ctx, double* host, double* w, const double* slots
   const int ns = ctx->d.ns;
   if (!w) {
     if (int rc = ensure_stage(ctx)) return rc;
-    launch_ref_scatter(slots, ctx->ref_stage, ns, stride, c0, c1, ctx->nsm, st);
+    launch_ref_scatter(slots, ctx->ref_stage, ns, stride, c0, c1, 2 * ctx->nsm, st);
     ctx->launches += 1;
     CKL("reference-layout scatter");
     CK(cudaMemcpyAsync(host + c0 * ns, ctx->ref_stage + c0 * ns, sizeof(double) * ns * (c1 - c0),
                        cudaMemcpyDeviceToHost, st));
     return RAMGPU_OK;
   }
-  launch_ref_scatter(slots, w, ns, stride, c0, c1, ctx->nsm, st);
+  launch_ref_scatter(slots, w, ns, stride, c0, c1, 2 * ctx->nsm, st);
   ctx->launches += 1;
   CKL("reference-layout scatter");
   return RAMGPU_OK;
@@ -1947,7 +1956,8 @@ int ramgpu_ram_run_ref(ramgpu_ctx* ctx, double dts, double* const* f2, double* c
           CK(cudaMemcpyAsync(mem[m].f2ce + o, mem[m].f2 + o, b, cudaMemcpyHostToDevice, st));
           src = mem[m].f2ce;
         }
-        launch_ref_gather(src, ctx->d.f2 + (size_t)m * ns * n, ns, n, l0 * plane, l1 * plane, ctx->nsm, st);
+        launch_ref_gather(src, ctx->d.f2 + (size_t)m * ns * n, ns, n, l0 * plane, l1 * plane,
+                          mem[m].f2ce ? 2 * ctx->nsm : std::max(1, ctx->nsm / 2), st);
         ctx->launches += 1;
       }
     CKL("reference-layout gather");
@@ -1958,7 +1968,8 @@ int ramgpu_ram_run_ref(ramgpu_ctx* ctx, double dts, double* const* f2, double* c
     for (int m = 0; m < nm && a < l1; ++m)
       if (mem[m].f2) {
         double* dst = mem[m].f2ce ? mem[m].f2ce : mem[m].f2r;
-        launch_ref_scatter(ctx->d.f2 + (size_t)m * ns * n, dst, ns, n, a * plane, l1 * plane, ctx->nsm, st);
+        launch_ref_scatter(ctx->d.f2 + (size_t)m * ns * n, dst, ns, n, a * plane, l1 * plane,
+                           mem[m].f2ce ? 2 * ctx->nsm : std::max(1, ctx->nsm / 2), st);
         ctx->launches += 1;
         if (mem[m].f2ce) {
           const size_t o = (size_t)a * plane * ns, b = sizeof(double) * (size_t)(l1 - a) * plane * ns;

@@ -144,9 +144,9 @@ void launch_sum_pressure(const Dev& d, int member, unsigned mask, double* pall, 
 // <-> ref[c*ns + s] for cells c in [c0, c1); ref may be host memory the
 // device reaches (mapped page-locked, or pageable over a coherent link).
 void launch_ref_gather(const double* ref, double* slots, int ns, long long stride, long long c0, long long c1,
-                       int nsm, cudaStream_t st);
+                       int ctas, cudaStream_t st);
 void launch_ref_scatter(const double* slots, double* ref, int ns, long long stride, long long c0, long long c1,
-                        int nsm, cudaStream_t st);
+                        int ctas, cudaStream_t st);
 
 void launch_selftest_mul(long long n, unsigned long long seed, unsigned long long* bad, cudaStream_t st);
 // Status word of the active items (status.cu): st[5] device words.

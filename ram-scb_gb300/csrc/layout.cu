@@ -48,24 +48,27 @@ __global__ void __launch_bounds__(kLayoutTile) k_ref_scatter(const double* __res
   }
 }
 
-// The host link, not the SMs, limits these copies when one side is host
-// memory; a grid of one CTA per SM keeps enough loads in flight.
-static int layout_grid(long long ncells, int nsm) {
+// At most `ctas` CTAs: two per SM, but half as many as SMs where the kernel
+// reads or writes host memory beside other chunks' sweeps (the host link is
+// the limit and waiting CTAs take the sweeps' room: a four-species call from
+// the pageable reference array with 4, 2, 1, 1/2 CTAs per SM 820, 799, 793,
+// 787 us; with nothing beside it fewer are slower, 807 -> 844 us in one piece).
+static int layout_grid(long long ncells, int ctas) {
   const long long tiles = (ncells + kLayoutTile - 1) / kLayoutTile;
-  return (int)std::max(1LL, std::min(tiles, (long long)nsm * 2));
+  return (int)std::max(1LL, std::min(tiles, (long long)ctas));
 }
 
 void launch_ref_gather(const double* ref, double* slots, int ns, long long stride, long long c0, long long c1,
-                       int nsm, cudaStream_t st) {
+                       int ctas, cudaStream_t st) {
   if (c1 <= c0) return;
-  k_ref_gather<<<layout_grid(c1 - c0, nsm), kLayoutTile, kLayoutTile * ns * sizeof(double), st>>>(ref, slots, ns,
+  k_ref_gather<<<layout_grid(c1 - c0, ctas), kLayoutTile, kLayoutTile * ns * sizeof(double), st>>>(ref, slots, ns,
                                                                                                   stride, c0, c1);
 }
 
 void launch_ref_scatter(const double* slots, double* ref, int ns, long long stride, long long c0, long long c1,
-                        int nsm, cudaStream_t st) {
+                        int ctas, cudaStream_t st) {
   if (c1 <= c0) return;
-  k_ref_scatter<<<layout_grid(c1 - c0, nsm), kLayoutTile, kLayoutTile * ns * sizeof(double), st>>>(slots, ref, ns,
+  k_ref_scatter<<<layout_grid(c1 - c0, ctas), kLayoutTile, kLayoutTile * ns * sizeof(double), st>>>(slots, ref, ns,
                                                                                                    stride, c0, c1);
 }
 
