@@ -31,8 +31,12 @@ namespace ramgpu {
 // direction in the low one, which ORs its code into that byte.  (The
 // reverse half is transposed first; its nibble is the cheaper one to read.)
 __device__ __forceinline__ unsigned rget(const unsigned char* p, int rsh) { return (unsigned)*p >> rsh; }
-__device__ __forceinline__ void rput(unsigned char* p, int rsh, unsigned v) {
-  *p = (unsigned char)(rsh ? (v << 4) : (*p | v));
+// The forward half writes the high nibble (rsh 4), the reverse half adds the
+// low one to `old`, the byte as rold read it before the face's arithmetic (at
+// the store, every face waited for the read).
+__device__ __forceinline__ unsigned rold(const unsigned char* p, int rsh) { return rsh ? 0u : (unsigned)*p; }
+__device__ __forceinline__ void rput(unsigned char* p, int rsh, unsigned old, unsigned v) {
+  *p = (unsigned char)(rsh ? (v << 4) : (old | v));
 }
 
 // phi of a face by the FP64 unit, for what face_flux leaves out.  Out of
@@ -210,6 +214,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_r(Dev d, double dts, unsigned 
       // face f, 2 <= f <= NR-1: the new cell f
       auto step = [&](int f, double c, double gpp) {
         limit(f, c);
+        const unsigned old = kRec == 1 ? rold(rl + (f - 1), rsh) : 0u;
         const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
         int cs = kRec == 2 ? (int)(rget(rl + (f - 1), rsh) & 7) : 0;
         const double phi = face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), beta,
@@ -217,7 +222,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_r(Dev d, double dts, unsigned 
         const double raw = (g0 - phi) + phi_prev;
         const double v = (kRec == 2) ? clip_frozen(raw, rget(rl + (f - 1), rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
-        if (kRec == 1) rput(rl + (f - 1), rsh, cs | (is_neg(raw) ? kClipBit : 0));
+        if (kRec == 1) rput(rl + (f - 1), rsh, old, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
         gm = g0; g0 = gp; gp = gpp;
         return v;
@@ -297,7 +302,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_r(Dev d, double dts, unsigned 
         a.store(fl + nr - W);
       }
       if (kRec == kRecCount) nclip += is_neg(rawn);
-      if (kRec == 1) rput(rl + (nr - 1), rsh, csn | (is_neg(rawn) ? kClipBit : 0));
+      if (kRec == 1) rput(rl + (nr - 1), rsh, rold(rl + (nr - 1), rsh), csn | (is_neg(rawn) ? kClipBit : 0));
     }
     if (kRec == kRecCount) warp_atomic_add(&d.clipq[slot], nclip);
     if (kCfl) warp_atomic_max(&d.cflq[slot * 4 + 0], q);
@@ -363,6 +368,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
       double gm = G1, g0 = G2, gp = G3;
       auto step = [&](int J, double c, double gpp, auto wrap) {
         limit(J, c);
+        const unsigned old = kRec == 1 ? rold(rl + (long long)(J - 1) * st, rsh) : 0u;
         const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
         const unsigned char* rj = (kRec == 1 || kRec == 2) ? rl + (long long)(J - 1) * st : nullptr;
         int cs = kRec == 2 ? (int)(rget(rj, rsh) & 7) : 0;
@@ -380,7 +386,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
         const double raw = (g0 - phi) + phi_prev;
         GJ(J) = (kRec == 2) ? clip_frozen(raw, rget(rj, rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
-        if (kRec == 1) rput(rl + (long long)(J - 1) * st, rsh, cs | (is_neg(raw) ? kClipBit : 0));
+        if (kRec == 1) rput(rl + (long long)(J - 1) * st, rsh, old, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
         gm = g0; g0 = gp; gp = gpp;
       };
@@ -399,7 +405,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
       if (kRec == kRecCount) nclip += is_neg(rawN);
       GJ(nt) = vN;
       GJ(1) = vN;
-      if (kRec == 1) rput(rl + (long long)(nt - 1) * st, rsh, csN | (is_neg(rawN) ? kClipBit : 0));
+      if (kRec == 1) rput(rl + (long long)(nt - 1) * st, rsh, rold(rl + (long long)(nt - 1) * st, rsh), csN | (is_neg(rawN) ? kClipBit : 0));
   #undef GJ
   #undef CJ
     }
@@ -505,11 +511,12 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
         int cs = kRec == 2 ? (int)(rget(rb, rsh) & 7) : 0;
         phi_prev = face(b, bins[b - 1], fma(bins[b - 1].k, wet, ue), w0, w1, w2, w3, cs, std::false_type());
         if (closed && r == 0) phi_prev = 0.0;
-        if (kRec == 1 && r == 0) rput(rb, rsh, cs);
+        if (kRec == 1 && r == 0) rput(rb, rsh, rold(rb, rsh), cs);
       }
       double gm = w1, g0 = w2, gp = w3;
       auto step = [&](int K, double v, double gpp, auto end) {
         const FaceBin bin = bins[K - 1];
+        const unsigned old = kRec == 1 ? rold(rl + (uint64_t)(K - 1) * st, rsh) : 0u;
         const unsigned char* rk = (kRec == 1 || kRec == 2) ? rl + (uint64_t)(K - 1) * st : nullptr;
         int cs = kRec == 2 ? (int)(rget(rk, rsh) & 7) : 0;
         double phi = face(K, bin, v, gm, g0, gp, gpp, cs, end);
@@ -517,7 +524,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
         const double raw = fma(phi_prev - phi, bin.iw, g0);
         GK(K) = (kRec == 2) ? clip_frozen(raw, rget(rk, rsh)) : clip(raw);
         if (kRec == kRecCount) nclip += is_neg(raw);
-        if (kRec == 1) rput(rl + (uint64_t)(K - 1) * st, rsh, cs | (is_neg(raw) ? kClipBit : 0));
+        if (kRec == 1) rput(rl + (uint64_t)(K - 1) * st, rsh, old, cs | (is_neg(raw) ? kClipBit : 0));
         phi_prev = phi;
         gm = g0; g0 = gp; gp = gpp;
       };
@@ -643,8 +650,8 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
       }
       double gm = w1, g0 = w2, gp = w3;
       // cell L from its raw value, with its record
-      auto put = [&](int L, double raw, int cs) {
-        if (kRec == 1) rput(rl + (uint64_t)(L - 1) * st, rsh, cs | (is_neg(raw) ? kClipBit : 0));
+      auto put = [&](int L, double raw, int cs, unsigned old) {
+        if (kRec == 1) rput(rl + (uint64_t)(L - 1) * st, rsh, old, cs | (is_neg(raw) ? kClipBit : 0));
         if (kRec == kRecCount) nclip += is_neg(raw);
         return (kRec == 2) ? clip_frozen(raw, rget(rl + (uint64_t)(L - 1) * st, rsh)) : clip(raw);
       };
@@ -656,9 +663,10 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
         // 40x49x70x144, the two launches' mean: 633 -> 591 us; 20x25x35x72: 58.1 -> 56.3)
         const double loss = kLoss == 1 ? LA(L) : 1.0;
         const FaceMu bin = bins[L - 1];
+        const unsigned old = kRec == 1 ? rold(rl + (uint64_t)(L - 1) * st, rsh) : 0u;
         int cs = kRec == 2 ? (int)(rget(rl + (uint64_t)(L - 1) * st, rsh) & 7) : 0;
         const double phi = face(L, bin, CL(L), gm, g0, gp, nxt, cs);
-        double v = put(L, fma(phi_prev - phi, bin.iw, g0), cs);
+        double v = put(L, fma(phi_prev - phi, bin.iw, g0), cs, old);
         if (kLoss == 1) v *= loss;
         GL(L) = v;
         phi_prev = phi;
@@ -672,7 +680,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const do
         const double c = CL(L);
         if (kCfl && inside) quotient(L, c);
         const double phi = c * (closed ? 0.0 : gp);
-        const double v = put(L, fma(phi_prev - phi, bin.iw, g0), 0);
+        const double v = put(L, fma(phi_prev - phi, bin.iw, g0), 0, kRec == 1 ? rold(rl + (uint64_t)(L - 1) * st, rsh) : 0u);
         const double vN = v * d.rho[fij];
         if (kLoss == 1) {
           GL(L) = v * LA(L);
