@@ -424,8 +424,11 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
 // neighbours' cells is loaded before a __syncwarp, and no lane writes before
 // it; the flux of a face is the same bits in either lane.  S >= 4, so no
 // lane but the first sees the extrapolated cells.
+// Four lanes are for short lists, where 24 warps an SM are plenty: their
+// instance may hold 85 registers (with 8 lanes in DRIFTMU alike; a call on
+// 6x9x35x72 0.1033 -> 0.1023 ms from the graph, 0.1233 -> 0.1213 direct).
 template <bool kCfl, int kRec, bool kB32, int kSplit>
-__global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
+__global__ void __launch_bounds__(256, kSplit > 2 ? 3 : 4) k_sweep_e(Dev d, double dts, unsigned char* __restrict__ rec, int rsh) {
   chain_enter();
   const int nr = d.nr, nt = d.nt, ne = d.ne;
   const int line0 = d.lw0 * (nr - 1) * nt;  // the L window, as in DRIFTR
@@ -562,7 +565,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_e(Dev d, double dts, unsigned 
 // last to NPA) and forms face b anew (the first lane's face 1 carries
 // nothing).  S >= 4, so no lane but the first sees the F(1) = F(2) rule.
 template <bool kCfl, int kLoss, int kRec, bool kB32, int kSplit>
-__global__ void __launch_bounds__(256, 4) k_sweep_mu(Dev d, double dts, const double* __restrict__ lossA,
+__global__ void __launch_bounds__(256, kSplit > 4 ? 3 : 4) k_sweep_mu(Dev d, double dts, const double* __restrict__ lossA,
                                                      unsigned char* __restrict__ rec, int rsh) {
   chain_enter();
   const int nr = d.nr, nt = d.nt, ne = d.ne, npa = d.npa;
