@@ -72,7 +72,7 @@ NCU_CAPTURE = {
                           "driftmu": 0.5 * (6.62 + 5.69)},
 }
 SWEEP_SOURCES = ["ram-scb_gb300/csrc/sweeps.cu", "ram-scb_gb300/csrc/ramgpu_internal.cuh",
-                 "ram-scb_gb300/csrc/kernels.cuh"]
+                 "ram-scb_gb300/csrc/kernels.cuh", "ram-scb_gb300/csrc/face.cuh"]
 SECTIONS = ("headline", "single", "refined", "padif", "ensemble", "adjoint")
 
 
@@ -99,7 +99,7 @@ def parse():
     ap.add_argument("--no-graph", action="store_true")
     ap.add_argument("--no-autotune", action="store_true")
     ap.add_argument("--no-coef-store", action="store_true",
-                    help="recompute the face coefficients in the reverse half instead of storing them")
+                    help="recompute the face coefficients in the second DRIFTE transpose instead of keeping them")
     ap.add_argument("--members", type=int, default=256, help="ensemble members")
     ap.add_argument("--ensemble-calls", type=int, default=0,
                     help="ram_run calls of the ensemble run (0: until the last member retires)")
@@ -1119,7 +1119,7 @@ def run_gb300(args, rank, world, local_rank):
                    "cells_per_step": head["cells_per_step"], "l2": "flushed between timed steps (256 MB write)",
                    "graph": not args.no_graph, "launch_shapes": head["launch_shapes"],
                    "autotune_trials": head["autotune_trials"], "item_groups": head["item_groups"],
-                   "coef_store": "none" if args.no_coef_store else "DRIFTE",
+                   "coef_store": "none" if args.no_coef_store else "DRIFTE transposes",
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
         "roofline": head["roofline"], "kernels_ms": head["kernels_ms"],
         "kernel_pass_ms_per_step": head["kernel_pass_ms_per_step"],

@@ -255,7 +255,8 @@ int ramgpu_pipeline_groups(const ramgpu_ctx *ctx);
 int ramgpu_set_pipeline_trace(ramgpu_ctx *ctx, int enable);
 int ramgpu_pipeline_trace(ramgpu_ctx *ctx, int *groups, float *ms);
 /* Number of item groups whose sweeps ramgpu_ram_run (and _async) runs on
- * concurrent streams (1..8, default 4, at most one per item): one group's
+ * concurrent streams (1..8, at most one per item; until set or tuned 4, but 1
+ * for lists below 1.5 M cells, whose launches run in one wave): one group's
  * launch tails and the gaps between its dependent launches fill with the
  * others' CTAs.  Results are the same for every count; the loss
  * bookkeeping (RAMGPU_FLAG_LOSSES) and per-kernel timing passes run as one

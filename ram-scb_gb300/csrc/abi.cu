@@ -4,7 +4,7 @@
 //   member tables (VT, E x B, U terms) and DRIFTR ghost planes   2 kernels
 //   "last inflow line" scan of the stale DRIFTR ghosts           1
 // and then, for each item group (a slice of the active (member, species)
-// list, on its own stream; 1 to 8 groups, autotuned):
+// list, on its own stream; 1 for short lists, else 4, or 1 to 8 as tuned):
 //   R, P, E, MU (+ fused CEX/ATMOL)      4   (forward half, CFL tracked)
 //   MU, E, P, R                          4   (reverse half)
 //   periodic copy + magnetopause mask    1
@@ -902,8 +902,7 @@ static int chunk_count(const ramgpu_ctx* ctx, int auto_chunks) {
 // first) ; the per-member tables, ghost planes and CFL reset on the
 // context's stream -> event ; group g: its uploads, the tables event, its
 // sweeps and tail on a view of the work list, its read-back -> event the
-// context's stream waits for.  The coefficient store is indexed by the
-// item's place in the full list (Dev::item0), so groups never share it.
+// context's stream waits for.
 // f2 == NULL: no copies at all (the resident step over groups).
 // Enqueue only (direct launches or inside a graph capture of the context's
 // stream, which the group streams join through the events).
@@ -3136,11 +3135,9 @@ int ramgpu_set_adj_overlap(ramgpu_ctx* ctx, int on) {
 
 // The second stream, its events (2 per ring slot + 2) and the shadow copies
 // of everything a recorded call writes besides F2 and its record: the
-// per-member tables CR, CA, DRD1, DPD1, UE, UM and the DRIFTR ghost planes,
-// and a coefficient store of its own when the context has one (without it
-// the DRIFTE reverse recomputes its coefficients: the same bits, two FP64
-// operations per cell more).  Returns in q the context's Dev with those
-// pointers replaced and without clip counting.
+// per-member tables CR, CA, DRD1, DPD1, UE, UM and the DRIFTR ghost planes.
+// Returns in q the context's Dev with those pointers replaced and without
+// clip counting.
 // One set of the tables a call writes besides F2: per member CR, CA, DRD1,
 // DPD1, UE, UM, per slot the DRIFTR ghost planes (256-byte pieces).
 static size_t table_set_bytes(const Dev& d) {

@@ -334,8 +334,8 @@ __global__ void __launch_bounds__(128) k_adj_p(Dev d, const unsigned char* __res
 // kCo: 0 compute the face coefficients C, 1 compute and keep them in the
 // DRIFTE coefficient store, 2 read them from it.  A call's two DRIFTE
 // transposes (of the reverse and the forward half) share C (same DTs and
-// potential), so the first keeps it for the second, as the forward sweeps
-// do; the stored value is the recomputed one, so the results do not change.
+// potential), so the first keeps it for the second; the stored value is the
+// recomputed one, so the results do not change.
 // A warp's instructions issue in order: the cell entering the window was
 // masked, and so waited for, where it was loaded, an L2 round trip per face.
 // Loading a face ahead, backward ms a call with and without (one species,

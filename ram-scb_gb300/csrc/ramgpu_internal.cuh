@@ -12,8 +12,8 @@
 //
 // Cost model: on GB300 the FP64 pipe (add/mul/fma, and also FP64 min/max and
 // compares) issues ~0.53 T lane-ops/s while the integer and FP32 pipes are
-// ~35-70x faster, so every sign test, threshold test, min/max and select is
-// done on the integer bit pattern, leaving 8-9 FP64 add/mul/fma per face.
+// ~35-70x faster, so a face's flux is formed in integer fixed point
+// (face.cuh), leaving three FP64 add/mul/fma per face.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -165,8 +165,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_r(Dev d, double dts, unsigned 
     const int line = line0 + u.b * blockDim.x + threadIdx.x;
     unsigned long long q = kBits1em10;  // CFL quotient bits: |C| at least 1e-10
     unsigned nclip = 0;  // clip events (kRec == kRecCount)
-    // bounds-checked builds: the line's cells, its GRT and CR rows, the
-    // coefficient store's item
+    // bounds-checked builds: the line's cells, its GRT and CR rows
     const bool lok = line >= line0 + nlines ||
         rg_ok(d, rg_item(d, item) && rg_span((long long)line * nr, nr, 1, d.ncell) &&
                      rg_span(((long long)(line / (nt * ne)) * nt + line % nt) * nr, nr, 1, (long long)nr * nt * d.npa) &&
@@ -326,8 +325,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
     const int line = line0 + u.b * blockDim.x + threadIdx.x;
     unsigned long long q = kBits1em10;  // CFL quotient bits: |C| at least 1e-10
     unsigned nclip = 0;  // clip events (kRec == kRecCount)
-    // bounds-checked builds: the line's cells, its GPT and CA columns, the
-    // coefficient store's item
+    // bounds-checked builds: the line's cells, its GPT and CA columns
     const bool lok = line >= line0 + nlines ||
         rg_ok(d, rg_item(d, item) &&
                      rg_span((long long)(line / (nr - 1)) * nt * nr + 1 + line % (nr - 1), nt, nr, d.ncell) &&

@@ -652,8 +652,9 @@ class RamGpu:
         return {KCLASS[k]: (float(ms[k]), int(cnt[k])) for k in range(len(KCLASS)) if cnt[k]}
 
     def set_coef_store(self, mask):
-        """Sweeps (bit 0 R, 1 P, 2 E, 3 MU; True = 4, False = 0) whose forward
-        face coefficients are kept for the reverse half."""
+        """Bit 2 (True = 4, False = 0): the adjoint's first DRIFTE transpose of a
+        call keeps its face coefficients for the second.  Other bits are
+        accepted and change nothing."""
         m = (4 if mask else 0) if isinstance(mask, bool) else int(mask)
         self._ck(self.lib.ramgpu_set_coef_store(self.h, m), "set_coef_store")
 
