@@ -48,28 +48,28 @@ UNIT = "cell-updates/s"
 # launch.  The line reports whether the current sources still have that
 # digest; a changed kernel makes the figures stale until the next capture.
 NCU_CAPTURE = {
-    # ncu on the sources named by sources_sha16 (profiles/sweeps_four_sp.md,
-    # profiles/driftr_refined.md, profiles/sweeps_l2.md): one kernel per
-    # command, each captured launch advances one species, so a four-species
-    # launch of the timing pass is scaled by 4.
-    "sources_sha16": "8faa21e4265be355",
+    # ncu on the sources named by sources_sha16 (profiles/sweeps_four_sp.md):
+    # the sweep launches of one whole call, summed over its item groups; the
+    # mean of the forward and the reverse half, as the timing pass counts them
+    "sources_sha16": "f67598a11b2ae3d7",
     "command": ("ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum,lts__t_bytes.sum,"
                 "smsp__sass_thread_inst_executed_op_{dadd,dfma,dmul}_pred_on.sum --clock-control none "
-                "-k regex:k_sweep_<r|p|e|mu> -c 2 python bench.py --steps 2 --warmup 1 --sections headline "
+                "-k regex:k_sweep_ -c <32|8> python bench.py --steps 2 --warmup 1 --sections headline "
                 "--no-cpu-baseline --no-e2e --no-autotune [--workload refined|single_h]"),
-    "dram_bytes": {"four_sp": {"driftr": 4 * 11.02e6, "driftp": 4 * 10.39e6,
-                               "drifte": 4 * 0.5 * (11.34e6 + 29.98e6), "driftmu": 4 * 0.5 * (20.47e6 + 10.52e6)},
-                   "single_h": {"driftr": 11.03e6, "driftp": 10.40e6,
-                                "drifte": 0.5 * (11.33e6 + 29.98e6), "driftmu": 0.5 * (20.47e6 + 10.52e6)},
-                   "refined": {"driftr": 4 * 0.5 * (268.51e6 + 267.80e6)}},
-    # lts__t_bytes.sum per launch of the timing pass (profiles/sweeps_l2.md)
-    "l2_bytes": {"four_sp": {"driftr": 4 * 0.5 * (112.45e6 + 112.11e6), "driftp": 4 * 0.5 * (39.40e6 + 39.16e6),
-                             "drifte": 4 * 0.5 * (70.01e6 + 70.05e6), "driftmu": 4 * 0.5 * (78.02e6 + 58.62e6)},
-                 "single_h": {"driftr": 0.5 * (112.54e6 + 111.96e6), "driftp": 0.5 * (39.44e6 + 39.26e6),
-                              "drifte": 0.5 * (70.63e6 + 70.04e6), "driftmu": 0.5 * (78.13e6 + 58.64e6)},
-                 "refined": {"driftr": 4 * 0.5 * (2156.6e6 + 2314.6e6)}},
-    "fp64_ops_per_cell": {"driftr": 5.02, "driftp": 4.64, "drifte": 0.5 * (6.70 + 4.78),
-                          "driftmu": 0.5 * (6.62 + 5.69)},
+    "dram_bytes": {"four_sp": {"driftr": 44.10e6, "driftp": 41.58e6, "drifte": 41.61e6,
+                               "driftmu": 0.5 * (42.13e6 + 81.92e6)},
+                   "single_h": {"driftr": 11.03e6, "driftp": 10.39e6, "drifte": 10.40e6,
+                                "driftmu": 0.5 * (10.53e6 + 20.48e6)},
+                   "refined": {"driftr": 0.5 * (1112.3e6 + 1142.4e6), "driftp": 1041.0e6, "drifte": 1029.8e6,
+                               "driftmu": 0.5 * (1044.4e6 + 1743.1e6)}},
+    "l2_bytes": {"four_sp": {"driftr": 0.5 * (448.5e6 + 454.6e6), "driftp": 0.5 * (156.7e6 + 157.7e6),
+                             "drifte": 0.5 * (143.9e6 + 145.3e6), "driftmu": 0.5 * (280.6e6 + 394.8e6)},
+                 "single_h": {"driftr": 0.5 * (111.7e6 + 113.3e6), "driftp": 0.5 * (39.2e6 + 39.4e6),
+                              "drifte": 0.5 * (41.9e6 + 44.4e6), "driftmu": 0.5 * (70.1e6 + 98.8e6)},
+                 "refined": {"driftr": 0.5 * (3555.1e6 + 3660.7e6), "driftp": 0.5 * (2441.8e6 + 2453.5e6),
+                             "drifte": 0.5 * (2175.7e6 + 2184.5e6), "driftmu": 0.5 * (3360.9e6 + 4480.2e6)}},
+    "fp64_ops_per_cell": {"driftr": 3.06, "driftp": 2.74, "drifte": 0.5 * (2.90 + 2.99),
+                          "driftmu": 0.5 * (2.84 + 3.89)},
 }
 SWEEP_SOURCES = ["ram-scb_gb300/csrc/sweeps.cu", "ram-scb_gb300/csrc/ramgpu_internal.cuh",
                  "ram-scb_gb300/csrc/kernels.cuh", "ram-scb_gb300/csrc/face.cuh"]
