@@ -653,10 +653,9 @@ static int enqueue_ram_run(ramgpu_ctx* ctx, double dts) {
   if (!ctx->graph_on || ctx->timing) {
     // chained (launch_k) unless events come between the launches or the
     // caller's capture takes them
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool chained = !ctx->timing && cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess &&
-                         cap == cudaStreamCaptureStatusNone;
-    return enqueue_body(ctx, dts, chained);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+    if (!ctx->timing && cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) cudaGetLastError();
+    return enqueue_body(ctx, dts, cap == cudaStreamCaptureStatusNone);
   }
   // CUDA graph: capture once per (dts, work list, flags, launch shapes), replay
   if (!ctx->graph_exec || ctx->graph_dts != dts || ctx->graph_items != ctx->items_version ||
