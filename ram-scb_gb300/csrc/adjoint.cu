@@ -741,9 +741,9 @@ void launch_obs_adj(const Dev& d, const ObsDev* obs, int nobs, int call, const d
 // Order-independent digest of a branch record: two sums (mod 2^32) of
 // position-mixed 32-bit hashes of its 32-bit words, read 16 bytes at a time
 // (a ragged tail byte by byte).  Equal digests of two runs mean an
-// unchanged pattern with overwhelming probability.  One atomic a block: the
-// 8192 of one a warp to the same address took most of 12.6 us a call (20 MB
-// of record), this 9.4.
+// unchanged pattern with overwhelming probability.  One atomic a block: with
+// one a warp, 8192 to the same address, 12.6 us a call (20 MB of record),
+// so 9.4.
 __device__ __forceinline__ unsigned mix32(unsigned w, unsigned long long i, unsigned c1, unsigned c2) {
   unsigned h = (w + (unsigned)i * 0x9E3779B9u + (unsigned)(i >> 32)) * c1;
   h ^= h >> 15;
