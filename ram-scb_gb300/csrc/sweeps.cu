@@ -631,7 +631,8 @@ __global__ void __launch_bounds__(256, kSplit > 4 ? 3 : 4) k_sweep_mu(Dev d, dou
       const uint64_t betaf = beta_fix(dbits(beta));
       const bool closed = d.flags & 1u;
   #define CL(L) fma(ekv, strided_b(wm, (L)-1, sij), strided_b(um, (L)-1, sij))
-      // face L's flux; the CFL quotient |C|/DMU is the Courant number
+      // face L's flux; the CFL quotient |C|/DMU is the Courant number, which
+      // counts from L = 2 on (lanes that share a line form face 1 as well)
       Largest big;
       auto quotient = [&](int L, double c) { q = umax64(q, dbits(c * d.idmu[L - 1]) & kAbsMask); };
       auto face = [&](int L, const FaceMu& bin, double c, double gm, double g0, double gp, double gpp, int& cs) {
@@ -640,7 +641,7 @@ __global__ void __launch_bounds__(256, kSplit > 4 ? 3 : 4) k_sweep_mu(Dev d, dou
         const bool neg = fc.sign;  // C = 0 carries nothing either way
         return face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, fc, beta, betaf, cs,
                                     [&] { return c; }, [&] { return d.mhdmu[L - 1]; },
-                                    [&] { if (kCfl && inside) quotient(L, c); });
+                                    [&] { if (kCfl && inside && L > 1) quotient(L, c); });
       };
       double phi_prev = 0.0;
       if (kSplit > 1) {
