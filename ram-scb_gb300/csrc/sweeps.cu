@@ -41,21 +41,25 @@ __device__ __forceinline__ void rput(unsigned char* p, int rsh, unsigned old, un
 
 // phi of a face by the FP64 unit, for what face_flux leaves out.  Out of
 // line, so that its FP64 instructions are not issued predicated off.
-// x, dd: the reference's X and D; kRec 2: with the branch rcs.
+// x, dd: the reference's X and D, u and d: the cells upwind and downwind by
+// C's sign bit.  That differs from C < 0 for -0 alone, whose flux comes from
+// F(f), here d, as for +0: it carries nothing but a NaN.  kRec 2: with the
+// branch rcs.
 struct PhiCase {
   double phi;
   int cs;
 };
 template <int kRec>
-static __device__ __noinline__ PhiCase face_phi_fp64(double x, double dd, double u, double c, double mh, double beta,
-                                                     int rcs) {
+static __device__ __noinline__ PhiCase face_phi_fp64(double x, double dd, double u, double d, double c, double mh,
+                                                     double beta, int rcs) {
   const BetaBits b(beta);
   const bool neg = is_neg(c);
   const double a = fma(c, mh, neg ? -0.5 : 0.5);
   PhiCase r;
   r.cs = rcs;
-  const double fb = kRec == 2 ? face_value_frozen(x, dd, u, a, b, rcs)
-                              : face_value_case(x, babs_bits(b, x), dd, babs_bits(b, dd), u, a, r.cs);
+  double fb = kRec == 2 ? face_value_frozen(x, dd, u, a, b, rcs)
+                        : face_value_case(x, babs_bits(b, x), dd, babs_bits(b, dd), u, a, r.cs);
+  if (dbits(c) == kSignMask) fb = d;
   r.phi = __dmul_rn(c, fb);
   return r;
 }
@@ -85,7 +89,7 @@ __device__ __forceinline__ double face_phi(double uu, double u, double d, double
       return bitsd((bits64)q.sign << 32);
     }
     const bool neg = q.sign != 0;
-    const PhiCase r = face_phi_fp64<kRec>(neg ? u - d : d - u, neg ? uu - u : u - uu, u, cf(), mh(), beta, cs);
+    const PhiCase r = face_phi_fp64<kRec>(neg ? u - d : d - u, neg ? uu - u : u - uu, u, d, cf(), mh(), beta, cs);
     phi = r.phi;
     if (kRec == 1) cs = r.cs;
   }
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_r(Dev d, double dts, unsigned 
       auto step = [&](int f, double c, double gpp) {
         limit(f, c);
         const unsigned old = kRec == 1 ? rold(rl + (f - 1), rsh) : 0u;
-        const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
+        const bool neg = hi32(dbits(c)) < 0;  // (-0: face_phi_fp64)
         int cs = kRec == 2 ? (int)(rget(rl + (f - 1), rsh) & 7) : 0;
         const double phi = face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), beta,
                                                 betaf, cs, [&] { return c; }, mh);
@@ -359,7 +363,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
       };
       limit(nt, cN);
       int csN = kRec == 2 ? (int)(rget(rl + (long long)(nt - 1) * st, rsh) & 7) : 0;
-      const bool negN = is_neg(cN);
+      const bool negN = hi32(dbits(cN)) < 0;  // (-0: face_phi_fp64)
       const double phiN = face_phi<kRec, kB32>(negN ? G3 : GNm, negN ? G2 : GN, negN ? GN : G2, cN, face_coef(dbits(cN)),
                                                beta, betaf, csN, [&] { return cN; }, mh);
       double phi_prev = phiN;
@@ -367,7 +371,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
       auto step = [&](int J, double c, double gpp, auto wrap) {
         limit(J, c);
         const unsigned old = kRec == 1 ? rold(rl + (long long)(J - 1) * st, rsh) : 0u;
-        const bool neg = hi32(dbits(c)) < 0;  // C = 0 carries nothing either way
+        const bool neg = hi32(dbits(c)) < 0;  // (-0: face_phi_fp64)
         const unsigned char* rj = (kRec == 1 || kRec == 2) ? rl + (long long)(J - 1) * st : nullptr;
         int cs = kRec == 2 ? (int)(rget(rj, rsh) & 7) : 0;
         double phi = face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, face_coef(dbits(c)), beta,
@@ -375,8 +379,8 @@ __global__ void __launch_bounds__(256, 4) k_sweep_p(Dev d, double dts, unsigned 
         // The reference's D of face NT-1 against the flow is F(2)-F(1), with
         // F(1) in the place of F(NT); the two differ only in states that are
         // not periodic.
-        if (decltype(wrap)::value && neg && dbits(G1) != dbits(GN)) {
-          const PhiCase r = face_phi_fp64<kRec>(gp - g0, G2 - G1, gp, c, -0.5, beta,
+        if (decltype(wrap)::value && is_neg(c) && dbits(G1) != dbits(GN)) {
+          const PhiCase r = face_phi_fp64<kRec>(gp - g0, G2 - G1, gp, g0, c, -0.5, beta,
                                                 kRec == 2 ? (int)(rget(rj, rsh) & 7) : 0);
           phi = r.phi;
           cs = r.cs;
@@ -638,7 +642,7 @@ __global__ void __launch_bounds__(256, kSplit > 4 ? 3 : 4) k_sweep_mu(Dev d, dou
       auto face = [&](int L, const FaceMu& bin, double c, double gm, double g0, double gp, double gpp, int& cs) {
         const FaceCoef fc = face_coef_mu(dbits(c), bin);
         if (kCfl) big.see(fc, L);
-        const bool neg = fc.sign;  // C = 0 carries nothing either way
+        const bool neg = fc.sign;  // (-0: face_phi_fp64)
         return face_phi<kRec, kB32>(neg ? gpp : gm, neg ? gp : g0, neg ? g0 : gp, c, fc, beta, betaf, cs,
                                     [&] { return c; }, [&] { return d.mhdmu[L - 1]; },
                                     [&] { if (kCfl && inside && L > 1) quotient(L, c); });
