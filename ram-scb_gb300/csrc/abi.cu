@@ -1289,7 +1289,7 @@ int ramgpu_set_fields(ramgpu_ctx* ctx, const double* fnhs, const double* fnis, c
   CK(cudaMemcpy((void*)d.outside, outside_mgnp, sizeof(int) * d.nr * d.nt, cudaMemcpyHostToDevice));
   ctx->any_outside = 0;
   for (int i = 0; i < d.nr * d.nt; ++i)
-    if (outside_mgnp[i] == 1) ctx->any_outside = 1;
+    if (outside_mgnp[i] != 0) ctx->any_outside = 1;  // the limits count cells of flag 0, the mask those of 1
   ctx->have_fields = true;
   ctx->field_dirty = true;
   return RAMGPU_OK;
