@@ -392,7 +392,8 @@ int ramgpu_set_mu_lanes(ramgpu_ctx *ctx, int lanes);
  * SMs), timing whole ram_run steps on the context's active items (best of
  * reps), keeps the fastest, then times 1, 2, 4 and 8 item groups
  * (ramgpu_set_step_groups) on those shapes and keeps the fastest, and
- * restores F2 afterwards (it allocates a temporary snapshot).  best_ms4
+ * restores what the trial steps changed (F2, loss books, moments, limits,
+ * status word; it allocates a temporary snapshot).  best_ms4
  * (may be NULL) receives the best step time of each sweep's round. */
 int ramgpu_autotune(ramgpu_ctx *ctx, double dts, int reps, double *best_ms4);
 /* The best whole-step trial time of the last ramgpu_autotune for each sweep

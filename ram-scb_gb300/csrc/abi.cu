@@ -2407,6 +2407,71 @@ int ramgpu_get_launch_shape(ramgpu_ctx* ctx, int* threads4, int* persistent4) {
   return RAMGPU_OK;
 }
 
+// One trial of the tuner: a whole ram_run step (direct launches) with the
+// shapes as they are, as the sweeps interact through L2 and the SM schedule,
+// so isolated sweeps mislead; best of reps after one warm-up step.
+static int tune_trial(ramgpu_ctx* ctx, double dts, int reps, cudaEvent_t e0, cudaEvent_t e1, float& best) {
+  best = 1e30f;
+  for (int r = 0; r <= reps; ++r) {
+    cudaEventRecord(e0, ctx->stream);
+    if (int rc = enqueue_body(ctx, dts, !ctx->graph_on)) return rc;
+    cudaEventRecord(e1, ctx->stream);
+    cudaEventSynchronize(e1);
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    if (r > 0 && ms < best) best = ms;
+  }
+  return RAMGPU_OK;
+}
+
+static int tune(ramgpu_ctx* ctx, double dts, int reps, cudaEvent_t e0, cudaEvent_t e1, double* best_ms4) {
+  const int cand_blk[4] = {32, 64, 128, 256};
+  for (int w = 0; w < 4; ++w) {
+    ctx->tune_plain_ms[w] = ctx->tune_pers_ms[w] = 0.0;
+    float best = 1e30f;
+    int bb = ctx->d.blk[w], bp = ctx->d.pers[w], bl = ctx->d.mu_lanes;
+    // DRIFTMU: 4, 2 and 1 lanes per line, as NPA allows
+    const int nlanes = w != 3 ? 1 : (ctx->d.npa >= 24 ? 4 : (ctx->d.npa >= 12 ? 2 : 1));
+    for (int lanes = nlanes; lanes >= 1; lanes /= 2)
+      for (int ib = 0; ib < 4; ++ib) {
+        for (int persist = 0; persist < 2; ++persist) {
+          const int blk = cand_blk[ib];
+          if (w == 3) ctx->d.mu_lanes = lanes;
+          int pc = 0;
+          if (persist) {
+            const int per_sm = sweep_max_blocks_per_sm(w, blk);
+            if (per_sm <= 0) continue;
+            pc = per_sm * ctx->d.nsm;
+          }
+          ctx->d.blk[w] = blk;
+          ctx->d.pers[w] = pc;
+          float t;
+          if (int rc = tune_trial(ctx, dts, reps, e0, e1, t)) return rc;
+          if (t < best) { best = t; bb = blk; bp = pc; bl = ctx->d.mu_lanes; }
+          double& rec = persist ? ctx->tune_pers_ms[w] : ctx->tune_plain_ms[w];
+          if (rec == 0.0 || t < rec) rec = t;
+        }
+      }
+    ctx->d.blk[w] = bb;
+    ctx->d.pers[w] = bp;
+    if (w == 3) ctx->d.mu_lanes = bl;
+    if (best_ms4) best_ms4[w] = best;
+  }
+  // then the number of concurrent item groups, 1, 2, 4 or 8 (at most one
+  // per item), on the chosen shapes
+  float best = 1e30f;
+  int bg = ctx->step_groups;
+  ctx->groups_set = true;
+  for (int G = 1; G <= 8 && G <= ctx->d.nitems; G *= 2) {
+    ctx->step_groups = G;
+    float t;
+    if (int rc = tune_trial(ctx, dts, reps, e0, e1, t)) return rc;
+    if (t < best) { best = t; bg = G; }
+  }
+  ctx->step_groups = bg;
+  return RAMGPU_OK;
+}
+
 int ramgpu_autotune(ramgpu_ctx* ctx, double dts, int reps, double* best_ms4) {
   if (check_ctx(ctx)) return RAMGPU_ERR_ARG;
   if (reps < 1) reps = 3;
@@ -2416,109 +2481,63 @@ int ramgpu_autotune(ramgpu_ctx* ctx, double dts, int reps, double* best_ms4) {
   launch_member_coef(ctx->d, dts, ctx->stream);
   launch_ghost(ctx->d, ctx->stream);
   ctx->launches += 3;
-  // the trials advance F2: keep a copy of every active slot and restore it
-  const size_t ncell = ctx->d.ncell;
-  double* snap = nullptr;
-  CK(cudaMalloc(&snap, sizeof(double) * ncell * ctx->items_h.size()));
-  for (size_t i = 0; i < ctx->items_h.size(); ++i) {
-    const int slot = ctx->items_h[i].x * ctx->d.ns + ctx->items_h[i].y;
-    CK(cudaMemcpyAsync(snap + i * ncell, ctx->d.f2 + (size_t)slot * ncell, sizeof(double) * ncell,
-                       cudaMemcpyDeviceToDevice, ctx->stream));
-  }
-  int nsm = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  const int cand_blk[4] = {32, 64, 128, 256};
-  for (int w = 0; w < 4; ++w) {
-    ctx->tune_plain_ms[w] = ctx->tune_pers_ms[w] = 0.0;
-    float best = 1e30f;
-    int bb = ctx->d.blk[w], bp = ctx->d.pers[w], bl = ctx->d.mu_lanes;
-    // DRIFTMU: 4, 2 and 1 lanes per line, as NPA allows
-    const int nlanes = w != 3 ? 1 : (ctx->d.npa >= 24 ? 4 : (ctx->d.npa >= 12 ? 2 : 1));
-    for (int lanes = nlanes; lanes >= 1; lanes /= 2)
-    for (int ib = 0; ib < 4; ++ib) {
-      for (int persist = 0; persist < 2; ++persist) {
-        const int blk = cand_blk[ib];
-        if (w == 3) ctx->d.mu_lanes = lanes;
-        int pc = 0;
-        if (persist) {
-          const int per_sm = sweep_max_blocks_per_sm(w, blk);
-          if (per_sm <= 0) continue;
-          pc = per_sm * nsm;
-        }
-        ctx->d.blk[w] = blk;
-        ctx->d.pers[w] = pc;
-        // one trial = a whole ram_run step (direct launches) with this
-        // sweep's shape and the others' current ones: the sweeps interact
-        // through L2 and the SM schedule, so isolated sweeps mislead; best
-        // of reps after one warm-up step
-        float tbest = 1e30f;
-        for (int r = 0; r <= reps; ++r) {
-          cudaEventRecord(e0, ctx->stream);
-          if (int rc2 = enqueue_body(ctx, dts, !ctx->graph_on)) {
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            cudaFree(snap);
-            return rc2;
-          }
-          cudaEventRecord(e1, ctx->stream);
-          cudaEventSynchronize(e1);
-          float ms = 0.f;
-          cudaEventElapsedTime(&ms, e0, e1);
-          if (r > 0 && ms < tbest) tbest = ms;
-        }
-        if (tbest < best) { best = tbest; bb = blk; bp = pc; bl = ctx->d.mu_lanes; }
-        double& rec = persist ? ctx->tune_pers_ms[w] : ctx->tune_plain_ms[w];
-        if (rec == 0.0 || tbest < rec) rec = tbest;
-      }
+  // a trial is a step: what a step leaves behind (F2, the loss books, the
+  // moments and their host copy, the limits and clip counts, the status
+  // word) is kept and restored
+  Dev& d = ctx->d;
+  const size_t nslot = (size_t)d.nm * d.ns, nm2 = nslot * d.nr * d.nt, ncell = d.ncell;
+  struct Part {
+    void* at;
+    size_t bytes;
+  };
+  std::vector<Part> parts = {{ctx->losses, sizeof(double) * nslot * 6},
+                             {d.ppert, sizeof(double) * nm2},
+                             {d.ppart, sizeof(double) * nm2},
+                             {d.cflq, sizeof(unsigned long long) * nslot * 5}};
+  for (const int2& it : ctx->items_h)
+    parts.push_back({d.f2 + ((size_t)it.x * d.ns + it.y) * ncell, sizeof(double) * ncell});
+  size_t total = 0;
+  for (const Part& q : parts) total += q.bytes;
+  char* snap = nullptr;
+  CK(cudaMalloc(&snap, total));
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaError_t e = cudaEventCreate(&e0);
+  if (e == cudaSuccess) e = cudaEventCreate(&e1);
+  auto copies = [&](bool back) {
+    size_t o = 0;
+    for (const Part& q : parts) {
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(back ? q.at : snap + o, back ? snap + o : q.at, q.bytes, cudaMemcpyDeviceToDevice,
+                            ctx->stream);
+      o += q.bytes;
     }
-    ctx->d.blk[w] = bb;
-    ctx->d.pers[w] = bp;
-    if (w == 3) ctx->d.mu_lanes = bl;
-    if (best_ms4) best_ms4[w] = best;
-  }
-  // then the number of concurrent item groups, 1, 2, 4 or 8 (at most one
-  // per item), on the chosen shapes
-  {
-    float best = 1e30f;
-    int bg = ctx->step_groups;
-    ctx->groups_set = true;
-    for (int G = 1; G <= 8 && G <= ctx->d.nitems; G *= 2) {
-      ctx->step_groups = G;
-      float tbest = 1e30f;
-      for (int r = 0; r <= reps; ++r) {
-        cudaEventRecord(e0, ctx->stream);
-        if (int rc2 = enqueue_body(ctx, dts, !ctx->graph_on)) {
-          cudaEventDestroy(e0);
-          cudaEventDestroy(e1);
-          cudaFree(snap);
-          return rc2;
-        }
-        cudaEventRecord(e1, ctx->stream);
-        cudaEventSynchronize(e1);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (r > 0 && ms < tbest) tbest = ms;
-      }
-      if (tbest < best) { best = tbest; bg = G; }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  };
+  copies(false);
+  if (e == cudaSuccess) {
+    const std::vector<double> mom(ctx->mom_h, ctx->mom_h + 2 * nm2);
+    const std::vector<unsigned long long> st(ctx->status_h, ctx->status_h + 5);
+    const Dev shapes = d;
+    const int groups = ctx->step_groups;
+    const bool set = ctx->groups_set;
+    rc = tune(ctx, dts, reps, e0, e1, best_ms4);
+    if (rc) {  // as it was, once the groups' streams are done with F2
+      cudaDeviceSynchronize();
+      d = shapes;
+      ctx->step_groups = groups;
+      ctx->groups_set = set;
     }
-    ctx->step_groups = bg;
+    copies(true);
+    std::copy(mom.begin(), mom.end(), ctx->mom_h);
+    std::copy(st.begin(), st.end(), ctx->status_h);
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  for (size_t i = 0; i < ctx->items_h.size(); ++i) {
-    const int slot = ctx->items_h[i].x * ctx->d.ns + ctx->items_h[i].y;
-    cudaMemcpyAsync(ctx->d.f2 + (size_t)slot * ncell, snap + i * ncell, sizeof(double) * ncell,
-                    cudaMemcpyDeviceToDevice, ctx->stream);
-  }
-  cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
   cudaFree(snap);
+  ctx->shape_version += 1;
+  if (rc) return rc;
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "autotune");
-  ctx->shape_version += 1;
   return RAMGPU_OK;
 }
 

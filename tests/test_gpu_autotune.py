@@ -1,0 +1,53 @@
+"""GPU: the autotuner leaves no trace but the launch shapes."""
+import numpy as np
+import pytest
+
+from ramgpu import abi, workload as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _gpu(wl, flags=0):
+    gpu = abi.RamGpu(wl.grid, wl.fields, flags=flags)
+    for s in range(len(wl.grid.species)):
+        gpu.upload_f2(0, s, np.asfortranarray(wl.f2[s]))
+        gpu.set_boundary(0, s, wl.fgeos[s])
+    gpu.set_kp(0, 4.0)
+    return gpu
+
+
+def _state(gpu, ns):
+    out = [gpu.download_f2(0, s) for s in range(ns)]
+    out += [np.concatenate(gpu.moments(0, s)) for s in range(ns)]
+    return out + [gpu.cfl(0, s) for s in range(ns)]
+
+
+@pytest.mark.parametrize("flags", [0, abi.FLAG_LOSSES])
+@pytest.mark.parametrize("check", [False, True])
+def test_autotune_leaves_the_results_alone(flags, check):
+    """F2, the loss books, the moments, the Courant limits and the status word
+    are those of the last call after a tuning, and the next call's are those of
+    a context that was never tuned."""
+    wl = W.make_workload("tiny_pert")
+    ns = len(wl.grid.species)
+    ref, tun = _gpu(wl, flags), _gpu(wl, flags)
+    try:
+        for g in (ref, tun):
+            g.set_check(check)
+            if flags:
+                g.reset_losses()
+            g.ram_run(wl.dts)
+        tun.autotune(wl.dts, reps=1)
+        for step in range(2):
+            for a, b in zip(_state(ref, ns), _state(tun, ns)):
+                assert np.array_equal(a, b), step
+            if flags:
+                for s in range(ns):
+                    assert np.array_equal(ref.losses(0, s), tun.losses(0, s)), (step, s)
+            if check:
+                assert ref.last_status() == tun.last_status(), step
+            for g in (ref, tun):
+                g.ram_run(wl.dts)
+    finally:
+        ref.close()
+        tun.close()
