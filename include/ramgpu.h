@@ -384,8 +384,8 @@ int ramgpu_set_graph(ramgpu_ctx *ctx, int enable);
 int ramgpu_set_launch_shape(ramgpu_ctx *ctx, int sweep, int threads, int persistent_ctas);
 int ramgpu_get_launch_shape(ramgpu_ctx *ctx, int *threads4, int *persistent4);
 /* Lanes per DRIFTMU line: 4 (NPA >= 24), 2 (adjacent lanes share a line,
- * NPA >= 12) or 1; until set, the number of lines decides (1 to 8).  Results
- * are the same bit for bit; the autotuner tries 1, 2 and 4. */
+ * NPA >= 12), 1, or 0, the default: the number of lines decides (1 to 8).
+ * Results are the same bit for bit; the autotuner tries 0, then the others. */
 int ramgpu_set_mu_lanes(ramgpu_ctx *ctx, int lanes);
 /* Autotuner: for each sweep in turn, tries 32/64/128/256 threads per CTA,
  * each with a one-unit-per-CTA grid and a persistent grid (resident CTAs x

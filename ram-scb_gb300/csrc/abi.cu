@@ -2393,7 +2393,8 @@ int ramgpu_set_launch_shape(ramgpu_ctx* ctx, int sweep, int threads, int persist
 
 int ramgpu_set_mu_lanes(ramgpu_ctx* ctx, int lanes) {
   if (check_ctx(ctx)) return RAMGPU_ERR_ARG;
-  if (lanes != 1 && lanes != 2 && lanes != 4) return fail(ctx, RAMGPU_ERR_ARG, "lanes must be 1, 2 or 4");
+  if (lanes != 0 && lanes != 1 && lanes != 2 && lanes != 4)
+    return fail(ctx, RAMGPU_ERR_ARG, "lanes must be 1, 2, 4 or 0 (by the number of lines)");
   if (lanes == 2 && ctx->d.npa < 12) return fail(ctx, RAMGPU_ERR_ARG, "two lanes per line need NPA >= 12");
   if (lanes == 4 && ctx->d.npa < 24) return fail(ctx, RAMGPU_ERR_ARG, "four lanes per line need NPA >= 24");
   ctx->d.mu_lanes = lanes;
@@ -2430,9 +2431,17 @@ static int tune(ramgpu_ctx* ctx, double dts, int reps, cudaEvent_t e0, cudaEvent
     ctx->tune_plain_ms[w] = ctx->tune_pers_ms[w] = 0.0;
     float best = 1e30f;
     int bb = ctx->d.blk[w], bp = ctx->d.pers[w], bl = ctx->d.mu_lanes;
-    // DRIFTMU: 4, 2 and 1 lanes per line, as NPA allows
-    const int nlanes = w != 3 ? 1 : (ctx->d.npa >= 24 ? 4 : (ctx->d.npa >= 12 ? 2 : 1));
-    for (int lanes = nlanes; lanes >= 1; lanes /= 2)
+    // DRIFTMU: the lanes per line that the number of lines gives (0, which
+    // keeps to the rule as the work list changes), then those of 4, 2 and 1
+    // that NPA allows and the rule does not give here
+    std::vector<int> cand_lanes = {0};
+    if (w == 3) {
+      ctx->d.mu_lanes = 0;
+      const int rule = mu_lanes(ctx->d);
+      for (int n = ctx->d.npa >= 24 ? 4 : (ctx->d.npa >= 12 ? 2 : 1); n >= 1; n /= 2)
+        if (n != rule) cand_lanes.push_back(n);
+    }
+    for (const int lanes : cand_lanes)
       for (int ib = 0; ib < 4; ++ib) {
         for (int persist = 0; persist < 2; ++persist) {
           const int blk = cand_blk[ib];

@@ -62,6 +62,7 @@ void launch_sweep_mu(const Dev& d, double dts, bool cfl, int loss_mode, const do
                      cudaStream_t st, unsigned char* rec = nullptr, bool replay = false, int rsh = 0);
 
 int sweep_max_blocks_per_sm(int w, int blk);
+int mu_lanes(const Dev& d);  // lanes per DRIFTMU line of the list d: as set or by the number of lines
 
 void launch_field_tables(const Dev& d, cudaStream_t st);
 void launch_species_static(const Dev& d, unsigned long long* sep_dev, cudaStream_t st);

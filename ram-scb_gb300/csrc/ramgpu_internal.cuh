@@ -130,7 +130,7 @@ struct Dev {
   // a persistent grid of that many CTAs looping over (item, line-block) units
   int blk[4];
   int pers[4];
-  int mu_lanes;  // lanes per DRIFTMU line: 1, 2 or 4 as set, 0 by the number of lines
+  int mu_lanes;  // lanes per DRIFTMU line: 1, 2 or 4 as set, 0 by the number of lines (1 to 8)
   // L window of the R, P and E sweeps and the closing copy/mask: planes
   // [lw0, lw1) (0 and NPA: all); a host pipeline runs them chunk by chunk
   int lw0, lw1;

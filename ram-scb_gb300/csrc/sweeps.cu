@@ -818,8 +818,8 @@ void launch_sweep_e(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigne
 // unless said: one species (3.4 warps an SM with one lane) 0.264, 0.224,
 // 0.203; four (14) 0.422, 0.390, 0.387; two members of four (27) 0.675,
 // 0.679, 0.698; eight (109) 2.52, 2.64, 2.71; 6x9x35x72, four species (1.3)
-// 0.193, 0.153, 0.134, and 0.122 with 8.  Segments keep at least four cells.
-static int mu_lanes(const Dev& d) {
+// 0.193, 0.153, 0.134, and 0.122 with 8.  Segments keep at least six cells.
+int mu_lanes(const Dev& d) {
   int want = d.mu_lanes;
   if (!want) {
     const long long warps = (long long)(d.nr - 1) * d.nt * d.ne * d.nlist / 32;

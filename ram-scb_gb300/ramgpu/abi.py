@@ -733,7 +733,8 @@ class RamGpu:
         return J
 
     def set_mu_lanes(self, lanes: int):
-        """Lanes per DRIFTMU line (2: lane pairs, NPA >= 12; 1)."""
+        """Lanes per DRIFTMU line: 4 (NPA >= 24), 2 (NPA >= 12) or 1; 0, the
+        default: by the number of lines."""
         self._ck(self.lib.ramgpu_set_mu_lanes(self.h, int(lanes)), "set_mu_lanes")
 
     def set_adj_record_budget(self, nbytes: int):

@@ -51,3 +51,25 @@ def test_autotune_leaves_the_results_alone(flags, check):
     finally:
         ref.close()
         tun.close()
+
+
+def test_lanes_return_to_the_rule():
+    """A fixed DRIFTMU lane count, and what a tuning chose, go back to the
+    automatic one with 0, whose results are the same bits."""
+    wl = W.make_workload("tiny_pert")
+    ns = len(wl.grid.species)
+    ref, gpu = _gpu(wl), _gpu(wl)
+    try:
+        for act in (lambda: gpu.set_mu_lanes(2), lambda: gpu.set_mu_lanes(0), lambda: gpu.autotune(wl.dts, reps=1),
+                    lambda: gpu.set_mu_lanes(0)):
+            act()
+            ref.ram_run(wl.dts)
+            gpu.ram_run(wl.dts)
+            for a, b in zip(_state(ref, ns), _state(gpu, ns)):
+                assert np.array_equal(a, b)
+        for lanes in (3, 8, -1):
+            with pytest.raises(abi.RamGpuError):
+                gpu.set_mu_lanes(lanes)
+    finally:
+        ref.close()
+        gpu.close()
