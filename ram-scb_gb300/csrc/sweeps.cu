@@ -98,9 +98,16 @@ __device__ __forceinline__ double face_phi(double uu, double u, double d, double
 
 // The line's largest Courant number, as the face with the smallest 1 - U:
 // its quotient is formed once, after the line, in FP64 (a few operations a
-// line; every face's took 16 integer instructions and cut the quotient).  Faces whose U differ by less
-// than 2^-63 count as equal, which moves DtDrift by at most one rounding
-// wherever it is below its cap.
+// line; every face's took 16 integer instructions and cut the quotient).
+// 1 - U has units of 2^-63, so another face's quotient may be larger than the
+// one formed, by less than 2^-62/U of it: below a rounding from U = 2^-9 on.
+// A limit just below its cap of 1e4 s has U = FracCFL*DTs/1e4, so up to 5e-16
+// at DTs = 5 s and 3e-14 at 0.1 s (the parity bar is 1e-12).  Telling such
+// faces apart cost more than it gives, four species on 20x25x35x72 and
+// 40x49x70x144, ms a call: 0.3625, 4.634 as it is; 0.368, 4.668 with the line's
+// quotients all formed where two faces tie; 0.378, 4.717 where the largest U
+// is below 2^-10 and the slot's limit is not above it yet; 0.376, 4.913 with
+// the quotient of a face that ties formed at once.
 struct Largest {
   uint64_t a63 = 1ULL << 63;
   int at = 0;
