@@ -102,7 +102,8 @@ __device__ __forceinline__ double face_phi(double uu, double u, double d, double
 // 1 - U has units of 2^-63, so another face's quotient may be larger than the
 // one formed, by less than 2^-62/U of it: below a rounding from U = 2^-9 on.
 // A limit just below its cap of 1e4 s has U = FracCFL*DTs/1e4, so up to 5e-16
-// at DTs = 5 s and 3e-14 at 0.1 s (the parity bar is 1e-12).  Telling such
+// at DTs = 5 s and 3e-14 at 0.1 s (the parity bar is 1e-12), while one below
+// 40 s, as sets the next step, is within a rounding at either.  Telling such
 // faces apart cost more than it gives, four species on 20x25x35x72 and
 // 40x49x70x144, ms a call: 0.3625, 4.634 as it is; 0.368, 4.668 with the line's
 // quotients all formed where two faces tie; 0.378, 4.717 where the largest U
