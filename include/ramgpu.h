@@ -224,9 +224,10 @@ int ramgpu_ram_run_ref(ramgpu_ctx *ctx, double dts, double *const *f2, double *c
  * unpipelined; 2 page-locked F2 arrays of ramgpu_ram_run_ref through the
  * copy engines plane chunk by plane chunk into a device staging area
  * inside the pipeline, the others in place.  On GB300's coherent Grace
- * link in place is fastest (0.88 ms per four-species call, against
- * 0.95-1.08 ms for 2 and 1.00 ms for 1); 1 and 2 are for hosts whose link
- * favours the copy engines. */
+ * link in place is fastest (0.74 ms per four-species call from page-locked
+ * memory, against 0.83-0.97 ms for 2 and 0.89 ms for 1; 0.78 ms from pageable
+ * memory, 0.96 ms for 1); 1 and 2 are for hosts whose link favours the copy
+ * engines. */
 int ramgpu_set_ref_staging(ramgpu_ctx *ctx, int force);
 /* Chunks of L planes the host calls (ramgpu_ram_run_host, ramgpu_ram_run_ref)
  * pipeline F2 over: 1..8, or 0 for the item-group pipeline of
@@ -242,7 +243,7 @@ int ramgpu_set_ref_staging(ramgpu_ctx *ctx, int force);
  * Results are the same for every count. */
 int ramgpu_set_pipeline_chunks(ramgpu_ctx *ctx, int chunks);
 /* Number of item groups ramgpu_ram_run_host pipelines its copies over
- * (1..8, default 4, at most one per item; 1 with RAMGPU_FLAG_LOSSES). */
+ * (1..8, default 4, at most one per item). */
 int ramgpu_set_pipeline_groups(ramgpu_ctx *ctx, int groups);
 /* The configured pipeline group count (0 for a bad context). */
 int ramgpu_pipeline_groups(const ramgpu_ctx *ctx);
@@ -258,9 +259,8 @@ int ramgpu_pipeline_trace(ramgpu_ctx *ctx, int *groups, float *ms);
  * concurrent streams (1..8, at most one per item; until set or tuned 4, but 1
  * for lists below 1.5 M cells, whose launches run in one wave): one group's
  * launch tails and the gaps between its dependent launches fill with the
- * others' CTAs.  Results are the same for every count; the loss
- * bookkeeping (RAMGPU_FLAG_LOSSES) and per-kernel timing passes run as one
- * group.  The autotuner picks the count. */
+ * others' CTAs.  Results are the same for every count; per-kernel timing
+ * passes run as one group.  The autotuner picks the count. */
 int ramgpu_set_step_groups(ramgpu_ctx *ctx, int groups);
 /* The configured step group count (0 for a bad context). */
 int ramgpu_step_groups(const ramgpu_ctx *ctx);

@@ -886,9 +886,10 @@ static int enqueue_chunked(ramgpu_ctx* ctx, double dts, int C, In&& in, Out&& ou
 // the item-group pipeline), and only with at least two planes per chunk.
 // auto_chunks: the count used while the setting is automatic (-1).  Measured
 // on the four-species step: per-species page-locked arrays go faster over
-// the item-group pipeline (0.69 ms per call against 0.93-1.07 ms chunked),
-// the reference layout over 4 chunks (us a call with 2, 3, 4, 5, 6, 8: 805,
-// 770, 772, 791, 790, 790; unchunked 807).
+// the item-group pipeline (0.61 ms per call against 0.81-0.93 ms chunked),
+// the reference layout over 3 or 4 chunks (us a call with 2, 3, 4, 5, 6, 8:
+// pageable 802, 769, 776, 789, 822, 798, unchunked 807; page-locked 763, 732,
+// 741, 750, 754, 744, unchunked 764).
 static int chunk_count(const ramgpu_ctx* ctx, int auto_chunks) {
   const int want = ctx->pipe_chunks < 0 ? auto_chunks : ctx->pipe_chunks;
   if (want <= 0 || (ctx->cfg.flags & RAMGPU_FLAG_LOSSES) || ctx->pd_any() || ctx->pipe_trace) return 0;
@@ -2359,7 +2360,7 @@ int ramgpu_set_coef_store(ramgpu_ctx* ctx, int mask) {
   if ((unsigned)mask == ctx->coef_mask) return RAMGPU_OK;
   ctx->coef_mask = (unsigned)mask;
   CK(cudaStreamSynchronize(ctx->stream));
-  cudaFree(ctx->d.coef);  // reallocated for the new set by the next step
+  cudaFree(ctx->d.coef);  // allocated again by the next ramgpu_adj_backward
   ctx->d.coef = nullptr;
   ctx->d.coef_items = 0;
   ctx->shape_version += 1;

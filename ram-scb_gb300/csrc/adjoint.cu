@@ -9,7 +9,8 @@
 //   Fnew(i) = G(i) + w(i) (Phi(i-1) - Phi(i)),  Phi(f) = C(f) FBND(f),
 //   FBND(f) = FUP(f) + a(f) LX(f),  LX in {beta D, X, D, beta X},
 // so its adjoint is the transposed map, applied here line by line with the
-// coefficients recomputed from the same tables as the forward pass.  The
+// coefficients recomputed, from the forward pass's tables or, in DRIFTE, from
+// EDOT and EB (the forward sweep's factored form agrees to rounding).  The
 // tail of ram_run (periodic copy, magnetopause mask, ANISCH's F2(:,:,:,:,1)
 // side effect), the CEX/ATMOL factors and the log-flux observation operator
 // are transposed too.  dJ/dFGEOS collects the ghost cells of DRIFTR,
@@ -43,7 +44,8 @@ namespace ramgpu {
 // The transposes are bound by the FP64 unit, so the two FP64 operations that
 // form the weights move to integer instructions (as in face.cuh).  Backward
 // ms a call on 20x25x35x72, one species and four: 0.270 -> 0.262, 0.532 ->
-// 0.502.  That is FP64 for 81 % of the time with four species; forming the
+// 0.502.  The 46 FP64 operations a cell and call that the eight transposes
+// execute (five to eight each) take 0.44 of the 0.50 ms of four species; forming the
 // product FBb = C*DL on the integer pipe as well was slower or even in every
 // sweep.
 

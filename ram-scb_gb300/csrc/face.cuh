@@ -26,11 +26,11 @@
 // FP64 sequence held the FP64 pipe, five operations a face in DRIFTR and
 // DRIFTP and up to seven in DRIFTE and DRIFTMU (phi, beta|X| and the Courant
 // products were integer products already).  Here three remain (the coefficient's fma
-// and the update); instruction issue (55-64 %, 170-210 instructions a face),
-// the integer ALU (60 %) and the FP64 pipe (58 %) are about even.  DRIFTR
-// 64.5 -> 52.1 us, DRIFTP 61.8 -> 46.9, DRIFTE 66.8 -> 54.4, DRIFTMU 68.6 ->
-// 61.5; on 40x49x70x144 DRIFTP 783 -> 543, DRIFTE 875 -> 580, DRIFTMU 946 ->
-// 691.  Normalising the factor and the
+// and the update); instruction issue (50-61 %, 170-210 instructions a face),
+// the integer ALU (51-59 %) and the FP64 pipe (52-67 %) are about even.  With the
+// sweeps as they are now, DRIFTR 64.5 -> 52.8 us, DRIFTP 61.8 -> 46.8, DRIFTE
+// 66.8 -> 54.7, DRIFTMU 68.6 -> 56.1; on 40x49x70x144 DRIFTR 944 -> 610, DRIFTP
+// 783 -> 538, DRIFTE 875 -> 572, DRIFTMU 946 -> 593.  Normalising the factor and the
 // differences, as the FP64 form's integer products did, took more
 // instructions than aligning the cells once.  The rare forms must stay rare:
 // before face_plain and the exact threshold below, eight warps of meridian

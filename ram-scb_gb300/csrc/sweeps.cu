@@ -66,9 +66,10 @@ static __device__ __noinline__ PhiCase face_phi_fp64(double x, double dd, double
 
 // Flux of a limited face (face.cuh) with the prepared coefficient q of C.
 // v: C or a factor of it that vanishes with it; cf(): C, and mh(): -1/2 (R, P)
-// or -1/2 over the bin width, formed only for the FP64 form.  kRec 1: cs is the branch taken; 2: the recorded branch cs
-// is applied (the same bits as the recording sweep's where that is the
-// branch the values select).  over(): called where U >= 1 or C is not finite.
+// or -1/2 over the bin width, formed only for the FP64 form.  kRec 1: cs is
+// the branch taken; 2: the recorded branch cs is applied (the same bits as the
+// recording sweep's where that is the branch the values select).  over():
+// called where U >= 1 or C is not finite.
 struct NoOver {
   __device__ __forceinline__ void operator()() const {}
 };
@@ -781,7 +782,13 @@ static void r_launch(const Dev& d, double dts, bool cfl, cudaStream_t st, unsign
 // two, 51.6 with four; the call 0.386, 0.397, 0.389 ms).  Longer lines fall
 // out of L1 between a lane's cells, and the widest access that divides NR
 // (then every line, GRT and CR row starts on its boundary) reads and writes
-// whole sectors once (NR = 40: 863, 733, 610; L2 traffic down to 0.4).
+// whole sectors once (NR = 40: 863, 733, 610; L2 traffic down to 0.4).  How
+// much that gains depends on how the lanes' lines fall into L1's sets: on
+// NR x 25x35x72, one cell against four, 72.9 and 67.5 at NR = 28, 148.8 and
+// 79.8 at 32, 89.9 and 83.0 at 36, 133.1 and 90.3 at 40.  Odd NR spread over
+// all sets and lose nothing one cell at a time (63.1 at 25, 65.6 at 27).  Two
+// cells against one: 69.4 and 66.0, 77.9 and 73.7, 88.3 and 82.2 at NR = 26, 30
+// and 34, but 444 and 440, 506 and 512, 569 and 585 on NR x 49x70x144.
 static int r_width(const Dev& d) { return d.nr <= 24 || d.nr % 2 ? 1 : (d.nr % 4 ? 2 : 4); }
 void launch_sweep_r(const Dev& d, double dts, bool cfl, cudaStream_t st, unsigned char* rec, bool replay, int rsh) {
   const bool kb = beta_b32(d);
