@@ -49,25 +49,27 @@ UNIT = "cell-updates/s"
 # digest; a changed kernel makes the figures stale until the next capture.
 NCU_CAPTURE = {
     # ncu on the sources named by sources_sha16 (profiles/sweeps_four_sp.md):
-    # the sweep launches of one whole call, summed over its item groups; the
-    # mean of the forward and the reverse half, as the timing pass counts them
-    "sources_sha16": "f67598a11b2ae3d7",
+    # one kernel a command, its forward and its reverse launch over the whole
+    # list (one item group); the timing pass counts the mean of the two.  Run
+    # the python command alone first; refined holds 4 GB on the device.
+    "sources_sha16": "2ce1f33da8605f3e",
     "command": ("ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum,lts__t_bytes.sum,"
                 "smsp__sass_thread_inst_executed_op_{dadd,dfma,dmul}_pred_on.sum --clock-control none "
-                "-k regex:k_sweep_ -c <32|8> python bench.py --steps 2 --warmup 1 --sections headline "
-                "--no-cpu-baseline --no-e2e --no-autotune [--workload refined|single_h]"),
-    "dram_bytes": {"four_sp": {"driftr": 44.10e6, "driftp": 41.58e6, "drifte": 41.61e6,
-                               "driftmu": 0.5 * (42.13e6 + 81.92e6)},
-                   "single_h": {"driftr": 11.03e6, "driftp": 10.39e6, "drifte": 10.40e6,
-                                "driftmu": 0.5 * (10.53e6 + 20.48e6)},
-                   "refined": {"driftr": 0.5 * (1112.3e6 + 1142.4e6), "driftp": 1041.0e6, "drifte": 1029.8e6,
-                               "driftmu": 0.5 * (1044.4e6 + 1743.1e6)}},
-    "l2_bytes": {"four_sp": {"driftr": 0.5 * (448.5e6 + 454.6e6), "driftp": 0.5 * (156.7e6 + 157.7e6),
-                             "drifte": 0.5 * (143.9e6 + 145.3e6), "driftmu": 0.5 * (280.6e6 + 394.8e6)},
-                 "single_h": {"driftr": 0.5 * (111.7e6 + 113.3e6), "driftp": 0.5 * (39.2e6 + 39.4e6),
-                              "drifte": 0.5 * (41.9e6 + 44.4e6), "driftmu": 0.5 * (70.1e6 + 98.8e6)},
-                 "refined": {"driftr": 0.5 * (3555.1e6 + 3660.7e6), "driftp": 0.5 * (2441.8e6 + 2453.5e6),
-                             "drifte": 0.5 * (2175.7e6 + 2184.5e6), "driftmu": 0.5 * (3360.9e6 + 4480.2e6)}},
+                "-k regex:<k_sweep_r|k_sweep_p|k_sweep_e|k_sweep_mu> -c 2 python bench.py --steps 2 --warmup 1 "
+                "--sections headline --no-cpu-baseline --no-e2e --no-autotune --item-groups 1 "
+                "--workload <four_sp|single_h|refined>"),
+    "dram_bytes": {"four_sp": {"driftr": 44.65e6, "driftp": 40.65e6, "drifte": 39.8e6,
+                               "driftmu": 0.5 * (86.2e6 + 40.6e6)},
+                   "single_h": {"driftr": 11.0e6, "driftp": 10.4e6, "drifte": 10.4e6,
+                                "driftmu": 0.5 * (20.5e6 + 10.5e6)},
+                   "refined": {"driftr": 0.5 * (1310.9e6 + 1278.1e6), "driftp": 0.5 * (1225.3e6 + 1215.4e6),
+                               "drifte": 1205.6e6, "driftmu": 0.5 * (1875.8e6 + 1208.8e6)}},
+    "l2_bytes": {"four_sp": {"driftr": 0.5 * (507.3e6 + 501.6e6), "driftp": 0.5 * (160.0e6 + 156.1e6),
+                             "drifte": 0.5 * (140.9e6 + 139.8e6), "driftmu": 0.5 * (416.1e6 + 271.9e6)},
+                 "single_h": {"driftr": 0.5 * (113.5e6 + 112.0e6), "driftp": 0.5 * (40.1e6 + 39.5e6),
+                              "drifte": 0.5 * (44.5e6 + 42.2e6), "driftmu": 0.5 * (99.0e6 + 69.0e6)},
+                 "refined": {"driftr": 0.5 * (3735.4e6 + 3625.9e6), "driftp": 0.5 * (2486.6e6 + 2451.6e6),
+                             "drifte": 0.5 * (2200.2e6 + 2187.6e6), "driftmu": 0.5 * (4582.5e6 + 3444.7e6)}},
     "fp64_ops_per_cell": {"driftr": 3.06, "driftp": 2.74, "drifte": 0.5 * (2.90 + 2.99),
                           "driftmu": 0.5 * (2.84 + 3.89)},
 }
@@ -98,6 +100,9 @@ def parse():
     ap.add_argument("--flush-mb", type=int, default=256)
     ap.add_argument("--no-graph", action="store_true")
     ap.add_argument("--no-autotune", action="store_true")
+    ap.add_argument("--item-groups", type=int, default=0,
+                    help="concurrent item groups of the step and the adjoint (0: as tuned or the library's default; "
+                         "1 for profiling: one launch per kernel over the whole list)")
     ap.add_argument("--no-coef-store", action="store_true",
                     help="recompute the face coefficients in the second DRIFTE transpose instead of keeping them")
     ap.add_argument("--members", type=int, default=256, help="ensemble members")
@@ -584,6 +589,8 @@ def measure(args, torch, np, abi, W, stream, name, steps, warmup, world=1, clock
     gpu.set_kp(-1, wl.kp(0))
     if args.no_coef_store:
         gpu.set_coef_store(0)
+    if args.item_groups:
+        gpu.set_step_groups(args.item_groups)
     if args.no_autotune:
         shapes, trials = gpu.launch_shape(), None
     else:
@@ -889,7 +896,10 @@ def run_adjoint(args, torch, np, abi, W, stream):
         torch.cuda.synchronize()
 
     reset()
-    gpu.autotune(wl.dts)
+    if not args.no_autotune:
+        gpu.autotune(wl.dts)
+    if args.item_groups:
+        gpu.set_step_groups(args.item_groups)
     gpu.set_graph(True)
     for c in range(2):
         gpu.set_kp(-1, kp[c, 0])
