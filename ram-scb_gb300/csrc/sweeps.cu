@@ -78,13 +78,13 @@ __device__ __forceinline__ double face_phi(double uu, double u, double d, double
                                            uint64_t betaf, int& cs, C&& cf, M&& mh, O&& over = O()) {
   bool special;
   int taken = 0;
-  double phi =
-      bitsd(face_flux<kRec == 1 || kRec == 2, kB32>(dbits(uu), dbits(u), dbits(d), q, betaf, special, taken));
-  if (kRec == 2) special = special || taken != cs;
+  double phi = bitsd(
+      kRec == 2 ? face_flux_frozen<kB32>(dbits(uu), dbits(u), dbits(d), q, betaf, cs, special)
+                : face_flux<kRec == 1, kB32>(dbits(uu), dbits(u), dbits(d), q, betaf, special, taken));
   if (kRec == 1) cs = taken;
   if (special) {
     if (q.bad < 0) over();
-    if (kRec != 2 && face_plain(dbits(uu), dbits(u), dbits(d), dbits(v))) {
+    if ((kRec != 2 || cs == 0) && face_plain(dbits(uu), dbits(u), dbits(d), dbits(v))) {
       if (kRec == 1) cs = 0;
       if (q.bad < 0 || (dbits(u) != 0ULL && (dbits(v) << 1) != 0ULL)) return __dmul_rn(cf(), u);
       return bitsd((bits64)q.sign << 32);
