@@ -52,26 +52,26 @@ NCU_CAPTURE = {
     # one kernel a command, its forward and its reverse launch over the whole
     # list (one item group); the timing pass counts the mean of the two.  Run
     # the python command alone first; refined holds 4 GB on the device.
-    "sources_sha16": "2ce1f33da8605f3e",
+    "sources_sha16": "b4c8b26f201d0847",
     "command": ("ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum,lts__t_bytes.sum,"
                 "smsp__sass_thread_inst_executed_op_{dadd,dfma,dmul}_pred_on.sum --clock-control none "
                 "-k regex:<k_sweep_r|k_sweep_p|k_sweep_e|k_sweep_mu> -c 2 python bench.py --steps 2 --warmup 1 "
                 "--sections headline --no-cpu-baseline --no-e2e --no-autotune --item-groups 1 "
                 "--workload <four_sp|single_h|refined>"),
-    "dram_bytes": {"four_sp": {"driftr": 44.65e6, "driftp": 40.65e6, "drifte": 39.8e6,
-                               "driftmu": 0.5 * (86.2e6 + 40.6e6)},
-                   "single_h": {"driftr": 11.0e6, "driftp": 10.4e6, "drifte": 10.4e6,
-                                "driftmu": 0.5 * (20.5e6 + 10.5e6)},
-                   "refined": {"driftr": 0.5 * (1310.9e6 + 1278.1e6), "driftp": 0.5 * (1225.3e6 + 1215.4e6),
-                               "drifte": 1205.6e6, "driftmu": 0.5 * (1875.8e6 + 1208.8e6)}},
-    "l2_bytes": {"four_sp": {"driftr": 0.5 * (507.3e6 + 501.6e6), "driftp": 0.5 * (160.0e6 + 156.1e6),
-                             "drifte": 0.5 * (140.9e6 + 139.8e6), "driftmu": 0.5 * (416.1e6 + 271.9e6)},
-                 "single_h": {"driftr": 0.5 * (113.5e6 + 112.0e6), "driftp": 0.5 * (40.1e6 + 39.5e6),
-                              "drifte": 0.5 * (44.5e6 + 42.2e6), "driftmu": 0.5 * (99.0e6 + 69.0e6)},
-                 "refined": {"driftr": 0.5 * (3735.4e6 + 3625.9e6), "driftp": 0.5 * (2486.6e6 + 2451.6e6),
-                             "drifte": 0.5 * (2200.2e6 + 2187.6e6), "driftmu": 0.5 * (4582.5e6 + 3444.7e6)}},
-    "fp64_ops_per_cell": {"driftr": 3.06, "driftp": 2.74, "drifte": 0.5 * (2.90 + 2.99),
-                          "driftmu": 0.5 * (2.84 + 3.89)},
+    "dram_bytes": {"four_sp": {"driftr": 0.5 * (44.8e6 + 44.6e6), "driftp": 40.7e6,
+                   "drifte": 39.8e6, "driftmu": 0.5 * (86.1e6 + 40.6e6)},
+                   "single_h": {"driftr": 11.0e6, "driftp": 10.4e6,
+                   "drifte": 10.4e6, "driftmu": 0.5 * (20.5e6 + 10.5e6)},
+                   "refined": {"driftr": 0.5 * (1311.6e6 + 1278.4e6), "driftp": 0.5 * (1225.6e6 + 1215.2e6),
+                   "drifte": 0.5 * (1205.5e6 + 1205.8e6), "driftmu": 0.5 * (1876.0e6 + 1209.6e6)}},
+    "l2_bytes": {"four_sp": {"driftr": 0.5 * (508.9e6 + 502.2e6), "driftp": 0.5 * (159.7e6 + 155.8e6),
+                   "drifte": 0.5 * (140.9e6 + 139.8e6), "driftmu": 0.5 * (415.5e6 + 272.5e6)},
+                   "single_h": {"driftr": 0.5 * (113.4e6 + 111.8e6), "driftp": 0.5 * (40.0e6 + 39.2e6),
+                   "drifte": 0.5 * (44.4e6 + 42.0e6), "driftmu": 0.5 * (98.8e6 + 68.6e6)},
+                   "refined": {"driftr": 0.5 * (3738.5e6 + 3625.9e6), "driftp": 0.5 * (2490.2e6 + 2452.7e6),
+                   "drifte": 0.5 * (2201.8e6 + 2188.2e6), "driftmu": 0.5 * (4565.6e6 + 3437.3e6)}},
+    "fp64_ops_per_cell": {"driftr": 3.06, "driftp": 2.74, "drifte": 0.5 * (2.99 + 2.90),
+                          "driftmu": 0.5 * (3.89 + 2.84)},
 }
 SWEEP_SOURCES = ["ram-scb_gb300/csrc/sweeps.cu", "ram-scb_gb300/csrc/ramgpu_internal.cuh",
                  "ram-scb_gb300/csrc/kernels.cuh", "ram-scb_gb300/csrc/face.cuh"]
